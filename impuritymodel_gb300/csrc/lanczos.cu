@@ -101,85 +101,279 @@ __global__ void spmm_alpha_kernel(int64_t n, const int64_t* __restrict__ rp, con
   }
 }
 
-// alpha_r = sum of partials; W = Y - alpha Vc - beta_prev Vp; beta partial ||W||^2.
-template <typename T>
-__global__ void axpy_beta_kernel(int64_t n, int R, typename Cx<T>::V* __restrict__ Y,
-                                 const typename Cx<T>::V* __restrict__ Vc, const typename Cx<T>::V* __restrict__ Vp,
-                                 const double* __restrict__ palpha, int nrb, const double* __restrict__ beta_prev,
-                                 double* __restrict__ alpha_out, int K, int j, double* __restrict__ pbeta) {
-  using V = typename Cx<T>::V;
-  extern __shared__ double red[];
-  __shared__ double alpha_s[32];
-  const int tr = threadIdx.x, ti = threadIdx.y;
-  const int r = blockIdx.y * blockDim.x + tr;
-  if (ti == 0 && r < R) {
-    double a = 0.0;
-    for (int b = 0; b < nrb; ++b) a += palpha[(int64_t)b * R + r];
-    alpha_s[tr] = a;
-    if (blockIdx.x == 0) alpha_out[(int64_t)r * K + j] = a;
+// ---------------------------------------------------------------------------------------
+// Grid-wide batched Lanczos (lanczos_impl): two launches per step on vectors kept unnormalised.
+//
+// w_j is stored as it leaves the three-term update and v_j = w_j / beta_{j-1} is never formed:
+// the first launch takes y = H w_j and the partial sums of <y, w_j>, the second
+//   alpha_j = <y, w_j> / beta_{j-1}^2,
+//   w_{j+1} = y / beta_{j-1} - (alpha_j / beta_{j-1}) w_j - (beta_{j-1} / beta_{j-2}) w_{j-1}
+// with the partial sums of |w_{j+1}|^2, so the normalising pass over the vectors and its launch
+// are gone.  What bounded the three-launch form on the 47 895-state sector (R = 3: 36 us each)
+// was not the vectors but every block adding the other blocks' 564 partials one after another
+// (dependent FP64 adds, ~64 cycles each on GB300) and one CSR entry in flight per thread; here
+// a block's threads share the partials (four chains each, then a fixed tree) and each thread
+// keeps kStepUnroll gathers in flight.  Per step 108 -> 33 us there, most of it FP64 issue (1300
+// FP64 warp instructions an SM in the product, rows of 3 to 13 entries side by side in a warp).
+// ---------------------------------------------------------------------------------------
+constexpr int kStepUnroll = 4;
+constexpr int kStepMaxThreads = 512;
+
+// The tile of a batch: run tiles as make_tile, in blocks of 512 threads (at most two an SM) where
+// there are rows for three quarters of those, else in blocks of 256.  Every block adds up all
+// blocks' partials, and the FP64 pipe takes ~15 cycles a warp instruction: 304 blocks instead of
+// 564 take the update from 15 to 12 us at n = 47 895, R = 3; 1024 threads (152 blocks) take it to 10
+// but the product from 20 to 23, its phases no longer overlapping another block's.
+inline RunTile make_step_tile(int64_t n, int R) {
+  RunTile t = make_tile(n, R);
+  const int rb = kStepMaxThreads / t.rt;
+  const int64_t blocks = (n + rb - 1) / rb, cap = std::max(1, 2 * grid_cap() / t.nrt);
+  if (2 * blocks * t.nrt >= 3 * grid_cap()) {
+    t.rb = rb;
+    t.nrb = (int)std::min(blocks, cap);
   }
+  return t;
+}
+
+// Sum over the thread rows ti of the block's per-thread values (thread (tr, ti) holds run tr's
+// part), in a fixed tree; valid for every thread of run tr after the call.  Synchronises.
+__device__ __forceinline__ double tile_sum(double v, double* red) {
+  const int tr = threadIdx.x, ti = threadIdx.y, rt = blockDim.x;
   __syncthreads();
-  double acc = 0.0;
+  red[ti * rt + tr] = v;
+  __syncthreads();
+  for (int len = blockDim.y; len > 1;) {
+    const int h = (len + 1) >> 1;
+    if (ti + h < len) red[ti * rt + tr] += red[(ti + h) * rt + tr];
+    __syncthreads();
+    len = h;
+  }
+  return red[tr];
+}
+
+// Sum of run r's nb per-block partials p[b * R + r], shared by the block's thread rows.
+__device__ __forceinline__ double tile_partials(const double* __restrict__ p, int nb, int R, int r, double* red) {
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
   if (r < R) {
-    const double a = alpha_s[tr];
-    const double bp = beta_prev ? beta_prev[(int64_t)r * K + (j - 1)] : 0.0;
-    const T af = (T)a, bf = (T)bp;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.y + ti; i < n; i += (int64_t)gridDim.x * blockDim.y) {
-      V y = Y[i * R + r];
-      const V c = ld(Vc + i * R + r);
-      y.x -= af * c.x;
-      y.y -= af * c.y;
-      if (Vp) {
-        const V p = ld(Vp + i * R + r);
-        y.x -= bf * p.x;
-        y.y -= bf * p.y;
+    const int step = blockDim.y;
+    int b = threadIdx.y;
+    for (; b + 3 * step < nb; b += 4 * step) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] += p[(int64_t)(b + q * step) * R + r];
+    }
+    for (; b < nb; b += step) s[0] += p[(int64_t)b * R + r];
+  }
+  return tile_sum((s[0] + s[1]) + (s[2] + s[3]), red);
+}
+
+// A row's products, one thread per run, entries [e, e1) in steps of `stride`, kStepUnroll gathers
+// in flight.
+template <typename T, bool VALC>
+__device__ __forceinline__ typename Cx<T>::V row_products(int64_t e, int64_t e1, int stride,
+                                                          const int32_t* __restrict__ col,
+                                                          const T* __restrict__ vals, int R, int r,
+                                                          const typename Cx<T>::V* __restrict__ X) {
+  using V = typename Cx<T>::V;
+  T yr = 0, yi = 0;
+  for (; e < e1; e += (int64_t)kStepUnroll * stride) {
+    int c[kStepUnroll];
+    T hr[kStepUnroll], hi[kStepUnroll];
+#pragma unroll
+    for (int u = 0; u < kStepUnroll; ++u) {
+      const int64_t eu = e + (int64_t)u * stride;
+      const bool ok = eu < e1;
+      c[u] = ok ? __ldg(col + eu) : -1;
+      hr[u] = ok ? __ldg(vals + (VALC ? 2 * eu : eu)) : T(0);
+      hi[u] = VALC && ok ? __ldg(vals + 2 * eu + 1) : T(0);
+    }
+    V x[kStepUnroll];
+#pragma unroll
+    for (int u = 0; u < kStepUnroll; ++u)
+      if (c[u] >= 0) x[u] = ld(X + (int64_t)c[u] * R + r);
+#pragma unroll
+    for (int u = 0; u < kStepUnroll; ++u) {
+      if (c[u] < 0) break;
+      yr += hr[u] * x[u].x;
+      yi += hr[u] * x[u].y;
+      if (VALC) {
+        yr -= hi[u] * x[u].y;
+        yi += hi[u] * x[u].x;
       }
-      Y[i * R + r] = y;
-      acc += (double)y.x * (double)y.x + (double)y.y * (double)y.y;
     }
   }
-  red[ti * blockDim.x + tr] = acc;
-  __syncthreads();
+  V y;
+  y.x = yr;
+  y.y = yi;
+  return y;
+}
+
+// Rows longer than this are split among kStepSplit threads per run.  The sectors' first rows (few
+// bath holes) are the long ones: 3045 of the 47 895 hold 43 % of the entries, about 65 each,
+// against 7 in the others, and one thread's chain of 65 gathers was the launch's length.
+constexpr int kStepHeavy = 24;
+constexpr int kStepSplit = 8;
+
+// Y = H X, per-block partials of Re<Y, X> per run into pa.  Thread (tr, ti) takes run tr of row
+// ti of the block's pass; consecutive rows go to different blocks (groups of `group` rows) so that
+// the long rows, neighbours in the basis, spread over all SMs.  The first row block also turns
+// the previous update's norm partials pb into beta[.][j - 1] (nothing else reads them).
+template <typename T, bool VALC>
+__global__ void __launch_bounds__(kStepMaxThreads, 2) step_spmm_kernel(int64_t n, const int64_t* __restrict__ rp,
+                                                        const int32_t* __restrict__ col, const T* __restrict__ vals,
+                                                        int R, int group, const typename Cx<T>::V* __restrict__ X,
+                                                        typename Cx<T>::V* __restrict__ Y, double* __restrict__ pa,
+                                                        const double* __restrict__ pb, double* __restrict__ beta,
+                                                        int K, int j, const int32_t* __restrict__ k_max,
+                                                        int32_t* status) {
+  using V = typename Cx<T>::V;
+  extern __shared__ double red[];
+  __shared__ int64_t heavy_row[kStepMaxThreads];
+  __shared__ int warp_heavy[kStepMaxThreads / 32];
+  __shared__ V part[kStepMaxThreads];
+  const int tr = threadIdx.x, ti = threadIdx.y, rb = blockDim.y;
+  const int tid = ti * blockDim.x + tr, lane = tid & 31, warp = tid >> 5;
+  const int r = blockIdx.y * blockDim.x + tr;
+  double acc = 0.0;
+  for (int64_t base = 0; base * gridDim.x < n; base += rb) {  // block-uniform
+    const int64_t lin = base + ti;
+    const int64_t i = (lin / group * gridDim.x + blockIdx.x) * group + lin % group;
+    int64_t e0 = 0, e1 = 0;
+    if (i < n) {
+      e0 = __ldg(rp + i);
+      e1 = __ldg(rp + i + 1);
+    }
+    const bool heavy = e1 - e0 > kStepHeavy;
+    if (i < n && !heavy && r < R) {
+      const V v = ld(X + i * R + r);
+      const V y = row_products<T, VALC>(e0, e1, 1, col, vals, R, r, X);
+      Y[i * R + r] = y;
+      acc += (double)y.x * (double)v.x + (double)y.y * (double)v.y;
+    }
+    // the pass's long rows, listed in thread order: kStepSplit threads per run and row, their
+    // parts added in a fixed order by the first of them
+    const bool mine = heavy && tr == 0;
+    const int nh = __syncthreads_count(mine);
+    if (nh == 0) continue;
+    const int in_warp = (int)(blockDim.x * blockDim.y) - 32 * warp;  // threads of this warp
+    const unsigned bal = __ballot_sync(in_warp >= 32 ? 0xffffffffu : (1u << in_warp) - 1u, mine);
+    if (lane == 0) warp_heavy[warp] = __popc(bal);
+    __syncthreads();
+    if (mine) {
+      int at = __popc(bal & ((1u << lane) - 1u));
+      for (int q = 0; q < warp; ++q) at += warp_heavy[q];
+      heavy_row[at] = i;
+    }
+    __syncthreads();
+    const int slots = rb / kStepSplit, slot = ti / kStepSplit, seg = ti % kStepSplit;
+    for (int h0 = 0; h0 < nh; h0 += slots) {
+      const bool on = slot < slots && h0 + slot < nh && r < R;
+      const int64_t ih = on ? heavy_row[h0 + slot] : 0;
+      if (on) part[tid] = row_products<T, VALC>(__ldg(rp + ih) + seg, __ldg(rp + ih + 1), kStepSplit, col, vals, R, r, X);
+      __syncthreads();
+      if (on && seg == 0) {
+        V y = part[tid];
+#pragma unroll
+        for (int q = 1; q < kStepSplit; ++q) {
+          const V p = part[tid + q * blockDim.x];
+          y.x += p.x;
+          y.y += p.y;
+        }
+        const V v = ld(X + ih * R + r);
+        Y[ih * R + r] = y;
+        acc += (double)y.x * (double)v.x + (double)y.y * (double)v.y;
+      }
+      __syncthreads();
+    }
+  }
+  const double s = tile_sum(acc, red);
+  if (ti == 0 && r < R) pa[(int64_t)blockIdx.x * R + r] = s;
+  if (blockIdx.x != 0 || j == 0) return;
+  const double bt = sqrt(tile_partials(pb, gridDim.x, R, r, red));
   if (ti == 0 && r < R) {
-    double s = 0.0;
-    for (int k = 0; k < (int)blockDim.y; ++k) s += red[k * blockDim.x + tr];
-    pbeta[(int64_t)blockIdx.x * R + r] = s;
+    beta[(int64_t)r * K + (j - 1)] = bt;
+    if (k_max[r] > j && !(bt > 0.0)) atomicExch(status, (int32_t)(bt == 0.0 ? EDGPU_ERR_BREAKDOWN : EDGPU_ERR_NAN));
   }
 }
 
-// beta_r = sqrt(sum partials); Vn = W / beta.
+// alpha_j and, unless it is the last step, w_{j+1} into the buffer of w_{j-1} with the per-block
+// partials of its squared norm.  nb: row blocks of the launch that wrote pa (and of this one
+// unless it is the last step's, which runs one row block per run tile).
+constexpr int kUpdateUnroll = 2;
+
 template <typename T>
-__global__ void normalize_kernel(int64_t n, int R, const typename Cx<T>::V* __restrict__ Wv,
-                                 typename Cx<T>::V* __restrict__ Vn, const double* __restrict__ pbeta, int nrb,
-                                 double* __restrict__ beta_out, int K, int j, const int32_t* __restrict__ k_max,
-                                 int32_t* status) {
+__global__ void __launch_bounds__(kStepMaxThreads, 2) step_update_kernel(int64_t n, int R, const typename Cx<T>::V* __restrict__ Y,
+                                                          const typename Cx<T>::V* __restrict__ Wc,
+                                                          typename Cx<T>::V* __restrict__ Wp,
+                                                          const double* __restrict__ pa, int nb,
+                                                          const double* __restrict__ beta, double* __restrict__ alpha,
+                                                          int K, int j, double* __restrict__ pb) {
   using V = typename Cx<T>::V;
-  __shared__ double beta_s[32];
+  extern __shared__ double red[];
+  __shared__ double coef[3][32];  // of y, w_j, w_{j-1}
   const int tr = threadIdx.x, ti = threadIdx.y;
   const int r = blockIdx.y * blockDim.x + tr;
-  if (ti == 0 && r < R) {
-    double s = 0.0;
-    for (int b = 0; b < nrb; ++b) s += pbeta[(int64_t)b * R + r];
-    const double bt = sqrt(s);
-    beta_s[tr] = bt;
-    if (blockIdx.x == 0) {
-      beta_out[(int64_t)r * K + j] = bt;
-      if (k_max[r] > j + 1 && !(bt > 0.0))
-        atomicExch(status, (int32_t)(bt == 0.0 ? EDGPU_ERR_BREAKDOWN : EDGPU_ERR_NAN));
+  double b1 = 1.0, i1 = 1.0, i2 = 1.0;  // beta_{j-1}, 1 / beta_{j-1}, 1 / beta_{j-2}; 1 where there is none
+  if (ti == 0 && r < R) {  // one warp divides, not the whole block
+    // a run whose beta was 0 has ended: its vector stays 0
+    if (j > 0) {
+      b1 = beta[(int64_t)r * K + (j - 1)];
+      i1 = b1 > 0.0 ? 1.0 / b1 : 0.0;
+    }
+    if (j > 1) {
+      const double b2 = beta[(int64_t)r * K + (j - 2)];
+      i2 = b2 > 0.0 ? 1.0 / b2 : 0.0;
     }
   }
-  __syncthreads();
-  if (r >= R) return;
-  const double beta = beta_s[tr];
-  const T inv = beta > 0.0 ? (T)(1.0 / beta) : (T)0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.y + ti; i < n; i += (int64_t)gridDim.x * blockDim.y) {
-    V w = Wv[i * R + r];
-    V o;
-    // one reciprocal per run and step: FP64 division is many times the cost of an FMA
-    o.x = w.x * inv;
-    o.y = w.y * inv;
-    Vn[i * R + r] = o;
+  // the thread's first elements are in flight while the partials are summed
+  const int64_t step = (int64_t)gridDim.x * blockDim.y;
+  const int64_t first = (int64_t)blockIdx.x * blockDim.y + ti;
+  V y[kUpdateUnroll], w[kUpdateUnroll], p[kUpdateUnroll];
+  auto fetch = [&](int64_t i0) {
+#pragma unroll
+    for (int u = 0; u < kUpdateUnroll; ++u) {
+      const int64_t i = i0 + u * step;
+      if (i < n) {
+        y[u] = ld(Y + i * R + r);
+        w[u] = ld(Wc + i * R + r);
+        if (j > 0) p[u] = Wp[i * R + r];
+      }
+    }
+  };
+  if (r < R && j + 1 < K) fetch(first);
+  const double sa = tile_partials(pa, nb, R, r, red);
+  if (ti == 0 && r < R) {
+    const double a = sa * i1 * i1;
+    if (blockIdx.x == 0) alpha[(int64_t)r * K + j] = a;
+    coef[0][tr] = i1;
+    coef[1][tr] = -a * i1;
+    coef[2][tr] = j > 0 ? -b1 * i2 : 0.0;
   }
+  if (j + 1 >= K) return;  // the same for the whole launch
+  __syncthreads();
+  double acc = 0.0;
+  if (r < R) {
+    const T cy = (T)coef[0][tr], cw = (T)coef[1][tr], cp = (T)coef[2][tr];
+    for (int64_t i0 = first; i0 < n; i0 += kUpdateUnroll * step) {
+      if (i0 != first) fetch(i0);
+#pragma unroll
+      for (int u = 0; u < kUpdateUnroll; ++u) {
+        const int64_t i = i0 + u * step;
+        if (i >= n) break;
+        T re = cy * y[u].x + cw * w[u].x, im = cy * y[u].y + cw * w[u].y;
+        if (j > 0) {
+          re += cp * p[u].x;
+          im += cp * p[u].y;
+        }
+        V o;
+        o.x = re;
+        o.y = im;
+        Wp[i * R + r] = o;
+        acc += (double)re * (double)re + (double)im * (double)im;
+      }
+    }
+  }
+  const double s = tile_sum(acc, red);
+  if (ti == 0 && r < R) pb[(int64_t)blockIdx.x * R + r] = s;
 }
 
 __global__ void to_c64_kernel(const double2* in, float2* out, int64_t n) {
@@ -644,14 +838,14 @@ int spmv_impl(const edgpu_csr* h, const typename Cx<T>::V* x, typename Cx<T>::V*
 }
 
 // Optional per-kernel timing with CUDA events on the launching stream: kernel_ms[0..2] receive
-// the summed durations of the SpMM, axpy/beta and normalise launches (host array).
+// the summed durations of the SpMM and the update launches (host array; [2] is 0).
 struct KernelTimer {
   double* out;
-  std::vector<cudaEvent_t> ev[3];
+  std::vector<cudaEvent_t> ev[2];
   cudaStream_t s;
   KernelTimer(double* o, int K, cudaStream_t st) : out(o), s(st) {
     if (!out) return;
-    for (int k = 0; k < 3; ++k) {
+    for (int k = 0; k < 2; ++k) {
       ev[k].resize(2 * (size_t)K);
       for (auto& e : ev[k]) cudaEventCreate(&e);
     }
@@ -661,17 +855,17 @@ struct KernelTimer {
   }
   void finish(int K) {
     if (!out) return;
-    for (int k = 0; k < 3; ++k) {
+    out[2] = 0.0;
+    for (int k = 0; k < 2; ++k) {
       double tot = 0.0;
       for (int j = 0; j < K; ++j) {
-        if (k == 2 && j == K - 1) continue;
         float ms = 0.f;
         cudaEventSynchronize(ev[k][2 * (size_t)j + 1]);
         if (cudaEventElapsedTime(&ms, ev[k][2 * (size_t)j], ev[k][2 * (size_t)j + 1]) == cudaSuccess) tot += ms;
       }
       out[k] = tot;
     }
-    for (int k = 0; k < 3; ++k)
+    for (int k = 0; k < 2; ++k)
       for (auto& e : ev[k]) cudaEventDestroy(e);
   }
 };
@@ -682,7 +876,7 @@ int lanczos_impl(const edgpu_csr* h, const double* v0, int R, const int32_t* k_m
   using V = typename Cx<T>::V;
   const int64_t n = h->n;
   const int64_t nv = n * (int64_t)R;
-  RunTile t = make_tile(n, R);
+  const RunTile t = make_step_tile(n, R);  // no more row blocks than the workspace was sized for
   size_t off = 0;
   auto carve = [&](size_t bytes) {
     unsigned char* p = ws + off;
@@ -715,30 +909,29 @@ int lanczos_impl(const edgpu_csr* h, const double* v0, int R, const int32_t* k_m
     vals = (const T*)(valc ? (const void*)h->val_cf : (const void*)h->val_rf);
   }
   if (!vals) return EDGPU_ERR_ARG;
-  V* Vc = A;
-  V* Vp = B;
+  V* Wc = A;
+  V* Wp = B;
+  // one pass over the rows: single rows dealt to the blocks; several: groups of 8, so that the
+  // CSR of neighbouring rows is read by one block
+  const int group = (int64_t)t.nrb * t.rb >= n ? 1 : 8;
   KernelTimer timer(kernel_ms, K, s);
   for (int j = 0; j < K; ++j) {
     timer.mark(0, j, 0);
     if (valc)
-      spmm_alpha_kernel<T, true><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, Vc, Wb, pa, 1);
+      step_spmm_kernel<T, true><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, group, Wc, Wb, pa, pb, beta, K, j,
+                                                         k_max, status);
     else
-      spmm_alpha_kernel<T, false><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, Vc, Wb, pa, 1); note_launch();
+      step_spmm_kernel<T, false><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, group, Wc, Wb, pa, pb, beta, K, j,
+                                                          k_max, status);
+    note_launch();
     timer.mark(0, j, 1);
     timer.mark(1, j, 0);
-    axpy_beta_kernel<T><<<grid, block, red, s>>>(n, R, Wb, Vc, j > 0 ? Vp : nullptr, pa, t.nrb,
-                                                 j > 0 ? beta : nullptr, alpha, K, j, pb); note_launch();
+    const dim3 ugrid(j + 1 < K ? t.nrb : 1, t.nrt);  // the last step only adds up alpha
+    step_update_kernel<T><<<ugrid, block, red, s>>>(n, R, Wb, Wc, Wp, pa, t.nrb, beta, alpha, K, j, pb);
+    note_launch();
     timer.mark(1, j, 1);
-    if (j + 1 < K) {
-      timer.mark(2, j, 0);
-      normalize_kernel<T><<<grid, block, 0, s>>>(n, R, Wb, Vp, pb, t.nrb, beta, K, j, k_max, status);
-      note_launch();
-      timer.mark(2, j, 1);
-    }
     if ((rc = check_launch())) return rc;
-    V* tmp = Vc;
-    Vc = Vp;
-    Vp = tmp;
+    std::swap(Wc, Wp);
   }
   timer.finish(K);
   return EDGPU_OK;

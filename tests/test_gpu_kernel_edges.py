@@ -1,0 +1,74 @@
+"""Kernels at the sizes where their tiles, remainders and dispatch rules change."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _random_csr(eng, n, seed, complex_vals=False, heavy=()):
+    """Hermitian CSR with 2-9 entries a row, rows of ``heavy`` linked to 40 others each."""
+    from impuritymodel_gb300.engine import CsrMatrix
+
+    rng = np.random.default_rng(seed)
+    h = {}
+    for i in range(n):
+        h[(i, i)] = complex(rng.normal() * 3.0)
+        for j in rng.integers(0, n, size=40 if i in heavy else 2):
+            if i != j:
+                v = complex(rng.normal(), rng.normal() if complex_vals else 0.0)
+                h[(i, int(j))] = v
+                h[(int(j), i)] = v.conjugate()
+    keys = sorted(h)
+    rows = np.array([k[0] for k in keys])
+    col = torch.tensor([k[1] for k in keys], dtype=torch.int32, device=eng.device)
+    vals = np.array([h[k] for k in keys])
+    rp = torch.from_numpy(np.searchsorted(rows, np.arange(n + 1)).astype(np.int64)).to(eng.device)
+    if complex_vals:
+        csr = CsrMatrix(rp, col, val_c=torch.from_numpy(np.stack([vals.real, vals.imag], 1)).to(eng.device).contiguous())
+    else:
+        csr = CsrMatrix(rp, col, val_r=torch.from_numpy(np.ascontiguousarray(vals.real)).to(eng.device))
+    import scipy.sparse
+
+    return csr, scipy.sparse.csr_matrix((vals, (rows, [k[1] for k in keys])), shape=(n, n))
+
+
+def _recurrence(H, v, K):
+    """Upstream's three-term recurrence in NumPy (finite.py:1974-1992)."""
+    alpha, beta = [], []
+    p, bp = np.zeros_like(v), 0.0
+    for _ in range(K):
+        y = H @ v
+        a = np.vdot(v, y).real
+        w = y - a * v - bp * p
+        alpha.append(a)
+        bp = np.linalg.norm(w)
+        beta.append(bp)
+        p, v = v, w / bp
+    return np.array(alpha), np.array(beta)
+
+
+@pytest.mark.parametrize("n,R,K,precision,cplx", [
+    (4300, 1, 12, 0, False),    # 256-thread blocks, one run
+    (4300, 33, 12, 0, False),   # two run tiles, the second of one run
+    (9000, 31, 3, 0, True),     # a run tile that does not divide the block
+    (40011, 3, 12, 0, False),   # 512-thread blocks, one pass, a ragged last row
+    (40011, 7, 12, 1, True),    # complex64 vectors and values
+    (12000, 16, 1, 0, False),   # a single step: alpha only
+    (12000, 16, 2, 1, False),
+])
+def test_grid_wide_lanczos(eng, n, R, K, precision, cplx):
+    csr, H = _random_csr(eng, n, n + R, cplx, heavy=(0, 1, 2, 5, n // 2, n - 1))
+    g = np.random.default_rng(R)
+    v = g.normal(size=(n, R)) + 1j * g.normal(size=(n, R))
+    v /= np.linalg.norm(v, axis=0)
+    k = np.full(R, K, dtype=np.int32)
+    a, b = eng.lanczos(csr, torch.from_numpy(v).to(eng.device), k, precision=precision)
+    a, b = a.cpu().numpy(), b.cpu().numpy()
+    # a dozen steps of an unconverged recurrence amplify rounding by less than 1e3
+    tol = (1e-12 if precision == 0 else 6e-5) * abs(H).sum(1).max()
+    for r in {0, R // 2, R - 1}:
+        ar, br = _recurrence(H, v[:, r], K)
+        assert np.abs(a[r] - ar).max() < tol
+        assert np.abs(b[r, : K - 1] - br[: K - 1]).max(initial=0.0) < tol

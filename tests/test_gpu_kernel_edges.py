@@ -72,3 +72,40 @@ def test_grid_wide_lanczos(eng, n, R, K, precision, cplx):
         ar, br = _recurrence(H, v[:, r], K)
         assert np.abs(a[r] - ar).max() < tol
         assert np.abs(b[r, : K - 1] - br[: K - 1]).max(initial=0.0) < tol
+
+
+def _fraction(alpha, beta, k, omega, delta, e, scale):
+    """The continued fraction of upstream's getGreen (spectra.py:678-680), from its end."""
+    g = np.zeros((len(k), len(omega)), dtype=np.complex128)
+    for r, kl in enumerate(k):
+        x = np.zeros(len(omega), dtype=np.complex128)
+        for i in range(kl - 1, -1, -1):
+            d = omega + e[r] + 1j * delta - alpha[r, i]
+            x = 1.0 / (d - (beta[r, i] ** 2 * x if i != kl - 1 else 0.0))
+        g[r] = scale[r] * x
+    return g
+
+
+@pytest.mark.parametrize("R,K,nw,delta", [
+    (1, 1, 1, 0.1),         # one coefficient, one frequency
+    (5, 7, 3, -0.2),        # several runs a block, negative broadening, ragged lengths
+    (130, 9, 1, 0.05),      # more runs than a block holds
+    (3, 150, 129, 0.05),    # a second tile of one frequency
+    (2, 1030, 200, 0.05),   # more coefficients than one stage holds
+    (4, 60, 100, 1e-11),    # below the scaled form's smallest broadening
+    (4, 400, 64, 40.0),     # a broadening far above the spread of the coefficients
+])
+def test_continued_fraction(eng, R, K, nw, delta):
+    g = np.random.default_rng(K + nw)
+    alpha = -700.0 + 5.0 * g.normal(size=(R, K))
+    beta = 0.1 + 6.0 * g.random((R, K))
+    k = g.integers(1, K + 1, size=R).astype(np.int32)
+    k[0] = K
+    beta[np.arange(R), k - 1] = np.nan  # no part of the fraction
+    omega, e, scale = np.linspace(-8.0, 9.0, nw), -700.0 + g.random(R), 0.5 + g.random(R)
+    to = lambda x: torch.from_numpy(x).to(eng.device)  # noqa: E731
+    got = eng.cfrac(to(alpha), to(beta), k, omega, delta, e, scale).cpu().numpy()
+    want = _fraction(alpha, beta, k, omega, delta, e, scale)
+    # NumPy rounds omega + e at 700 eV (1.1e-13); a pole of width delta turns that into 1.1e-13 / delta
+    tol = 1e-12 + (4e-13 / abs(delta) if abs(delta) > 1e-9 else 1e-6)
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()

@@ -151,6 +151,7 @@ SIGNATURES = {
     "edgpu_gemm_tile_width": (_I, [_I, _I]),
     "edgpu_mlp_bits": (_I, [_P, _I, _I64, _I, _P, _P, _P]),
     "edgpu_mlp_head": (_I, [_P, _P, _P, _I64, _I, _P, _P]),
+    "edgpu_mlp_rank": (_I, [_P, _I, _I64, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "edgpu_mlp_head_backward": (_I, [_P, _P, _P, _P, _I64, _I, _P, _P, _P, _P]),
     "edgpu_mlp_row_dot": (_I, [_P, _I, _I64, _P, _P, _P]),
     "edgpu_mlp_adam": (_I, [_P, _P, _P, _P, _I64, C.c_float, C.c_float, C.c_float, C.c_float, _P]),

@@ -487,6 +487,347 @@ __global__ void mlp_to_bf16_kernel(const float* __restrict__ Wf, int rows, int c
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// Ranking states: the whole network in one launch, occupation words in, scores out.
+//
+// Layer by layer, ranking 462 120 states moved 2.2 GB through memory (the BF16 occupation matrix
+// written and read, both hidden layers written and read) for 18 MB of states and 2 MB of scores:
+// 0.86 ms, a third of it the expansion of bits into BF16.  Here a CTA takes tiles of 128 states (two
+// at a time when there are more tiles than SMs) and nothing but the words, the weights and the
+// scores crosses global memory:
+//   * the threads expand each state's words into a row of the A operand in shared memory (one
+//     word is one 64-column K tile; four bits at a time from a 16-entry table); the fifth K tile
+//     takes the first one's place once that has been read, so that A and two weight tiles fit;
+//   * the weights stream through a two-stage ring of K tiles (bulk-tensor copies, 32 KiB each),
+//     each tile feeding the MMAs of both state tiles;
+//   * the first layer's accumulator (tensor memory, 256 columns a tile) is read back, bias, ReLU,
+//     BF16, into the same A buffer as layer two's operand;
+//   * layer two's accumulator is read back, and the head's sum runs in the threads.
+// The BF16 roundings and the order of the K steps are those of the layer-by-layer kernels; the
+// head's FP32 sum runs in another order.  Time for 462 120 states: 0.86 -> 0.145 ms.  Bound: the
+// phases of a pass follow one another (expansion 1.7k cycles, layer one 6.7k, epilogue, layer two
+// 5.3k, epilogue; the MMAs alone 9.2k).  With 8 epilogue warps and the biases read through L1 the
+// epilogues took 4.7k and 7-9k cycles; 16 warps with the biases in shared memory took 0.03 ms off.
+// A third weight stage (in the room of the biases) gained nothing.
+// Every wait has an iteration limit, as in the GEMM above.
+// ---------------------------------------------------------------------------------------
+constexpr int kRankIn = 320, kRankHidden = 256;
+constexpr int kRankChunks1 = kRankIn / kBK, kRankChunks2 = kRankHidden / kBK;
+constexpr int kRankEpiThreads = 512;                    // 16 warps
+constexpr int kRankThreads = kRankEpiThreads + 64;      // + producer warp + MMA warp
+constexpr int kRankMmaWarp = kRankEpiThreads / 32;
+constexpr int kRankQuarter = kRankHidden / 4;           // columns of an epilogue thread
+constexpr uint32_t kRankABytes = kBM * kBK * 2;         // one K tile of 128 states: 16 KiB
+constexpr uint32_t kRankTileBytes = kRankChunks2 * kRankABytes;  // the fifth K tile follows the first in its place
+constexpr uint32_t kRankStageBytes = kRankHidden * kBK * 2;
+constexpr int kRankStages = 2;
+constexpr size_t kRankSmem = 2 * (size_t)kRankTileBytes + kRankStages * (size_t)kRankStageBytes + 1024;
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* m) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(m)) : "memory");
+}
+
+// Shared-memory writes of this thread become visible to the tensor core and the copy engine.
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// 16 consecutive FP32 columns of this thread's tensor-memory lane; the registers hold them after
+// tmem_wait_ld.
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+
+// Ties the registers of earlier loads to the wait, so that nothing reads them before it.
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16], uint32_t (&s)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int q = 0; q < 16; ++q) asm volatile("" : "+r"(r[q]), "+r"(s[q]));
+}
+
+// relu(v + b) of two columns as a BF16 pair.  The maximum is taken after the rounding (monotone, so
+// the same value) to work on both at once; like fmaxf it makes a NaN 0.
+__device__ __forceinline__ __nv_bfloat162 bias_relu2(uint32_t v0, uint32_t v1, float b0, float b1) {
+  const float2 x = __fadd2_rn(make_float2(__uint_as_float(v0), __uint_as_float(v1)), make_float2(b0, b1));
+  return __hmax2(__floats2bfloat162_rn(x.x, x.y), __float2bfloat162_rn(0.0f));
+}
+
+struct RankArgs {
+  const uint64_t* states;  // [n][W]
+  int W;
+  int64_t n;
+  const float *b1, *b2, *w3, *b3;
+  float* y;
+  int tiles;        // 128-state tiles per pass of a CTA: 1 or 2
+  int64_t passes;   // over the whole launch
+  int32_t* status;
+};
+
+__global__ void __launch_bounds__(kRankThreads, 1)
+    mlp_rank_kernel(const __grid_constant__ CUtensorMap w1map, const __grid_constant__ CUtensorMap w2map, RankArgs g) {
+  extern __shared__ unsigned char sm[];
+  __shared__ uint64_t full[kRankStages], empty[kRankStages], a_full, acc_full, first_read, last_full, quarter_sums, drained;
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed;
+  __shared__ uint2 nibble[16];
+  __shared__ float part[3][2 * kBM];
+  __shared__ __align__(16) float sb1[kRankHidden], sb2[kRankHidden], sw3[kRankHidden];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t abuf = (smem_u32(sm) + 1023u) & ~1023u;
+  const uint32_t ring = abuf + 2 * kRankTileBytes;
+  if (warp == kRankMmaWarp)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                 "r"(512u)
+                 : "memory");
+  if (tid == 0) {
+    for (int s = 0; s < kRankStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(&a_full, kRankEpiThreads);
+    mbar_init(&acc_full, 1);
+    mbar_init(&first_read, 1);
+    mbar_init(&last_full, kRankEpiThreads);
+    mbar_init(&quarter_sums, kRankEpiThreads / 4 * 3);
+    mbar_init(&drained, 1);
+    failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid < 16)  // four occupation bits, first column in the highest, as four BF16
+    nibble[tid] = make_uint2(((tid & 8) ? 0x3F80u : 0u) | ((tid & 4) ? 0x3F800000u : 0u),
+                             ((tid & 2) ? 0x3F80u : 0u) | ((tid & 1) ? 0x3F800000u : 0u));
+  for (int k = tid; k < kRankHidden; k += kRankThreads) {
+    sb1[k] = g.b1[k];
+    sb2[k] = g.b2[k];
+    sw3[k] = g.w3[k];
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base;
+  volatile int* gave_up = &failed;
+  if (warp == kRankMmaWarp + 1) {
+    if (lane == 0) {
+      // producer: the K tiles of W1 then W2 for every pass
+      int64_t it = 0;
+      bool ok = true;
+      for (int64_t p = blockIdx.x; ok && p < g.passes; p += gridDim.x) {
+        for (int c = 0; c < kRankChunks1 + kRankChunks2; ++c, ++it) {
+          const int s = (int)(it % kRankStages);
+          if (it >= kRankStages && !mbar_wait(&empty[s], (uint32_t)(it / kRankStages - 1) & 1u)) ok = false;
+          if (!ok || *gave_up) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&full[s], kRankStageBytes);
+          const bool first = c < kRankChunks1;
+          tma_load_2d(ring + (uint32_t)s * kRankStageBytes, first ? &w1map : &w2map,
+                      (first ? c : c - kRankChunks1) * kBK, 0, &full[s]);
+        }
+      }
+      if (!ok) atomicExch(&failed, 1);
+      // every copy issued has landed before the CTA may exit
+      for (int64_t t = it > kRankStages ? it - kRankStages : 0; t < it; ++t)
+        mbar_wait(&full[t % kRankStages], (uint32_t)(t / kRankStages) & 1u);
+    }
+    __syncwarp();
+  } else if (warp == kRankMmaWarp) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16(kBM, kRankHidden);
+      int64_t it = 0;
+      uint32_t pass_phase = 0;
+      bool ok = true;
+      for (int64_t p = blockIdx.x; ok && p < g.passes; p += gridDim.x, pass_phase ^= 1u) {
+        for (int layer = 0; ok && layer < 2; ++layer) {
+          // the A operand is written and the accumulator's last contents have been read
+          if (!mbar_wait(&a_full, (uint32_t)layer)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const int chunks = layer ? kRankChunks2 : kRankChunks1;
+          for (int c = 0; c < chunks; ++c, ++it) {
+            const int s = (int)(it % kRankStages);
+            if (!mbar_wait(&full[s], (uint32_t)(it / kRankStages) & 1u) ||
+                (c == kRankChunks2 && !mbar_wait(&last_full, pass_phase))) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t b = ring + (uint32_t)s * kRankStageBytes;
+            for (int q = 0; q < g.tiles; ++q) {
+              const uint32_t a = abuf + (uint32_t)q * kRankTileBytes + (uint32_t)(c % kRankChunks2) * kRankABytes;
+#pragma unroll
+              for (int k16 = 0; k16 < kBK / 16; ++k16)
+                mma_bf16(tmem + (uint32_t)(q * kRankHidden), smem_desc_sw128(a + (uint32_t)k16 * 32u),
+                         smem_desc_sw128(b + (uint32_t)k16 * 32u), idesc, (c > 0 || k16 > 0) ? 1u : 0u);
+            }
+            mma_commit(&empty[s]);
+            if (layer == 0 && c == 0) mma_commit(&first_read);
+          }
+          if (ok) mma_commit(&acc_full);
+        }
+      }
+      if (!ok) atomicExch(&failed, 1);
+      // no MMA is in flight when the tensor memory is freed
+      mma_commit(&drained);
+      if (!mbar_wait(&drained, 0u)) atomicExch(&failed, 1);
+    }
+    __syncwarp();
+  } else {
+    // Expansion: threads tid and tid + 256 write state tid of the pass.  Epilogues: the thread reads
+    // its warp's tensor-memory lane (a state of each tile) in 64 of the 256 columns, so that a bias
+    // value is loaded once for two states, and four warps a scheduler hide the loads' latency.
+    const int row = ((warp & 3) << 5) + lane, quarter = warp >> 2;
+    const int xs = tid & (2 * kBM - 1), xhalf = tid / (2 * kBM);
+    const uint32_t xrow = abuf + (uint32_t)(xs / kBM) * kRankTileBytes + (uint32_t)(xs % kBM) * 128u;
+    const uint32_t hrow = abuf + (uint32_t)row * 128u + (uint32_t)quarter * kRankABytes;
+    const uint32_t sw = (uint32_t)(row & 7), xsw = (uint32_t)(xs & 7);
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(quarter * kRankQuarter);
+    const bool two = g.tiles == 2;
+    uint32_t pass_phase = 0;
+    bool ok = true;
+    uint64_t words[3];  // two K tiles and the shared fifth of the thread's state, loaded a pass ahead
+    auto fetch = [&](int64_t p) {
+      const int64_t i = p * g.tiles * kBM + xs;
+      const bool on = xs < g.tiles * kBM && p < g.passes && i < g.n;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int c = k < 2 ? 2 * xhalf + k : kRankChunks2;
+        words[k] = on && c < g.W ? __ldg(g.states + i * g.W + c) : 0ull;
+      }
+    };
+    // byte q of the word, from the top, is piece `piece` (16 bytes, eight columns) of the K tile
+    auto expand = [&](uint64_t word, int q, int chunk, int piece) {
+      const uint2 h = nibble[(word >> (60 - 8 * q)) & 15u], l = nibble[(word >> (56 - 8 * q)) & 15u];
+      st_shared_v4(xrow + (uint32_t)chunk * kRankABytes + ((((uint32_t)piece) ^ xsw) << 4), h.x, h.y, l.x, l.y);
+    };
+    fetch(blockIdx.x);
+    for (int64_t p = blockIdx.x; ok && p < g.passes; p += gridDim.x, pass_phase ^= 1u) {
+      const int64_t base = p * g.tiles * kBM;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) expand(words[q >> 3], q & 7, 2 * xhalf + (q >> 3), q & 7);
+      fence_async_smem();
+      tc_fence_before();
+      mbar_arrive(&a_full);
+      // the fifth K tile takes the first one's place once the MMAs have read that
+      ok = __all_sync(0xffffffffu, mbar_wait(&first_read, pass_phase) && !*gave_up);
+      if (!ok) break;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) expand(words[2] << (32 * xhalf), q, 0, q + 4 * xhalf);
+      fence_async_smem();
+      mbar_arrive(&last_full);
+      fetch(p + gridDim.x);
+      // one answer for the warp: its tensor-memory loads are collective
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full, 0u) && !*gave_up);
+      if (!ok) break;
+      tc_fence_after();
+      for (int c0 = 0; c0 < kRankQuarter; c0 += 16) {
+        uint32_t v[16], u[16];
+        tmem_ld16_async(trow + (uint32_t)c0, v);
+        if (two) tmem_ld16_async(trow + (uint32_t)(kRankHidden + c0), u);
+        tmem_wait_ld(v, u);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float4* bias = reinterpret_cast<const float4*>(sb1 + quarter * kRankQuarter + c0 + 8 * q);
+          const float4 bl = bias[0], bh = bias[1];
+          const float bb[8] = {bl.x, bl.y, bl.z, bl.w, bh.x, bh.y, bh.z, bh.w};
+          const uint32_t at = hrow + (((uint32_t)(c0 / 8 + q) ^ sw) << 4);
+          uint32_t pk[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const __nv_bfloat162 h = bias_relu2(v[8 * q + 2 * k], v[8 * q + 2 * k + 1], bb[2 * k], bb[2 * k + 1]);
+            pk[k] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+          st_shared_v4(at, pk[0], pk[1], pk[2], pk[3]);
+          if (two) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const __nv_bfloat162 h = bias_relu2(u[8 * q + 2 * k], u[8 * q + 2 * k + 1], bb[2 * k], bb[2 * k + 1]);
+              pk[k] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            st_shared_v4(at + kRankTileBytes, pk[0], pk[1], pk[2], pk[3]);
+          }
+        }
+      }
+      fence_async_smem();
+      tc_fence_before();
+      mbar_arrive(&a_full);
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full, 1u) && !*gave_up);
+      if (!ok) break;
+      tc_fence_after();
+      // head: eight partial sums a state in packed pairs, added up, then the four quarters
+      float2 s[4], z[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s[k] = z[k] = make_float2(0.0f, 0.0f);
+      for (int c0 = 0; c0 < kRankQuarter; c0 += 16) {
+        uint32_t v[16], u[16];
+        tmem_ld16_async(trow + (uint32_t)c0, v);
+        if (two) tmem_ld16_async(trow + (uint32_t)(kRankHidden + c0), u);
+        tmem_wait_ld(v, u);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int at = quarter * kRankQuarter + c0 + 4 * q, k = 2 * (q & 1);
+          const float4 b = *reinterpret_cast<const float4*>(sb2 + at), w = *reinterpret_cast<const float4*>(sw3 + at);
+          const float2 w01 = make_float2(w.x, w.y), w23 = make_float2(w.z, w.w);
+          s[k] = __ffma2_rn(__bfloat1622float2(bias_relu2(v[4 * q], v[4 * q + 1], b.x, b.y)), w01, s[k]);
+          s[k + 1] = __ffma2_rn(__bfloat1622float2(bias_relu2(v[4 * q + 2], v[4 * q + 3], b.z, b.w)), w23, s[k + 1]);
+          if (two) {
+            z[k] = __ffma2_rn(__bfloat1622float2(bias_relu2(u[4 * q], u[4 * q + 1], b.x, b.y)), w01, z[k]);
+            z[k + 1] = __ffma2_rn(__bfloat1622float2(bias_relu2(u[4 * q + 2], u[4 * q + 3], b.z, b.w)), w23, z[k + 1]);
+          }
+        }
+      }
+      const float2 ss = __fadd2_rn(__fadd2_rn(s[0], s[1]), __fadd2_rn(s[2], s[3]));
+      const float2 zz = __fadd2_rn(__fadd2_rn(z[0], z[1]), __fadd2_rn(z[2], z[3]));
+      if (quarter > 0) {
+        part[quarter - 1][row] = ss.x + ss.y;
+        part[quarter - 1][kBM + row] = zz.x + zz.y;
+        mbar_arrive(&quarter_sums);
+      } else {
+        ok = mbar_wait(&quarter_sums, pass_phase);
+        const float b3 = __ldg(g.b3);
+        if (base + row < g.n) g.y[base + row] = ((ss.x + ss.y) + part[0][row]) + (part[1][row] + part[2][row]) + b3;
+        if (two && base + kBM + row < g.n)
+          g.y[base + kBM + row] =
+              ((zz.x + zz.y) + part[0][kBM + row]) + (part[1][kBM + row] + part[2][kBM + row]) + b3;
+      }
+      // the next pass writes part only after the first quarter has arrived on a_full again
+    }
+    if (!ok) atomicExch(&failed, 1);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (failed && tid == 0) atomicExch(g.status, (int32_t)EDGPU_ERR_NOCONV);
+  if (warp == kRankMmaWarp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+}
+
+int mlp_rank(const RankArgs& args, const __nv_bfloat16* W1, const __nv_bfloat16* W2, cudaStream_t s) {
+  RankArgs g = args;
+  alignas(64) CUtensorMap w1map, w2map;
+  if (!gemm_operand_map(&w1map, W1, kRankIn, kRankHidden, kRankHidden) ||
+      !gemm_operand_map(&w2map, W2, kRankHidden, kRankHidden, kRankHidden))
+    return EDGPU_ERR_CUDA;
+  const int64_t tiles = (g.n + kBM - 1) / kBM;
+  // two tiles a pass share each weight tile; with no more tiles than SMs one each is faster
+  g.tiles = tiles > grid_cap() ? 2 : 1;
+  g.passes = (tiles + g.tiles - 1) / g.tiles;
+  if (cudaFuncSetAttribute(mlp_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRankSmem) != cudaSuccess)
+    return EDGPU_ERR_CUDA;
+  const unsigned grid = (unsigned)(g.passes < grid_cap() ? g.passes : grid_cap());
+  mlp_rank_kernel<<<grid, kRankThreads, kRankSmem, s>>>(w1map, w2map, g);
+  note_launch();
+  return check_launch();
+}
+
 inline unsigned mlp_grid(int64_t n, int threads) {
   int64_t b = (n + threads - 1) / threads;
   const int64_t cap = (int64_t)grid_cap() * 8;
@@ -530,6 +871,26 @@ extern "C" int edgpu_mlp_head(const void* H, const float* w3, const float* b3, i
       reinterpret_cast<const __nv_bfloat16*>(H), w3, b3, B, n_h, y);
   note_launch();
   return check_launch();
+}
+
+extern "C" int edgpu_mlp_rank(const uint64_t* states, int W, int64_t n, int n_in, int n_h, const void* W1,
+                              const float* b1, const void* W2, const float* b2, const float* w3, const float* b3,
+                              float* y, int32_t* status_dev, void* stream) {
+  if (!states || W < 1 || n < 1 || !W1 || !b1 || !W2 || !b2 || !w3 || !b3 || !y || !status_dev) return EDGPU_ERR_ARG;
+  if (n_in != kRankIn || n_h != kRankHidden) return EDGPU_ERR_ARG;
+  if (!aligned16(W1) || !aligned16(W2)) return EDGPU_ERR_ARG;
+  RankArgs g{};
+  g.states = states;
+  g.W = W;
+  g.n = n;
+  g.b1 = b1;
+  g.b2 = b2;
+  g.w3 = w3;
+  g.b3 = b3;
+  g.y = y;
+  g.status = status_dev;
+  return mlp_rank(g, reinterpret_cast<const __nv_bfloat16*>(W1), reinterpret_cast<const __nv_bfloat16*>(W2),
+                  (cudaStream_t)stream);
 }
 
 extern "C" int edgpu_mlp_head_backward(const void* H, const float* y, const float* target, const float* w3,

@@ -165,16 +165,17 @@ class BasisNet:
         return losses
 
     def predict(self, states):
-        """Predicted log10 weights of padded states [N, WORDS] (any N)."""
-        n = states.shape[0]
-        nb = ((n + ROWS - 1) // ROWS) * ROWS
-        if nb != n:
-            pad = torch.zeros((nb - n, states.shape[1]), dtype=states.dtype, device=states.device)
-            states = torch.cat([states, pad], 0)
-        X, _ = self.inputs(states.contiguous())
-        y, _ = self.forward(X)
-        self.eng.read_status("mlp inference")
-        return y[:n]
+        """Predicted log10 weights of padded states [N, WORDS] (any N): the whole network in one
+        launch (:meth:`forward` on :meth:`inputs`, the head summed in another order)."""
+        e, p = self.eng, self.p
+        states = states.contiguous()
+        n, w = states.shape
+        y = torch.empty(n, dtype=torch.float32, device=e.device)
+        L.check(self._lib().edgpu_mlp_rank(_ptr(states), w, n, N_IN, N_H, _ptr(self.W1b), _ptr(p["b1"]), _ptr(self.W2b),
+                                           _ptr(p["b2"]), _ptr(p["w3"]), _ptr(p["b3"]), _ptr(y), _ptr(e.status),
+                                           e.stream), "mlp_rank")
+        e.read_status("mlp inference")
+        return y
 
 
 def ground_state_samples(eng, models, n_states=1, k_start=120):

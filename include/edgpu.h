@@ -527,6 +527,14 @@ int edgpu_gemm_bf16_epi(int epi, const void* A, const void* B, int M, int N, int
 int edgpu_mlp_bits(const uint64_t* states, int W, int64_t B, int n_in, void* X, void* Xt, void* stream);
 /* y[b] = sum_j H[b][j] w3[j] + b3[0] (H BF16 [B][n_h]). */
 int edgpu_mlp_head(const void* H, const float* w3, const float* b3, int64_t B, int n_h, float* y, void* stream);
+/* y[i] = the whole network's score of states [n][W] (occupation words, spin-orbitals beyond n_in
+ * ignored) in one launch: BF16 weights W1 [n_h][n_in] and W2 [n_h][n_h], FP32 biases b1, b2, head
+ * w3 [n_h], b3 [1]; hidden layers rounded to BF16 as edgpu_gemm_bf16_epi stores them.  n_in = 320 and
+ * n_h = 256 only; W1 and W2 16-byte aligned.
+ */
+int edgpu_mlp_rank(const uint64_t* states, int W, int64_t n, int n_in, int n_h, const void* W1, const float* b1,
+                   const void* W2, const float* b2, const float* w3, const float* b3, float* y, int32_t* status_dev,
+                   void* stream);
 /* Mean-squared-error head backward: dy = 2 (y - target) / B, dH = dy w3 masked by H > 0
  * (BF16 [B][n_h] and its transpose dHt). */
 int edgpu_mlp_head_backward(const void* H, const float* y, const float* target, const float* w3, int64_t B, int n_h,

@@ -109,3 +109,30 @@ def test_continued_fraction(eng, R, K, nw, delta):
     # NumPy rounds omega + e at 700 eV (1.1e-13); a pole of width delta turns that into 1.1e-13 / delta
     tol = 1e-12 + (4e-13 / abs(delta) if abs(delta) > 1e-9 else 1e-6)
     assert np.abs(got - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n,words", [
+    (1, 5), (127, 5), (129, 5),        # one tile, a ragged one, a second of one state
+    (130, 2), (300, 7),                # fewer and more words than the network reads
+    (152 * 128, 5), (152 * 128 + 1, 5),  # one tile a CTA, then two
+    (100001, 5),
+])
+def test_rank_in_one_launch(eng, n, words):
+    from impuritymodel_gb300.pruning import BasisNet, pad_words
+
+    net = BasisNet(eng, seed=n)
+    g = torch.Generator(device=eng.device)
+    g.manual_seed(n)
+    net.p["b1"].copy_(torch.randn(256, device=eng.device, generator=g))
+    net.p["b2"].copy_(torch.randn(256, device=eng.device, generator=g))
+    states = torch.randint(-(1 << 62), 1 << 62, (n, words), device=eng.device, generator=g) * 2
+    states[:, -1] |= 1  # the last column of the last word
+    got = net.predict(states)
+    # layer by layer: the same roundings and K order, the head's 256 products summed in another order
+    # (at most 14 roundings deep there, 22 here)
+    pad = (-n) % 128
+    X, _ = net.inputs(torch.cat([pad_words(states), states.new_zeros((pad, 5))], 0))
+    want, (_, _, H2, _) = net.forward(X)
+    bound = 36 * 2.0 ** -24 * (H2.double().abs() @ net.p["w3"].double().abs() + net.p["b3"].double().abs())
+    assert got.shape == (n,)
+    assert bool(((got.double() - want[:n].double()).abs() <= bound[:n]).all())

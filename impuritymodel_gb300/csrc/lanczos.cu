@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kStepMaxThreads, 2) step_spmm_kernel(int64_t n
   const int tid = ti * blockDim.x + tr, lane = tid & 31, warp = tid >> 5;
   const int r = blockIdx.y * blockDim.x + tr;
   double acc = 0.0;
-  for (int64_t base = 0; base * gridDim.x < n; base += rb) {  // block-uniform
+  for (int64_t base = 0; base / group * group * gridDim.x < n; base += rb) {  // block-uniform; rb may cut a group
     const int64_t lin = base + ti;
     const int64_t i = (lin / group * gridDim.x + blockIdx.x) * group + lin % group;
     int64_t e0 = 0, e1 = 0;

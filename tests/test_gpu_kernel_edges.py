@@ -55,6 +55,7 @@ def _recurrence(H, v, K):
     (9000, 31, 3, 0, True),     # a run tile that does not divide the block
     (40011, 3, 12, 0, False),   # 512-thread blocks, one pass, a ragged last row
     (40011, 7, 12, 1, True),    # complex64 vectors and values
+    (14620, 30, 12, 0, False),  # several passes of 17 rows: the last rows in the middle of a group of 8
     (12000, 16, 1, 0, False),   # a single step: alpha only
     (12000, 16, 2, 1, False),
 ])

@@ -82,6 +82,16 @@ SIGNATURES = {
         _I,
         [_I, _P, _I64, C.POINTER(Terms), C.POINTER(Restrictions), _D, _P, _I64, _I, _P, _P, _P, _P, _P, _I, _I, _P, _P],
     ),
+    "edgpu_apply_groups_max_terms": (_I, []),
+    "edgpu_apply_plan_bytes": (_SZ, [_I]),
+    "edgpu_apply_plan": (_I, [_I, C.POINTER(Terms), _P, _SZ, _P]),
+    "edgpu_apply_groups_workspace": (_SZ, [_I64]),
+    "edgpu_apply_groups_entry_bytes": (_SZ, []),
+    "edgpu_apply_groups": (
+        _I,
+        [_I, _P, _I64, _P, _I, _I, C.POINTER(Restrictions), _D, _P, _I64, _P, _I64, _I, _P, _P, _I64, _I, _P, _SZ, _P],
+    ),
+    "edgpu_apply_groups_gather": (_I, [_I, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _I, _P, _SZ, _P]),
     "edgpu_apply_vector": (_I, [_I, _P, _P, _I64, C.POINTER(Terms), C.POINTER(Restrictions), _P, _P, _P, _P, _P]),
     "edgpu_sort_states_workspace": (_SZ, [_I, _I64]),
     "edgpu_sort_states": (_I, [_I, _P, _P, _I64, C.POINTER(C.c_uint64), _P, _SZ, _P]),

@@ -461,10 +461,94 @@ class Engine:
         return u
 
     # -- operator application -------------------------------------------------------------
+    TABLE_MIN_BASIS = 4096  # basis lookups through a hash table from this size on
+
+    def _plan(self, dop, w):
+        """The operator's terms sorted into groups for states of ``w`` words (edgpu_apply_plan), made
+        on first use and kept with the operator (made again when its tables were written since).
+        Another stream than the one that made it waits for it, and the memory is kept until that
+        stream's work on it is done."""
+        plans = dop.__dict__.setdefault("_plans", {})
+        stream = torch.cuda.current_stream(self.device)
+        version = (dop.ops._version, dop.coeff._version)
+        hit = plans.get(w)
+        if hit is not None and hit[3] != version:
+            hit = None
+        if hit is None:
+            size = self.lib.edgpu_apply_plan_bytes(dop.n_terms)
+            plan = torch.empty(size, dtype=torch.uint8, device=self.device)
+            L.check(self.lib.edgpu_apply_plan(w, C.byref(dop.terms), _ptr(plan), size, self.stream), "apply_plan")
+            hit = plans[w] = (plan, stream.record_event(), stream.cuda_stream, version)
+        elif hit[2] != stream.cuda_stream:
+            stream.wait_event(hit[1])
+            hit[0].record_stream(stream)
+        return hit[0]
+
+    def _apply_groups(self, states, dop, restr, weight_min, basis, filt, want, conj):
+        """H|b> of every state in one pass (edgpu_apply_groups).  ``want``: names of the outputs
+        ("states", "index", "vals", "col", "real"); none: counts only.  Returns (offsets, dict)."""
+        n, w = states.shape
+        dev, lib = self.device, self.lib
+        plan = self._plan(dop, w)
+        # row offsets, then what one read tells of the pass (status word, entries), then the counts
+        buf = torch.empty(2 * n + 3, dtype=torch.int64, device=dev)
+        offsets = buf[: n + 1]
+        wsn = lib.edgpu_apply_groups_workspace(n)
+        # its own: the scan between the two launches uses the engine's
+        ws = torch.empty(wsn, dtype=torch.uint8, device=dev)
+        nb = basis.shape[0] if basis is not None else 0
+        table = None
+        # a table costs one pass over the basis, and saves each output some fifteen dependent reads
+        if filt != L.FILTER_NONE and nb >= self.TABLE_MIN_BASIS and 8 * n >= nb:
+            table = torch.empty(1 << int(2 * nb - 1).bit_length(), dtype=torch.int32, device=dev)
+            L.check(lib.edgpu_state_hash_build(w, _ptr(basis), nb, _ptr(table), table.numel(), self.stream),
+                    "state_hash")
+        rp = C.byref(restr) if restr is not None else None
+        entry = lib.edgpu_apply_groups_entry_bytes()
+        cap = min(16 * n + 4096, n * dop.n_terms) if want else 0
+        scan_ws, scan_n = self.workspace(lib.edgpu_scan_workspace(n))
+        while True:
+            arena = torch.empty(cap * entry, dtype=torch.uint8, device=dev) if want else None
+            L.check(
+                lib.edgpu_apply_groups(w, _ptr(states), n, _ptr(plan), dop.n_terms, int(dop.is_real), rp, weight_min,
+                                       _ptr(basis), nb, _ptr(table), 0 if table is None else table.numel(), filt,
+                                       _ptr(buf[n + 1:]), _ptr(arena), cap, self.scratch_entries, _ptr(ws), wsn,
+                                       self.stream),
+                "apply_groups",
+            )
+            L.check(lib.edgpu_scan_i64(_ptr(buf[n + 3:]), _ptr(offsets), n, scan_ws, scan_n, self.stream), "scan")
+            total, st, need = buf[n: n + 3].tolist()  # an overflowed pass is discarded
+            if st == L.EDGPU_ERR_OVERFLOW and self.scratch_entries < 8192:
+                self.scratch_entries *= 4
+                continue
+            if st != L.EDGPU_OK:
+                raise L.EdgpuError(st, "apply_groups")
+            if want and need > cap:
+                cap = need
+                continue
+            break
+        kinds = {"states": ((total, w), torch.int64), "index": ((total,), torch.int64), "col": ((total,), torch.int32),
+                 "vals": ((total, 2), torch.float64), "real": ((total,), torch.float64)}
+        out = {k: torch.empty(kinds[k][0], dtype=kinds[k][1], device=dev) for k in want}
+        if total and want:
+            L.check(
+                lib.edgpu_apply_groups_gather(w, _ptr(states), n, _ptr(offsets), _ptr(arena),
+                                              *(_ptr(out.get(k)) for k in ("states", "index", "col", "vals", "real")),
+                                              int(conj), _ptr(ws), wsn, self.stream), "apply_groups_gather")
+        return offsets, out
+
+    def _groups_ok(self, dop, w):
+        return 0 < dop.n_terms <= self.lib.edgpu_apply_groups_max_terms() and dop.max_orbital < 64 * w
+
     def apply_columns(self, states, dop, restr, weight_min, basis=None, filt=L.FILTER_NONE, want_states=False,
                       want_index=False, want_vals=False, conj=False):
         """Per-state H|b> (see edgpu_apply_columns). Returns (offsets, states, index, vals)."""
         n, w = states.shape
+        if n and self._groups_ok(dop, w):
+            want = [k for k, on in (("states", want_states), ("index", want_index), ("vals", want_vals)) if on]
+            offsets, out = self._apply_groups(states, dop, restr, weight_min, basis, filt, want, conj)
+            return offsets, out.get("states"), out.get("index"), out.get("vals")
+        # operators of more terms, or with orbitals beyond the states' words: a count and a fill pass
         offsets = torch.zeros(n + 1, dtype=torch.int64, device=self.device)
         empty = torch.empty((0, w), dtype=torch.int64, device=self.device)
         if n == 0 or dop.n_terms == 0:
@@ -659,6 +743,14 @@ class Engine:
         Column j of H (= H|b_j>) becomes row j with conjugated values, which for the
         Hermitian H is row j of H.  Real operators store float64 values.
         """
+        n, w = basis_sorted.shape
+        if n and self._groups_ok(dop, w):
+            val = "real" if dop.is_real else "vals"
+            offsets, out = self._apply_groups(basis_sorted, dop, restr, weight_min, basis_sorted, L.FILTER_IN_BASIS,
+                                              ("col", val), True)
+            if dop.is_real:
+                return CsrMatrix(offsets, out["col"], val_r=out["real"])
+            return CsrMatrix(offsets, out["col"], val_c=out["vals"])
         offsets, _, idx, vals = self.apply_columns(basis_sorted, dop, restr, weight_min, basis=basis_sorted,
                                                    filt=L.FILTER_IN_BASIS, want_index=True, want_vals=True, conj=True)
         col = idx.to(torch.int32)

@@ -117,6 +117,41 @@ int edgpu_apply_columns(int n_words, const uint64_t* states, int64_t n_states, c
                         int scratch_entries, int32_t* status_dev, void* stream);
 
 /*
+ * edgpu_apply_columns in one pass (same outputs, bit for bit) for operators of at most
+ * edgpu_apply_groups_max_terms terms.
+ *
+ * edgpu_apply_plan sorts the terms into groups that lead to the same output (plan: 16-byte aligned,
+ * edgpu_apply_plan_bytes; a function of the operator and n_words alone, to be kept with the
+ * operator).  Terms with an orbital beyond n_words * 64 contribute nothing.
+ *
+ * edgpu_apply_groups: a lane takes a group of a state, and the kept outputs go to ``arena``
+ * (arena_entries x edgpu_apply_groups_entry_bytes bytes) in the order the states finish.
+ * info_counts [2 + n_states] receives the status word (EDGPU_ERR_OVERFLOW: some state keeps more
+ * than scratch_entries outputs, 0 = 256; the caller retries larger), the number of arena entries and
+ * the count of every state.  With more entries than arena_entries the arena is incomplete: call
+ * again with a larger one.  arena == NULL: counts only.  real_terms: every coefficient's imaginary
+ * part is zero.  table: hash of the basis (edgpu_state_hash_build) or NULL for binary searches.
+ *
+ * edgpu_apply_groups_gather (same states, arena and workspace, offsets the exclusive scan of the
+ * counts) writes the rows: any of out_states, out_index or out_col (basis positions), out_vals
+ * (complex128) or out_real.
+ */
+int edgpu_apply_groups_max_terms(void);
+size_t edgpu_apply_plan_bytes(int n_terms);
+int edgpu_apply_plan(int n_words, const edgpu_terms* terms, void* plan, size_t bytes, void* stream);
+size_t edgpu_apply_groups_workspace(int64_t n_states);
+size_t edgpu_apply_groups_entry_bytes(void);
+int edgpu_apply_groups(int n_words, const uint64_t* states, int64_t n_states, const void* plan, int n_terms,
+                       int real_terms, const edgpu_restrictions* restr, double weight_min, const uint64_t* basis,
+                       int64_t n_basis, const int32_t* table, int64_t table_size, int filter, int64_t* info_counts,
+                       void* arena, int64_t arena_entries, int scratch_entries, void* workspace,
+                       size_t workspace_bytes, void* stream);
+int edgpu_apply_groups_gather(int n_words, const uint64_t* states, int64_t n_states, const int64_t* offsets,
+                              const void* arena, uint64_t* out_states, int64_t* out_index, int32_t* out_col,
+                              double* out_vals, double* out_real, int conj_vals, void* workspace,
+                              size_t workspace_bytes, void* stream);
+
+/*
  * Raw emissions of an operator on a multi-configurational state psi = sum_k amps[k] |states[k]>.
  * Replaces the inner loops of upstream ``applyOp`` (finite.py:1355-1388): for every
  * (state k, term t) in that order the valid result amps[k] * h_t * sign is emitted; outputs

@@ -137,3 +137,82 @@ def test_rank_in_one_launch(eng, n, words):
     bound = 36 * 2.0 ** -24 * (H2.double().abs() @ net.p["w3"].double().abs() + net.p["b3"].double().abs())
     assert got.shape == (n,)
     assert bool(((got.double() - want[:n].double()).abs() <= bound[:n]).all())
+
+
+def _random_operator(rng, n_orb, n_terms, cplx):
+    """Terms of 0 to 4 operators with repeated orbitals, spectators and several terms an output."""
+    op = {}
+    while len(op) < n_terms:
+        kind = rng.integers(0, 8)
+        i, j, k, l = (int(x) for x in rng.integers(0, n_orb, size=4))
+        key = [((i, "c"), (j, "a")), ((i, "c"), (k, "c"), (k, "a"), (j, "a")), ((k, "a"), (k, "c"), (i, "c"), (j, "a")),
+               ((i, "c"), (j, "c"), (l, "a"), (k, "a")), ((i, "c"), (i, "a")), ((i, "c"), (j, "c"), (i, "a"), (j, "a")),
+               ((i, "a"),), ((i, "c"), (j, "a"), (j, "c"))][kind]
+        v = float(rng.normal()) if rng.random() > 0.1 else -0.0
+        op[key] = complex(v, rng.normal()) if cplx else v
+    return op
+
+
+def _two_pass(eng, states, dop, restr, weight_min, basis, filt, conj):
+    """edgpu_apply_columns: a count and a fill launch."""
+    import ctypes as C
+
+    from impuritymodel_gb300 import _lib as L
+    from impuritymodel_gb300.engine import _ptr
+
+    n, w = states.shape
+    rp = C.byref(restr) if restr is not None else None
+    nb = 0 if basis is None else basis.shape[0]
+    counts = torch.empty(n, dtype=torch.int64, device=eng.device)
+    cap = 256
+    while True:
+        eng.reset_status()
+        L.check(eng.lib.edgpu_apply_columns(w, _ptr(states), n, C.byref(dop.terms), rp, weight_min, _ptr(basis), nb,
+                                            filt, None, _ptr(counts), None, None, None, 0, cap, _ptr(eng.status),
+                                            eng.stream), "apply_columns")
+        if int(eng.status.item()) == 0:
+            break
+        cap *= 4
+    offs = eng.scan(counts)
+    tot = int(offs[-1].item())
+    s = torch.empty((tot, w), dtype=torch.int64, device=eng.device)
+    i = torch.empty(tot, dtype=torch.int64, device=eng.device)
+    v = torch.empty((tot, 2), dtype=torch.float64, device=eng.device)
+    if tot:
+        L.check(eng.lib.edgpu_apply_columns(w, _ptr(states), n, C.byref(dop.terms), rp, weight_min, _ptr(basis), nb,
+                                            filt, _ptr(offs), None, _ptr(s), _ptr(i), _ptr(v), int(conj), cap,
+                                            _ptr(eng.status), eng.stream), "apply_columns")
+    return offs, s, i, v
+
+
+@pytest.mark.parametrize("n,n_orb,n_terms,cplx,filled", [
+    (1, 10, 1, False, 0.5),        # one state, one term
+    (3, 63, 40, True, 0.5),
+    (33, 64, 700, False, 0.9),     # a full word
+    (700, 26, 900, False, 0.4),    # a dense operator: more outputs than the first arena holds
+    (5000, 130, 3000, False, 0.95),  # table lookups, many groups
+    (257, 316, 2500, True, 0.97),
+    (40, 512, 8192, False, 0.9),   # eight words, the largest plan
+])
+def test_one_pass_application(eng, n, n_orb, n_terms, cplx, filled):
+    from impuritymodel_gb300 import _lib as L
+    from impuritymodel_gb300.engine import DeviceOp, make_restrictions
+
+    rng = np.random.default_rng(n + n_terms)
+    dop = DeviceOp(_random_operator(rng, n_orb, n_terms, cplx), eng.device)
+    w = (n_orb + 63) // 64
+    occ = np.zeros((n, 64 * w), dtype=np.uint8)
+    occ[:, :n_orb] = rng.random((n, n_orb)) < filled
+    words = np.packbits(occ, axis=1).view(">u8").astype(np.uint64).reshape(n, w)
+    basis = eng.sort_unique(eng.upload_states(np.unique(words, axis=0)))
+    # the basis and what one application adds to it, so that lookups hit
+    _, more, _, _ = eng.apply_columns(basis[:200].contiguous(), dop, None, 0.0, want_states=True)
+    wide = eng.sort_unique(torch.cat([basis, more], 0))
+    restr = make_restrictions({frozenset(range(0, n_orb, 2)): (0, n_orb // 2), frozenset(range(5)): (1, 4)}, n_orb)
+    for filt, b, r, wmin, conj in ((L.FILTER_NONE, None, None, 0.0, False), (L.FILTER_IN_BASIS, wide, None, 1e-12, True),
+                                   (L.FILTER_NOT_IN_BASIS, basis, restr, 0.5, False)):
+        want = _two_pass(eng, basis, dop, r, wmin, b, filt, conj)
+        got = eng.apply_columns(basis, dop, r, wmin, basis=b, filt=filt, want_states=True, want_index=True,
+                                want_vals=True, conj=conj)
+        for g, x in zip(got, want):
+            assert torch.equal(g.view(torch.int64), x.view(torch.int64))

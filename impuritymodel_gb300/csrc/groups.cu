@@ -20,9 +20,9 @@
 // bit-sliced sums), ~8 that survive, finished 32 at a time.
 //
 // Diagonal sums (some 600 valid terms a state in term order, one dependent FP64 add each, ~64 cycles)
-// run a state per lane in blocks of their own beside the off-diagonal ones, so that the chain of
-// one state is the launch's latency only once; the outputs go to an arena in the order the states
-// finish, and edgpu_apply_groups_gather moves them to their rows once the row offsets are known.
+// run a state per lane in other warps than the off-diagonal outputs, so that the chain is the launch's
+// latency only once; the outputs go to an arena in the order the states finish, and
+// edgpu_apply_groups_gather moves them to their rows once the row offsets are known.
 #include "common.cuh"
 
 namespace edgpu {

@@ -216,3 +216,37 @@ def test_one_pass_application(eng, n, n_orb, n_terms, cplx, filled):
                                 want_vals=True, conj=conj)
         for g, x in zip(got, want):
             assert torch.equal(g.view(torch.int64), x.view(torch.int64))
+
+
+@pytest.mark.parametrize("n,K,cplx,locked", [
+    (5, 5, False, 0),         # fewer rows than a lane group, the whole space
+    (300, 40, True, 0),       # two row chunks, complex H
+    (1770, 60, False, 3),     # seven chunks, deflated vectors
+    (1300, 1100, False, 0),   # more coefficients than shared memory keeps
+    (5000, 50, False, 0),     # more chunks than every block adds up itself
+    (30001, 24, False, 0),    # a chunk per SM, a ragged last one, four lanes a row
+    (65536, 8, False, 0),     # the largest sector of the cooperative form
+])
+def test_reorthogonalised_steps(eng, n, K, cplx, locked):
+    csr, H = _random_csr(eng, n, n, cplx, heavy=(0, n // 2) if n > 100 else ())
+    g = np.random.default_rng(n)
+    Q, _ = np.linalg.qr(g.normal(size=(n, locked + 1)) + 1j * g.normal(size=(n, locked + 1)))
+    lock = torch.from_numpy(np.ascontiguousarray(Q[:, :locked].T)).to(eng.device) if locked else None
+    v0 = torch.from_numpy(np.ascontiguousarray(Q[:, locked])).to(eng.device)
+    V, a, b = eng.krylov_reorth(csr, v0, K, chunk=16, locked=lock)
+    k = len(a)
+    V = V.cpu().numpy()
+    assert k == min(K, n - locked)
+    # orthonormal to working precision (the dot products of n terms round by up to n eps, about sqrt(n) eps)
+    every = np.concatenate([Q[:, :locked].T, V])
+    gram = every.conj() @ every.T
+    assert np.abs(gram - np.eye(len(every))).max() < 20 * np.sqrt(n) * 2.3e-16 + 1e-14
+    # H V = V T + beta v e^T on the complement of the locked vectors, to rounding
+    R = H @ V.T
+    R -= Q[:, :locked] @ (Q[:, :locked].conj().T @ R)
+    T = np.diag(a) + np.diag(b[: k - 1], 1) + np.diag(b[: k - 1], -1)
+    R -= V.T @ T
+    scale = abs(H).sum(1).max()
+    assert np.abs(R[:, : k - 1]).max() < 1e-13 * scale
+    if k < n - locked and K < 1000:
+        assert abs(np.linalg.norm(R[:, k - 1]) - b[k - 1]) < 1e-12 * scale or b[k - 1] == 0.0

@@ -1845,116 +1845,259 @@ int lanczos_small(const edgpu_csr* h, const double* v0, int R, const int32_t* k_
 // so the residual ||r|| / ||y|| = b_{m-1} |q_m| costs O(1) per step.
 // Replaces upstream's per-energy BiCGSTAB (spectra.py:962,1080).
 // ---------------------------------------------------------------------------------------
+//
+// FP64 form.  A step on one SM is bound by FP64 issue (~16 cycles a warp instruction) and its two
+// sums, so what the instructions are spent on decides: rows go to the warps sorted by length (a
+// warp's rows take as many entries as the longest of them), the sector's entries stay in shared
+// memory where they fit (column-major slices of 32 rows), one thread takes the root and the
+// reciprocal of beta (by all threads they were a quarter of the step), and the shifts' estimates
+// run in warps of their own beside the next step's H v (a step past convergence does no harm: only
+// the first m vectors are used).  360 rows, 15 right-hand sides, 50 shifts, ~490 steps:
+// 5.52 -> 3.19 ms, 6.4 us a step, of which some 4 are FP64 issue.
+constexpr int kShiftMaxThreads = 2 * kSmallThreads;
+
+// Sum over the first `mw` warps (the others pass by), returned to every thread; red: 34 doubles.
+// ROOT: red[32] becomes the root of the sum and red[33] its reciprocal (0 for 0).
+template <bool ROOT>
+__device__ __forceinline__ double main_sum(double v, double* red, int mw) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < mw) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[warp] = v;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double t = lane < mw ? red[lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) {
+      if (ROOT) {
+        const double s = sqrt(t);
+        red[32] = s;
+        red[33] = s > 0.0 ? 1.0 / s : 0.0;
+      } else {
+        red[32] = t;
+      }
+    }
+  }
+  __syncthreads();
+  return red[32];
+}
+
+struct ShiftedArgs {
+  int64_t n;
+  const int64_t* rp;
+  const int32_t* col;
+  const double* vals;
+  int n_rhs;
+  const double2 *Y, *zs;
+  int nz, k_cap;
+  double tol;
+  double2* V;
+  double *alpha, *beta;
+  int32_t* m_out;
+  double* ynorm;
+  int32_t* status;
+  int main_threads;  // the others track the shifts
+  int ent_cap;       // entries of the sliced copy that fit in shared memory
+};
+
 template <bool VALC>
-__global__ void __launch_bounds__(kSmallThreads) shifted_small_kernel(
-    int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ col, const double* __restrict__ vals,
-    int n_rhs, const double2* __restrict__ Y, const double2* __restrict__ zs, int nz, int k_cap, double tol,
-    double2* __restrict__ V, double* __restrict__ alpha, double* __restrict__ beta, int32_t* __restrict__ m_out,
-    double* __restrict__ ynorm_out, int32_t* status) {
+__global__ void __launch_bounds__(kShiftMaxThreads) shifted_small_kernel(ShiftedArgs g) {
   extern __shared__ __align__(16) unsigned char sm[];
+  const int n = (int)g.n, M = g.main_threads, mw = M >> 5, nz = g.nz, k_cap = g.k_cap;
+  const int npad = (n + 31) & ~31, slices = npad >> 5;
   double2* X = reinterpret_cast<double2*>(sm);
   double2* P = X + n;
   double2* Wv = P + n;
-  double* red = reinterpret_cast<double*>(Wv + n);
+  double* red = reinterpret_cast<double*>(Wv + n);  // [34]
+  double* sval = red + 34;
+  uint16_t* scol = reinterpret_cast<uint16_t*>(sval + (size_t)g.ent_cap * (VALC ? 2 : 1));
+  uint16_t* order = scol + g.ent_cap;               // [npad] row of each slot, 0xFFFF past the last
+  uint16_t* len = order + npad;                     // [npad]
+  __shared__ int soff[140];                         // slice starts in the copy
+  __shared__ int sliced;
   const int tid = threadIdx.x, bs = blockDim.x;
-  for (int r = blockIdx.x; r < n_rhs; r += gridDim.x) {
-    double2* Vr = V + (size_t)r * k_cap * n;
-    const double2* y = Y + (size_t)r * n;
+  const bool is_main = tid < M;
+  // rows by length, longest first, equal lengths in order
+  for (int i = tid; i < n; i += bs) {
+    const int64_t l = g.rp[i + 1] - g.rp[i];
+    len[i] = (uint16_t)(l < 0xFFFF ? l : 0xFFFF);
+  }
+  for (int i = n + tid; i < npad; i += bs) {
+    len[i] = 0;
+    order[i] = 0xFFFF;
+  }
+  __syncthreads();
+  for (int i = tid; i < n; i += bs) {
+    const int l = len[i];
+    int rank = 0;
+    for (int q = 0; q < n; ++q) rank += len[q] > l || (len[q] == l && q < i);
+    order[rank] = (uint16_t)i;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int at = 0;
+    for (int q = 0; q < slices; ++q) {
+      soff[q] = at;
+      at += 32 * (int)len[order[32 * q]];
+    }
+    soff[slices] = at;
+    sliced = at <= g.ent_cap;
+  }
+  __syncthreads();
+  if (sliced) {
+    for (int q = tid; q < npad; q += bs) {
+      const int row = order[q], s = q >> 5, width = (soff[s + 1] - soff[s]) >> 5;
+      const int l = row == 0xFFFF ? 0 : len[row];
+      const int64_t e0 = row == 0xFFFF ? 0 : g.rp[row];
+      for (int e = 0; e < width; ++e) {
+        const int at = soff[s] + 32 * e + (q & 31);
+        scol[at] = e < l ? (uint16_t)g.col[e0 + e] : 0;
+        if (VALC) {
+          sval[2 * at] = e < l ? g.vals[2 * (e0 + e)] : 0.0;
+          sval[2 * at + 1] = e < l ? g.vals[2 * (e0 + e) + 1] : 0.0;
+        } else {
+          sval[at] = e < l ? g.vals[e0 + e] : 0.0;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int r = blockIdx.x; r < g.n_rhs; r += gridDim.x) {
+    double2* Vr = g.V + (size_t)r * k_cap * n;
+    const double2* y = g.Y + (size_t)r * n;
     double acc = 0.0;
-    for (int64_t i = tid; i < n; i += bs) acc += y[i].x * y[i].x + y[i].y * y[i].y;
-    const double yn = sqrt(block_sum(acc, red));
-    if (tid == 0) ynorm_out[r] = yn;
+    if (is_main)
+      for (int i = tid; i < n; i += M) acc = fma(y[i].y, y[i].y, fma(y[i].x, y[i].x, acc));
+    __syncthreads();  // red is free
+    const double yn = main_sum<true>(acc, red, mw);
+    const double iyn = red[33];
+    if (tid == 0) g.ynorm[r] = yn;
     if (!(yn > 0.0)) {
-      if (tid == 0) m_out[r] = 0;
+      if (tid == 0) g.m_out[r] = 0;
+      __syncthreads();
       continue;
     }
-    const double iyn = 1.0 / yn;
-    for (int64_t i = tid; i < n; i += bs) {
-      const double2 v = make_double2(y[i].x * iyn, y[i].y * iyn);
-      X[i] = v;
-      P[i] = make_double2(0.0, 0.0);
-      Vr[i] = v;
-    }
+    if (is_main)
+      for (int i = tid; i < n; i += M) {
+        const double2 v = make_double2(y[i].x * iyn, y[i].y * iyn);
+        X[i] = v;
+        P[i] = make_double2(0.0, 0.0);
+        Vr[i] = v;
+      }
     __syncthreads();
     double2* x = X;
     double2* p = P;
-    double2 z = make_double2(0.0, 0.0), d = make_double2(1.0, 0.0), q = make_double2(1.0, 0.0);
-    if (tid < nz) z = zs[(size_t)r * nz + tid];
-    double bprev = 0.0;
+    const int tz = tid - M;
+    double2 z = make_double2(0.0, 0.0), id = make_double2(0.0, 0.0), q = make_double2(1.0, 0.0);
+    if (tz >= 0 && tz < nz) z = g.zs[(size_t)r * nz + tz];
+    // the shift's pivot and residual estimate for step k, from alpha_k, beta_{k-1} and beta_k
+    auto track = [&](int k, double a, double b0, double b1) -> bool {
+      if (tz < 0 || tz >= nz) return true;
+      double2 d = make_double2(z.x - a, z.y), qn = make_double2(1.0, 0.0);
+      if (k > 0) {
+        const double b2 = b0 * b0;
+        d.x -= b2 * id.x;
+        d.y -= b2 * id.y;
+        qn = make_double2(q.x * b0, q.y * b0);
+      }
+      const double rd = 1.0 / (d.x * d.x + d.y * d.y);
+      id = make_double2(d.x * rd, -d.y * rd);
+      q = make_double2(qn.x * id.x - qn.y * id.y, qn.x * id.y + qn.y * id.x);
+      return b1 * sqrt(q.x * q.x + q.y * q.y) <= g.tol;
+    };
+    double a = 0.0, b = 0.0, bprev = 0.0;  // alpha_{j-1}, beta_{j-1}, beta_{j-2} at the top of step j
     int m = k_cap;
-    for (int j = 0; j < k_cap; ++j) {
+    for (int j = 0;; ++j) {
+      bool ok = j > 0;
       acc = 0.0;
-      for (int64_t i = tid; i < n; i += bs) {
-        double yr = 0.0, yi = 0.0;
-        const int64_t e1 = rp[i + 1];
-        for (int64_t e = rp[i]; e < e1; ++e) {
-          const double2 xv = x[col[e]];
-          if (VALC) {
-            const double hr = vals[2 * e], hi = vals[2 * e + 1];
-            yr += hr * xv.x - hi * xv.y;
-            yi += hr * xv.y + hi * xv.x;
-          } else {
-            const double h = vals[e];
-            yr += h * xv.x;
-            yi += h * xv.y;
+      if (is_main) {
+        if (j < k_cap)
+          for (int s = tid; s < npad; s += M) {
+            const int row = order[s];
+            if (row == 0xFFFF) continue;
+            const int l = len[row];
+            double yr = 0.0, yi = 0.0;
+            if (sliced) {
+              const int base = soff[s >> 5] + (s & 31);
+#pragma unroll 4
+              for (int e = 0; e < l; ++e) {
+                const int at = base + 32 * e;
+                const double2 xv = x[scol[at]];
+                const double hr = sval[VALC ? 2 * at : at];
+                yr = fma(hr, xv.x, yr);
+                yi = fma(hr, xv.y, yi);
+                if (VALC) {
+                  const double hi = sval[2 * at + 1];
+                  yr = fma(-hi, xv.y, yr);
+                  yi = fma(hi, xv.x, yi);
+                }
+              }
+            } else {
+              const int64_t e1 = g.rp[row + 1];
+#pragma unroll 4
+              for (int64_t e = g.rp[row]; e < e1; ++e) {
+                const double2 xv = x[g.col[e]];
+                const double hr = g.vals[VALC ? 2 * e : e];
+                yr = fma(hr, xv.x, yr);
+                yi = fma(hr, xv.y, yi);
+                if (VALC) {
+                  const double hi = g.vals[2 * e + 1];
+                  yr = fma(-hi, xv.y, yr);
+                  yi = fma(hi, xv.x, yi);
+                }
+              }
+            }
+            Wv[row] = make_double2(yr, yi);
+            acc = fma(yi, x[row].y, fma(yr, x[row].x, acc));
           }
-        }
-        Wv[i] = make_double2(yr, yi);
-        acc += yr * x[i].x + yi * x[i].y;
-      }
-      const double a = block_sum(acc, red);
-      if (tid == 0) alpha[(size_t)r * k_cap + j] = a;
-      acc = 0.0;
-      for (int64_t i = tid; i < n; i += bs) {
-        double2 t = Wv[i];
-        const double2 c = x[i], pv = p[i];
-        t.x = (t.x - a * c.x) - bprev * pv.x;
-        t.y = (t.y - a * c.y) - bprev * pv.y;
-        Wv[i] = t;
-        acc += t.x * t.x + t.y * t.y;
-      }
-      const double b = sqrt(block_sum(acc, red));
-      if (tid == 0) beta[(size_t)r * k_cap + j] = b;
-      bool ok = true;
-      if (tid < nz) {
-        double2 dn = make_double2(z.x - a, z.y);
-        if (j > 0) {
-          const double b2 = bprev * bprev;
-          const double den = d.x * d.x + d.y * d.y;
-          dn.x -= b2 * d.x / den;
-          dn.y += b2 * d.y / den;
-        }
-        const double2 qn = make_double2(j > 0 ? q.x * bprev : 1.0, j > 0 ? q.y * bprev : 0.0);
-        const double den = dn.x * dn.x + dn.y * dn.y;
-        q = make_double2((qn.x * dn.x + qn.y * dn.y) / den, (qn.y * dn.x - qn.x * dn.y) / den);
-        d = dn;
-        ok = b * sqrt(q.x * q.x + q.y * q.y) <= tol;
+      } else if (j > 0) {
+        ok = track(j - 1, a, bprev, b);
       }
       const bool conv = __syncthreads_and(ok);
-      if (conv || !(b > 0.0) || j + 1 == k_cap) {
-        m = j + 1;
-        if (tid == 0) {
-          if (!(b >= 0.0))
-            atomicExch(status, (int32_t)EDGPU_ERR_NAN);
-          else if (!conv && b > 0.0)
-            atomicExch(status, (int32_t)EDGPU_ERR_NOCONV);
-        }
+      if (conv || j == k_cap) {  // step j - 1 was the last
+        m = j;
+        if (tid == 0 && !conv) atomicExch(g.status, (int32_t)EDGPU_ERR_NOCONV);
         break;
       }
-      const double ib = 1.0 / b;
-      double2* vn = Vr + (size_t)(j + 1) * n;
-      for (int64_t i = tid; i < n; i += bs) {
-        const double2 v = make_double2(Wv[i].x * ib, Wv[i].y * ib);
-        p[i] = v;  // v_{j-1} is no longer needed: its buffer becomes v_{j+1}
-        vn[i] = v;
+      bprev = b;
+      a = main_sum<false>(acc, red, mw);
+      if (tid == 0) g.alpha[(size_t)r * k_cap + j] = a;
+      acc = 0.0;
+      if (is_main)
+        for (int i = tid; i < n; i += M) {
+          double2 t = Wv[i];
+          const double2 c = x[i], pv = p[i];
+          t.x = fma(-bprev, pv.x, fma(-a, c.x, t.x));
+          t.y = fma(-bprev, pv.y, fma(-a, c.y, t.y));
+          Wv[i] = t;
+          acc = fma(t.y, t.y, fma(t.x, t.x, acc));
+        }
+      __syncthreads();  // red is free
+      b = main_sum<true>(acc, red, mw);
+      const double ib = red[33];
+      if (tid == 0) g.beta[(size_t)r * k_cap + j] = b;
+      if (!(b > 0.0)) {  // the space is exhausted, or a NaN
+        m = j + 1;
+        if (tid == 0 && !(b >= 0.0)) atomicExch(g.status, (int32_t)EDGPU_ERR_NAN);
+        break;
+      }
+      if (is_main) {
+        double2* vn = Vr + (size_t)(j + 1) * n;
+        for (int i = tid; i < n; i += M) {
+          const double2 v = make_double2(Wv[i].x * ib, Wv[i].y * ib);
+          p[i] = v;  // v_{j-1} is no longer needed: its buffer becomes v_{j+1}
+          if (j + 1 < k_cap) vn[i] = v;
+        }
       }
       __syncthreads();
       double2* t = p;
       p = x;
       x = t;
-      bprev = b;
     }
-    if (tid == 0) m_out[r] = m;
+    if (tid == 0) g.m_out[r] = m;
     __syncthreads();
   }
 }
@@ -2109,17 +2252,28 @@ __global__ void __launch_bounds__(THREADS, 1) shifted_small_df_kernel(
   }
 }
 
-// coef[r][k][z] = ynorm_r * ((z - T_m)^{-1} e_1)_k by the Thomas algorithm: block per
-// right-hand side with its alpha and beta staged in shared memory, thread per shift (one
-// FP64 reciprocal per step).  (z - T) has diagonal z - a_k and off-diagonals -b_k; the
-// forward-sweep ratios and the solution go through scratch laid out [r][k][z], so a warp's
-// accesses are contiguous.  DF writes the coefficients as double-float pairs (float4).
-template <bool DF>
-__global__ void shifted_coef_kernel(const double* __restrict__ alpha, const double* __restrict__ beta,
-                                    const int32_t* __restrict__ m_arr, const double* __restrict__ ynorm,
-                                    const double2* __restrict__ zs, int nz, int k_cap, double2* __restrict__ coef,
-                                    float4* __restrict__ coef_df, double2* __restrict__ cp,
-                                    double2* __restrict__ xs) {
+// coef[r][k][z] = ynorm_r * ((z - T_m)^{-1} e_1)_k, from the minors of z - T_m: with
+//   theta_k = (z - a_k) theta_{k+1} - b_k^2 theta_{k+2}, theta_m = 1, theta_{m+1} = 0
+// the solution is x_k = (b_0 ... b_{k-1}) theta_{k+1} / theta_0.  Neither product has a division, so
+// the chain per step is two dependent multiply-adds instead of a reciprocal and two sweeps, and what
+// follows the chains runs a component per thread over the whole chip (15 right-hand sides, 50
+// shifts, ~490 steps: the sweeps of an elimination 0.56 ms, chains and components 0.19 ms).  Values
+// are kept within +-300 bits of 1, the power of two taken out so far beside them.
+__device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
+
+// (z - a) t1 - b^2 t2
+__device__ __forceinline__ double2 minor_step(double2 z, double a, double b, double2 t1, double2 t2) {
+  const double dr = z.x - a, b2 = -(b * b);
+  return make_double2(fma(dr, t1.x, fma(-z.y, t1.y, b2 * t2.x)), fma(dr, t1.y, fma(z.y, t1.x, b2 * t2.y)));
+}
+
+// Block per right-hand side: a thread per shift runs its chain, one of the last warp the products.
+__global__ void __launch_bounds__(512) shifted_chain_kernel(const double* __restrict__ alpha,
+                                                            const double* __restrict__ beta,
+                                                            const int32_t* __restrict__ m_arr,
+                                                            const double2* __restrict__ zs, int nz, int k_cap,
+                                                            double2* __restrict__ theta, int* __restrict__ theta_exp,
+                                                            double* __restrict__ prod, int* __restrict__ prod_exp) {
   extern __shared__ double ab[];
   const int r = blockIdx.x;
   const int m = m_arr[r];
@@ -2130,67 +2284,138 @@ __global__ void shifted_coef_kernel(const double* __restrict__ alpha, const doub
     b[k] = beta[(size_t)r * k_cap + k];
   }
   __syncthreads();
-  if (m <= 0) return;
-  const double yn = ynorm[r];
   const size_t base = (size_t)r * k_cap * nz;
-  for (int zi = threadIdx.x; zi < nz; zi += blockDim.x) {
-    const double2 z = zs[(size_t)r * nz + zi];
-    double2 cprev = make_double2(0.0, 0.0), dprev = make_double2(0.0, 0.0);
+  if (threadIdx.x >= blockDim.x - 32) {  // a warp of its own
+    if (threadIdx.x != blockDim.x - 1) return;
+    double p = 1.0;
+    int e = 0;
     for (int k = 0; k < m; ++k) {
-      double2 den = make_double2(z.x - a[k], z.y);
-      double2 rk = make_double2(1.0, 0.0);
-      if (k > 0) {
-        den.x += b[k - 1] * cprev.x;
-        den.y += b[k - 1] * cprev.y;
-        rk = make_double2(b[k - 1] * dprev.x, b[k - 1] * dprev.y);
+      prod[(size_t)r * k_cap + k] = p;
+      prod_exp[(size_t)r * k_cap + k] = e;
+      p *= b[k];
+      const int ex = exponent_of(p);
+      if ((ex > 1323 && ex < 2046) || (ex < 723 && ex > 0)) {
+        p *= __hiloint2double((2046 - ex) << 20, 0);
+        e += ex - 1023;
       }
-      const double rdd = 1.0 / (den.x * den.x + den.y * den.y);
-      const double2 inv = make_double2(den.x * rdd, -den.y * rdd);
-      const double bk = (k + 1 < m) ? b[k] : 0.0;
-      cprev = make_double2(-bk * inv.x, -bk * inv.y);
-      dprev = make_double2(rk.x * inv.x - rk.y * inv.y, rk.x * inv.y + rk.y * inv.x);
-      cp[base + (size_t)k * nz + zi] = cprev;
-      xs[base + (size_t)k * nz + zi] = dprev;
     }
-    double2 xn = dprev;
-    for (int k = m - 1; k >= 0; --k) {
-      double2 xk = xs[base + (size_t)k * nz + zi];
-      if (k + 1 < m) {
-        const double2 c = cp[base + (size_t)k * nz + zi];
-        xk = make_double2(xk.x - (c.x * xn.x - c.y * xn.y), xk.y - (c.x * xn.y + c.y * xn.x));
+    return;
+  }
+  for (int zi = threadIdx.x; zi < nz; zi += blockDim.x - 32) {
+    const double2 z = zs[(size_t)r * nz + zi];
+    double2 t1 = make_double2(1.0, 0.0), t2 = make_double2(0.0, 0.0);
+    int e = 0;
+    // four steps between two looks at the exponents: what does not hang on the chain is ready early
+    for (int k0 = (m - 1) & ~3; k0 >= 0; k0 -= 4) {
+#pragma unroll
+      for (int u = 3; u >= 0; --u) {
+        const int k = k0 + u;
+        if (k < m) {
+          theta[base + (size_t)k * nz + zi] = t1;  // theta_{k+1}
+          theta_exp[base + (size_t)k * nz + zi] = e;
+          const double2 t = minor_step(z, a[k], b[k], t1, t2);
+          t2 = t1;
+          t1 = t;
+        }
       }
-      xn = xk;
-      const double2 o = make_double2(yn * xk.x, yn * xk.y);
-      if (DF) {
-        const dfl re = df_split(o.x), im = df_split(o.y);
-        coef_df[base + (size_t)k * nz + zi] = make_float4(re.hi, re.lo, im.hi, im.lo);
-      } else {
-        coef[base + (size_t)k * nz + zi] = o;
+      const int ex = max(max(exponent_of(t1.x), exponent_of(t1.y)), max(exponent_of(t2.x), exponent_of(t2.y)));
+      if ((ex > 1323 && ex < 2046) || (ex < 723 && ex > 0)) {
+        const double f = __hiloint2double((2046 - ex) << 20, 0);
+        t1.x *= f;
+        t1.y *= f;
+        t2.x *= f;
+        t2.y *= f;
+        e += ex - 1023;
       }
     }
   }
 }
 
-// X[r][z][i] = sum_k coef[r][k][z] V[r][k][i] (FP64)
-__global__ void combine_batched_kernel(const double2* __restrict__ V, const double2* __restrict__ coef,
-                                       const int32_t* __restrict__ m_arr, int64_t n, int nz, int k_cap,
-                                       double2* __restrict__ X) {
-  const int r = blockIdx.z;
-  const int zi = blockIdx.y;
+// A component per thread; DF writes the coefficients as double-float pairs (float4).
+template <bool DF>
+__global__ void __launch_bounds__(256) shifted_coef_kernel(
+    const double* __restrict__ alpha, const double* __restrict__ beta, const int32_t* __restrict__ m_arr,
+    const double* __restrict__ ynorm, const double2* __restrict__ zs, int nz, int k_cap,
+    const double2* __restrict__ theta, const int* __restrict__ theta_exp, const double* __restrict__ prod,
+    const int* __restrict__ prod_exp, double2* __restrict__ coef, float4* __restrict__ coef_df) {
+  const int r = blockIdx.y;
   const int m = m_arr[r];
-  const double2* c = coef + (size_t)r * k_cap * nz + zi;
-  const double2* Vr = V + (size_t)r * k_cap * n;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double xr = 0.0, xi = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < m; ++k) {
-      const double2 ck = c[(size_t)k * nz];
-      const double2 v = Vr[(size_t)k * n + i];
-      xr += ck.x * v.x - ck.y * v.y;
-      xi += ck.x * v.y + ck.y * v.x;
+  const size_t base = (size_t)r * k_cap * nz;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t)m * nz;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int k = (int)(t / nz), zi = (int)(t - (int64_t)k * nz);
+    // theta_0 from theta_1 and theta_2, in theta_1's power of two
+    const double2 t1 = theta[base + zi];
+    const int e0 = theta_exp[base + zi];
+    double2 t2 = make_double2(0.0, 0.0);
+    if (m > 1) {
+      const int d = theta_exp[base + nz + zi] - e0;
+      t2 = theta[base + nz + zi];
+      t2 = make_double2(ldexp(t2.x, d), ldexp(t2.y, d));
     }
-    X[((size_t)r * nz + zi) * n + i] = make_double2(xr, xi);
+    const double2 t0 = minor_step(zs[(size_t)r * nz + zi], alpha[(size_t)r * k_cap], beta[(size_t)r * k_cap], t1, t2);
+    const double2 v = theta[base + t];
+    const double s = ynorm[r] * prod[(size_t)r * k_cap + k] / (t0.x * t0.x + t0.y * t0.y);
+    const int e = prod_exp[(size_t)r * k_cap + k] + theta_exp[base + t] - e0;
+    const double2 o = make_double2(ldexp(s * fma(v.x, t0.x, v.y * t0.y), e), ldexp(s * fma(v.y, t0.x, -(v.x * t0.y)), e));
+    if (DF) {
+      const dfl re = df_split(o.x), im = df_split(o.y);
+      coef_df[base + t] = make_float4(re.hi, re.lo, im.hi, im.lo);
+    } else {
+      coef[base + t] = o;
+    }
   }
+}
+
+// X[r][z][i] = sum_k coef[r][k][z] V[r][k][i] (FP64): thread per row, kSumZ shifts per thread.  Bound
+// by FP64 issue, so a complex product takes three multiply-adds instead of four: with
+//   s1 += cr (vr + vi), s2 += vi (cr + ci), s3 += vr (ci - cr)
+// the sums are re = s1 - s2, im = s1 + s3; vr + vi is formed once for all shifts, the coefficient
+// sums once per block.  (Written as a sum of products the four compiled to six.)  15 x 50 sums of
+// ~490 vectors of 360 rows: 1.60 -> 0.81 ms.
+constexpr int kSumZ = 4, kSumRows = 64, kSumStage = 64;
+__global__ void __launch_bounds__(kSumRows) combine_batched_kernel(const double2* __restrict__ V,
+                                                                   const double2* __restrict__ coef,
+                                                                   const int32_t* __restrict__ m_arr, int64_t n,
+                                                                   int nz, int k_cap, double2* __restrict__ X) {
+  __shared__ double cs[kSumStage][kSumZ][3];
+  const int r = blockIdx.z, z0 = blockIdx.y * kSumZ;
+  const int m = m_arr[r];
+  const double2* c = coef + (size_t)r * k_cap * nz;
+  const double2* Vr = V + (size_t)r * k_cap * n;
+  const int64_t i = (int64_t)blockIdx.x * kSumRows + threadIdx.x;
+  double s1[kSumZ], s2[kSumZ], s3[kSumZ];
+#pragma unroll
+  for (int u = 0; u < kSumZ; ++u) s1[u] = s2[u] = s3[u] = 0.0;
+  for (int k0 = 0; k0 < m; k0 += kSumStage) {
+    const int kn = m - k0 < kSumStage ? m - k0 : kSumStage;
+    __syncthreads();
+    for (int t = threadIdx.x; t < kn * kSumZ; t += kSumRows) {
+      const int k = t / kSumZ, u = t % kSumZ;
+      const double2 v = z0 + u < nz ? c[(size_t)(k0 + k) * nz + z0 + u] : make_double2(0.0, 0.0);
+      cs[k][u][0] = v.x;
+      cs[k][u][1] = v.x + v.y;
+      cs[k][u][2] = v.y - v.x;
+    }
+    __syncthreads();
+    if (i < n) {
+#pragma unroll 4
+      for (int k = 0; k < kn; ++k) {
+        const double2 v = Vr[(size_t)(k0 + k) * n + i];
+        const double sum = v.x + v.y;
+#pragma unroll
+        for (int u = 0; u < kSumZ; ++u) {
+          s1[u] = fma(cs[k][u][0], sum, s1[u]);
+          s2[u] = fma(cs[k][u][1], v.y, s2[u]);
+          s3[u] = fma(cs[k][u][2], v.x, s3[u]);
+        }
+      }
+    }
+  }
+  if (i >= n) return;
+#pragma unroll
+  for (int u = 0; u < kSumZ; ++u)
+    if (z0 + u < nz) X[((size_t)r * nz + z0 + u) * n + i] = make_double2(s1[u] - s2[u], s1[u] + s3[u]);
 }
 
 // The same in double-float: thread per row i, kCombineZ shifts per thread (V[k][i] read once
@@ -2284,37 +2509,67 @@ int shifted_solve_impl(const edgpu_csr* h, const double* Y, int n_rhs, const dou
                                            m_out, yn, status_dev);
   } else {
     auto kern = h->val_c ? shifted_small_kernel<true> : shifted_small_kernel<false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSmallThreads, smem);
+    const int npad = (int)((n + 31) & ~(int64_t)31);
+    ShiftedArgs g{};
+    g.n = n;
+    g.rp = h->row_ptr;
+    g.col = h->col;
+    g.vals = h->val_c ? h->val_c : h->val_r;
+    g.n_rhs = n_rhs;
+    g.Y = Yc;
+    g.zs = zc;
+    g.nz = nz;
+    g.k_cap = k_cap;
+    g.tol = tol;
+    g.V = reinterpret_cast<double2*>(V);
+    g.alpha = alpha;
+    g.beta = beta;
+    g.m_out = m_out;
+    g.ynorm = yn;
+    g.status = status_dev;
+    g.main_threads = std::min(kSmallThreads, npad);
+    const int threads = g.main_threads + (nz + 31) / 32 * 32;
+    // shared memory: vectors, sums, slots; the sliced entries when a third more than nnz of them fit
+    const size_t fixed = 3 * sizeof(double2) * (size_t)n + 34 * sizeof(double) + 2 * sizeof(uint16_t) * (size_t)npad + 16;
+    const size_t per_entry = (h->val_c ? 16 : 8) + 2;
+    const int64_t want = h->nnz + h->nnz / 3 + 32;
+    g.ent_cap = fixed + per_entry * (size_t)want <= 220 * 1024 ? (int)((want + 3) & ~(int64_t)3) : 0;
+    const size_t bytes = fixed + per_entry * (size_t)g.ent_cap;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes);
     if (per_sm < 1) per_sm = 1;
     const int grid = std::min(grid_cap() * per_sm, n_rhs);
-    kern<<<grid, kSmallThreads, smem, s>>>(n, h->row_ptr, h->col, h->val_c ? h->val_c : h->val_r, n_rhs, Yc, zc, nz,
-                                           k_cap, tol, reinterpret_cast<double2*>(V), alpha, beta, m_out, yn,
-                                           status_dev);
+    kern<<<grid, threads, bytes, s>>>(g);
   }
   note_launch();
   int rc = check_launch();
   if (rc) return rc;
-  const int cthreads = nz < 128 ? ((nz + 31) / 32) * 32 : 128;
-  if (df) {
-    cudaFuncSetAttribute(shifted_coef_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coef_smem);
-    shifted_coef_kernel<true><<<n_rhs, cthreads, coef_smem, s>>>(alpha, beta, m_out, yn, zc, nz, k_cap, nullptr,
-                                                                 reinterpret_cast<float4*>(coef), cp, xs);
-  } else {
-    cudaFuncSetAttribute(shifted_coef_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coef_smem);
-    shifted_coef_kernel<false><<<n_rhs, cthreads, coef_smem, s>>>(alpha, beta, m_out, yn, zc, nz, k_cap,
-                                                                  reinterpret_cast<double2*>(coef), nullptr, cp, xs);
-  }
+  // the scratch of the coefficients: [products][their exponents][exponents of the minors]
+  double* prod = reinterpret_cast<double*>(xs);
+  int* prod_exp = reinterpret_cast<int*>(prod + (size_t)n_rhs * k_cap);
+  int* theta_exp = prod_exp + (size_t)n_rhs * k_cap;
+  cudaFuncSetAttribute(shifted_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coef_smem);
+  const int cthreads = std::min(512, (nz + 31) / 32 * 32 + 32);
+  shifted_chain_kernel<<<n_rhs, cthreads, coef_smem, s>>>(alpha, beta, m_out, zc, nz, k_cap, cp, theta_exp, prod,
+                                                          prod_exp);
+  note_launch();
+  const dim3 cgrid((unsigned)std::min<int64_t>(((int64_t)k_cap * nz + 255) / 256, grid_cap()), (unsigned)n_rhs);
+  if (df)
+    shifted_coef_kernel<true><<<cgrid, 256, 0, s>>>(alpha, beta, m_out, yn, zc, nz, k_cap, cp, theta_exp, prod,
+                                                    prod_exp, nullptr, reinterpret_cast<float4*>(coef));
+  else
+    shifted_coef_kernel<false><<<cgrid, 256, 0, s>>>(alpha, beta, m_out, yn, zc, nz, k_cap, cp, theta_exp, prod,
+                                                     prod_exp, reinterpret_cast<double2*>(coef), nullptr);
   note_launch();
   if (df) {
     dim3 g3((unsigned)((n + 127) / 128), (unsigned)((nz + kCombineZ - 1) / kCombineZ), (unsigned)n_rhs);
     combine_df_kernel<<<g3, 128, 0, s>>>(reinterpret_cast<const float4*>(V), reinterpret_cast<const float4*>(coef), m_out,
                                          n, nz, k_cap, reinterpret_cast<double2*>(X));
   } else {
-    dim3 g3((unsigned)((n + 255) / 256 > 16 ? 16 : (n + 255) / 256), nz, n_rhs);
-    combine_batched_kernel<<<g3, 256, 0, s>>>(reinterpret_cast<const double2*>(V),
-                                              reinterpret_cast<const double2*>(coef), m_out, n, nz, k_cap,
-                                              reinterpret_cast<double2*>(X));
+    dim3 g3((unsigned)((n + kSumRows - 1) / kSumRows), (unsigned)((nz + kSumZ - 1) / kSumZ), (unsigned)n_rhs);
+    combine_batched_kernel<<<g3, kSumRows, 0, s>>>(reinterpret_cast<const double2*>(V),
+                                                   reinterpret_cast<const double2*>(coef), m_out, n, nz, k_cap,
+                                                   reinterpret_cast<double2*>(X));
   }
   note_launch();
   return check_launch();

@@ -2,6 +2,7 @@
 
 import numpy as np
 import pytest
+import scipy.sparse
 import torch
 
 pytestmark = pytest.mark.gpu
@@ -250,3 +251,31 @@ def test_reorthogonalised_steps(eng, n, K, cplx, locked):
     assert np.abs(R[:, : k - 1]).max() < 1e-13 * scale
     if k < n - locked and K < 1000:
         assert abs(np.linalg.norm(R[:, k - 1]) - b[k - 1]) < 1e-12 * scale or b[k - 1] == 0.0
+
+
+@pytest.mark.parametrize("n,nz,cplx,precision", [
+    (1, 1, False, 0),       # one state: the space is exhausted at once
+    (33, 5, True, 0),       # a second slice of one row, complex H
+    (360, 512, False, 0),   # the most shifts: two rounds of coefficients
+    (700, 3, False, 0),     # more rows than threads
+    (3000, 2, True, 0),     # entries that do not fit in shared memory
+    (360, 50, False, 3),    # double-float recurrence, same coefficients
+])
+def test_shifted_solves(eng, n, nz, cplx, precision):
+    import scipy.sparse.linalg as spl
+
+    csr, H = _random_csr(eng, n, n + nz, cplx, heavy=(0, n // 3) if n > 100 else ())
+    g = np.random.default_rng(nz)
+    Y = g.normal(size=(3, n)) + 1j * g.normal(size=(3, n))
+    Y[1] = 0.0
+    zs = g.uniform(-8.0, 8.0, size=(3, nz)) + 0.5j
+    X, m = eng.shifted_solve(csr, torch.from_numpy(Y).to(eng.device), zs, 1e-10, min(6 * n + 50, 2000), precision)
+    X, m = X.cpu().numpy(), m.cpu().numpy()
+    assert m[1] == 0 and not X[1].any()
+    for r in (0, 2):
+        assert 1 <= m[r] <= min(6 * n + 50, 2000)
+        for q in {0, nz // 2, nz - 1}:
+            x = spl.spsolve(scipy.sparse.identity(n, format="csc") * zs[r, q] - H.tocsc(), Y[r]) if n > 1 else \
+                Y[r] / (zs[r, q] - H[0, 0])
+            # residual below 1e-10 |y|, and |(z - H)^{-1}| <= 1 / Im z; as much again for the rounding
+            assert np.linalg.norm(X[r, q] - x) <= 4e-10 * np.linalg.norm(Y[r])

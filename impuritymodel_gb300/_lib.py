@@ -165,6 +165,12 @@ SIGNATURES = {
     "edgpu_mlp_head_backward": (_I, [_P, _P, _P, _P, _I64, _I, _P, _P, _P, _P]),
     "edgpu_mlp_row_dot": (_I, [_P, _I, _I64, _P, _P, _P]),
     "edgpu_mlp_adam": (_I, [_P, _P, _P, _P, _I64, C.c_float, C.c_float, C.c_float, C.c_float, _P]),
+    "edgpu_mlp_step_workspace": (_SZ, [_I64]),
+    "edgpu_mlp_train_step": (
+        _I,
+        [_P, _I, _P, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _P, _P, C.c_float, C.c_float, C.c_float, C.c_float, _P, _P,
+         _P, _SZ, _P],
+    ),
     "edgpu_mlp_to_bf16": (_I, [_P, _I, _I, _P, _P, _P]),
     "edgpu_cfrac": (_I, [_P, _P, _P, _I, _I, _P, _I, _D, _P, _P, _P, _P]),
     "edgpu_cfrac_f32_workspace": (_SZ, [_I, _I]),

@@ -12,6 +12,7 @@ judge of the energy error (``pruned_ground_state`` reports both).
 
 from __future__ import annotations
 
+import ctypes as C
 import math
 
 import numpy as np
@@ -136,9 +137,13 @@ class BasisNet:
         L.check(lib.edgpu_mlp_row_dot(_ptr(dH1t), N_H, B, None, _ptr(self.g["b1"]), s), "row_dot")
         return ((y - target) ** 2).mean()
 
-    def adam_step(self, beta1=0.9, beta2=0.999, eps=1e-8):
+    def _next_rate(self, beta1, beta2):
+        """Counts a step; its bias-corrected Adam rate."""
         self.t += 1
-        lr_t = self.lr * math.sqrt(1.0 - beta2 ** self.t) / (1.0 - beta1 ** self.t)
+        return self.lr * math.sqrt(1.0 - beta2 ** self.t) / (1.0 - beta1 ** self.t)
+
+    def adam_step(self, beta1=0.9, beta2=0.999, eps=1e-8):
+        lr_t = self._next_rate(beta1, beta2)
         L.check(self._lib().edgpu_mlp_adam(_ptr(self.P), _ptr(self.G), _ptr(self.m), _ptr(self.v), self.P.numel(),
                                            lr_t, beta1, beta2, eps, self.eng.stream), "mlp_adam")
         self.refresh()
@@ -150,19 +155,30 @@ class BasisNet:
         n = states.shape[0]
         gen = torch.Generator(device=self.eng.device)
         gen.manual_seed(int(seed))
-        losses = []
+        e, lib = self.eng, self._lib()
+        dev = e.device
+        states, log_w = states.contiguous(), log_w.contiguous()
+        steps = n // batch
+        loss = torch.empty(max(1, epochs * steps), dtype=torch.float32, device=dev)
+        wsn = lib.edgpu_mlp_step_workspace(batch)
+        ws = torch.empty(wsn if steps else 1, dtype=torch.uint8, device=dev)
+        k = 0
         for ep in range(epochs):
-            perm = torch.randperm(n, device=self.eng.device, generator=gen)
-            for b0 in range(0, n - batch + 1, batch):
-                idx = perm[b0: b0 + batch]
-                X, Xt = self.inputs(states[idx].contiguous(), transposed=True)
-                loss = self.gradients(X, Xt, log_w[idx].contiguous())
-                self.adam_step()
-                losses.append(loss)
+            perm = torch.randperm(n, device=dev, generator=gen)
+            for s in range(steps):
+                # forward, gradients and Adam of one batch (inputs, gradients and adam_step in one call)
+                lr_t = self._next_rate(0.9, 0.999)
+                L.check(lib.edgpu_mlp_train_step(_ptr(states), states.shape[1], C.c_void_p(perm.data_ptr() + 8 * s * batch),
+                                                 _ptr(log_w), batch, N_IN, N_H, _ptr(self.P), _ptr(self.G),
+                                                 _ptr(self.m), _ptr(self.v), _ptr(self.W1b), _ptr(self.W2b),
+                                                 _ptr(self.W2t), lr_t, 0.9, 0.999, 1e-8,
+                                                 C.c_void_p(loss.data_ptr() + 4 * k), _ptr(e.status), _ptr(ws), wsn,
+                                                 e.stream), "mlp_train_step")
+                k += 1
             if log is not None:
-                log.append(float(torch.stack(losses[-max(1, n // batch):]).mean().item()))
-        self.eng.read_status("mlp training")
-        return losses
+                log.append(float(torch.stack(list(loss[:k].unbind())[-max(1, steps):]).mean().item()))
+        e.read_status("mlp training")
+        return list(loss[:k].unbind())
 
     def predict(self, states):
         """Predicted log10 weights of padded states [N, WORDS] (any N): the whole network in one

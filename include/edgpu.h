@@ -580,6 +580,17 @@ int edgpu_mlp_row_dot(const void* M, int rows, int64_t cols, const float* v, flo
 int edgpu_mlp_adam(float* p, const float* g, float* m, float* v, int64_t n, float lr_t, float beta1, float beta2,
                    float eps, void* stream);
 /* BF16 copy Wb of a row-major FP32 [rows][cols] matrix and/or of its transpose Wt. */
+/* One training step: forward, mean squared error, gradients into G and Adam on the flat FP32 parameters
+ * P = (W1 [n_h][n_in], b1, W2 [n_h][n_h], b2, w3, b3), with the BF16 copies W1b, W2b and W2t (W2
+ * transposed) read and written; the batch is states[idx[b]] [W words] and target[idx[b]], b < B (idx
+ * NULL: b itself), B a multiple of 128.  loss receives the batch's loss before the update.  n_in = 320
+ * and n_h = 256 only; W1b, W2b and W2t 16-byte aligned.
+ */
+size_t edgpu_mlp_step_workspace(int64_t B);
+int edgpu_mlp_train_step(const uint64_t* states, int W, const int64_t* idx, const float* target, int64_t B, int n_in,
+                         int n_h, float* P, float* G, float* m, float* v, void* W1b, void* W2b, void* W2t, float lr_t,
+                         float beta1, float beta2, float eps, float* loss, int32_t* status_dev, void* workspace,
+                         size_t workspace_bytes, void* stream);
 int edgpu_mlp_to_bf16(const float* Wf, int rows, int cols, void* Wb, void* Wt, void* stream);
 
 /*

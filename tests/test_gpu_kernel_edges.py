@@ -279,3 +279,32 @@ def test_shifted_solves(eng, n, nz, cplx, precision):
                 Y[r] / (zs[r, q] - H[0, 0])
             # residual below 1e-10 |y|, and |(z - H)^{-1}| <= 1 / Im z; as much again for the rounding
             assert np.linalg.norm(X[r, q] - x) <= 4e-10 * np.linalg.norm(Y[r])
+
+
+@pytest.mark.parametrize("batch,words", [(128, 5), (384, 2), (4096, 5)])
+def test_training_step(eng, batch, words):
+    """One fused step against the layer-by-layer calls."""
+    from impuritymodel_gb300.pruning import BasisNet
+
+    g = torch.Generator(device=eng.device)
+    g.manual_seed(batch)
+    states = torch.randint(-(1 << 62), 1 << 62, (batch, words), device=eng.device, generator=g) * 2
+    log_w = -14.0 * torch.rand(batch, device=eng.device, generator=g)
+    one, two = BasisNet(eng, seed=1), BasisNet(eng, seed=1)
+    losses = one.train(states, log_w, epochs=1, batch=batch)
+    order = torch.Generator(device=eng.device)
+    order.manual_seed(0)
+    perm = torch.randperm(batch, device=eng.device, generator=order)
+    X, Xt = two.inputs(states[perm].contiguous(), transposed=True)
+    loss = two.gradients(X, Xt, log_w[perm].contiguous())
+    two.adam_step()
+    # every gradient but b3's (the last) in the same order of additions
+    for a, b in ((one.G, two.G), (one.P, two.P), (one.m, two.m), (one.v, two.v)):
+        assert torch.equal(a[:-1], b[:-1])
+    for name in ("W1b", "W2b", "W2t"):
+        assert torch.equal(getattr(one, name), getattr(two, name))
+    # sums of `batch` terms of one size in two orders, both trees over 256 chains
+    depth = 2.0 ** -24 * (batch / 128 + 16)
+    bound = depth * float((2.0 / batch * (one.predict(states) - log_w).abs()).sum() + 1.0)
+    assert abs(float(one.G[-1] - two.G[-1])) <= bound
+    assert len(losses) == 1 and abs(float(losses[0] - loss)) <= depth * abs(float(loss))

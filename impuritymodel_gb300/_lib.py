@@ -104,6 +104,9 @@ SIGNATURES = {
     "edgpu_lookup_states": (_I, [_I, _P, _I64, _P, _I64, _P, _P]),
     "edgpu_spmv": (_I, [C.POINTER(CSR), _P, _P, _I, _P]),
     "edgpu_spmv_c64": (_I, [C.POINTER(CSR), _P, _P, _I, _P]),
+    "edgpu_spmv_shift_c64": (_I, [C.POINTER(CSR), C.c_float, _P, _P, _I, _P]),
+    "edgpu_spmv_planned_shift_c64": (_I, [C.POINTER(CSR), _P, _I64, _I, _I, C.c_float, _P, _P, _I, _P]),
+    "edgpu_spmv_paged_shift_c64": (_I, [C.POINTER(CSR), _P, _I64, _I, _I, _I, C.c_float, _P, _P, _I, _P]),
     "edgpu_spmv_plan_workspace": (_SZ, [_I64]),
     "edgpu_spmv_plan": (_I, [C.POINTER(CSR), _I64, _I, _P, C.POINTER(_I64), _P, _SZ, _P]),
     "edgpu_spmv_planned": (_I, [C.POINTER(CSR), _P, _I64, _I, _I, _P, _P, _I, _P]),

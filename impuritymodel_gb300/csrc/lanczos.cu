@@ -10,6 +10,7 @@
 // All reductions are deterministic: per-block partials in fixed order, summed in fixed order.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -800,20 +801,23 @@ struct Vec16<double> {
 
 constexpr int kRowsThreads = 128;  // smaller blocks shorten the tail of ragged rows
 
-template <typename T, bool VALC>
+// RV runs per thread: what 16 bytes hold, or one (8 bytes) for an odd number of complex64 runs.
+// shift != 0: Y = H X + shift X.
+template <typename T, bool VALC, int RV>
 __global__ void __launch_bounds__(kRowsThreads) spmm_rows_kernel(int64_t n, const int64_t* __restrict__ rp,
                                                                  const int32_t* __restrict__ col,
-                                                                 const T* __restrict__ vals, int R, int L,
+                                                                 const T* __restrict__ vals, int R, int L, T shift,
                                                                  const typename Cx<T>::V* __restrict__ X,
                                                                  typename Cx<T>::V* __restrict__ Y) {
-  using Q = typename Vec16<T>::type;
-  constexpr int RV = Vec16<T>::runs;
+  using Q = std::conditional_t<RV == Vec16<T>::runs, typename Vec16<T>::type, typename Cx<T>::V>;
   constexpr int UNROLL = 8;
   const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = gt / L;
   const int g = (int)(gt - i * L);
   if (i >= n) return;
   const int64_t r0 = (int64_t)g * RV;
+  Q own{};
+  if (shift != T(0)) own = __ldg(reinterpret_cast<const Q*>(X + i * R + r0));
   T ar[RV], ai[RV];
 #pragma unroll
   for (int q = 0; q < RV; ++q) ar[q] = ai[q] = 0;
@@ -857,54 +861,33 @@ __global__ void __launch_bounds__(kRowsThreads) spmm_rows_kernel(int64_t n, cons
   }
   Q out;
   T* os = reinterpret_cast<T*>(&out);
+  const T* xo = reinterpret_cast<const T*>(&own);
 #pragma unroll
   for (int q = 0; q < RV; ++q) {
-    os[2 * q] = ar[q];
-    os[2 * q + 1] = ai[q];
+    os[2 * q] = shift != T(0) ? ar[q] + shift * xo[2 * q] : ar[q];
+    os[2 * q + 1] = shift != T(0) ? ai[q] + shift * xo[2 * q + 1] : ai[q];
   }
   __stcs(reinterpret_cast<Q*>(Y + i * R + r0), out);
 }
 
-template <typename T>
-int spmv_impl(const edgpu_csr* h, const typename Cx<T>::V* x, typename Cx<T>::V* y, int R, cudaStream_t s) {
-  constexpr int RV = Vec16<T>::runs;
-  if (R % RV == 0) {
-    const int L = R / RV;
-    const int64_t threads = h->n * (int64_t)L;
-    const unsigned blocks = (unsigned)((threads + kRowsThreads - 1) / kRowsThreads);
-    const int bt = kRowsThreads;
-    if (sizeof(T) == 8) {
-      if (h->val_c)
-        spmm_rows_kernel<T, true><<<blocks, bt, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_c, R, L, x, y);
-      else
-        spmm_rows_kernel<T, false><<<blocks, bt, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_r, R, L, x, y);
-    } else {
-      if (h->val_cf)
-        spmm_rows_kernel<T, true><<<blocks, bt, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_cf, R, L, x, y);
-      else
-        spmm_rows_kernel<T, false><<<blocks, bt, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_rf, R, L, x, y);
-    }
-    note_launch();
-    return check_launch();
-  }
-  RunTile t = make_tile(h->n, R);
-  dim3 grid(t.nrb, t.nrt), block(t.rt, t.rb);
-  if (sizeof(T) == 8) {
-    if (h->val_c)
-      spmm_alpha_kernel<T, true><<<grid, block, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_c, R,
-                                                        x, y, nullptr, 0);
-    else
-      spmm_alpha_kernel<T, false><<<grid, block, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_r, R,
-                                                         x, y, nullptr, 0); note_launch();
-  } else {
-    if (h->val_cf)
-      spmm_alpha_kernel<T, true><<<grid, block, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_cf, R,
-                                                        x, y, nullptr, 0);
-    else
-      spmm_alpha_kernel<T, false><<<grid, block, 0, s>>>(h->n, h->row_ptr, h->col, (const T*)h->val_rf, R,
-                                                         x, y, nullptr, 0); note_launch();
-  }
+template <typename T, int RV>
+int launch_rows(const edgpu_csr* h, const T* val_c, const T* val_r, T shift, const typename Cx<T>::V* x,
+                typename Cx<T>::V* y, int R, cudaStream_t s) {
+  const int L = R / RV;
+  const int64_t blocks = (h->n * (int64_t)L + kRowsThreads - 1) / kRowsThreads;
+  if (blocks > 0x7fffffffLL) return EDGPU_ERR_ARG;
+  if (val_c)
+    spmm_rows_kernel<T, true, RV><<<(unsigned)blocks, kRowsThreads, 0, s>>>(h->n, h->row_ptr, h->col, val_c, R, L,
+                                                                            shift, x, y);
+  else
+    spmm_rows_kernel<T, false, RV><<<(unsigned)blocks, kRowsThreads, 0, s>>>(h->n, h->row_ptr, h->col, val_r, R, L,
+                                                                             shift, x, y);
+  note_launch();
   return check_launch();
+}
+
+inline bool spmv_aligned(const void* x, const void* y) {
+  return ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
 }
 
 // Optional per-kernel timing with CUDA events on the launching stream: kernel_ms[0..2] receive
@@ -1015,16 +998,24 @@ extern "C" int edgpu_spmv(const edgpu_csr* h, const double* x, double* y, int R,
   if (!h || !x || !y || R < 1 || h->n < 0) return EDGPU_ERR_ARG;
   if (!h->val_c && !h->val_r) return EDGPU_ERR_ARG;
   if (h->n == 0) return EDGPU_OK;
-  return spmv_impl<double>(h, reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(y), R,
-                           (cudaStream_t)stream);
+  return launch_rows<double, 1>(h, h->val_c, h->val_r, 0.0, reinterpret_cast<const double2*>(x),
+                                reinterpret_cast<double2*>(y), R, (cudaStream_t)stream);
 }
 
-extern "C" int edgpu_spmv_c64(const edgpu_csr* h, const float* x, float* y, int R, void* stream) {
+extern "C" int edgpu_spmv_shift_c64(const edgpu_csr* h, float shift, const float* x, float* y, int R, void* stream) {
   if (!h || !x || !y || R < 1 || h->n < 0) return EDGPU_ERR_ARG;
   if (!h->val_cf && !h->val_rf) return EDGPU_ERR_ARG;
   if (h->n == 0) return EDGPU_OK;
-  return spmv_impl<float>(h, reinterpret_cast<const float2*>(x), reinterpret_cast<float2*>(y), R,
-                          (cudaStream_t)stream);
+  const float2* xc = reinterpret_cast<const float2*>(x);
+  float2* yc = reinterpret_cast<float2*>(y);
+  // two runs a thread; one where their number is odd or a pair is not 16 bytes aligned
+  if (R % 2 == 0 && spmv_aligned(x, y))
+    return launch_rows<float, 2>(h, h->val_cf, h->val_rf, shift, xc, yc, R, (cudaStream_t)stream);
+  return launch_rows<float, 1>(h, h->val_cf, h->val_rf, shift, xc, yc, R, (cudaStream_t)stream);
+}
+
+extern "C" int edgpu_spmv_c64(const edgpu_csr* h, const float* x, float* y, int R, void* stream) {
+  return edgpu_spmv_shift_c64(h, 0.f, x, y, R, stream);
 }
 
 extern "C" size_t edgpu_lanczos_workspace(int64_t n, int R, int K, int precision) {

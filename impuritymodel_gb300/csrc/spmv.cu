@@ -46,7 +46,8 @@ struct Pack16<double> {
 template <typename T, bool VALC, int L, int U>
 __global__ void spmv_sched_kernel(int64_t n_heavy, int64_t n, const int64_t* __restrict__ rp,
                                   const int32_t* __restrict__ col, const T* __restrict__ vals,
-                                  const int32_t* __restrict__ sched, const typename Pack16<T>::type* __restrict__ X,
+                                  const int32_t* __restrict__ sched, T shift,
+                                  const typename Pack16<T>::type* __restrict__ X,
                                   typename Pack16<T>::type* __restrict__ Y) {
   using P = typename Pack16<T>::type;
   constexpr int RV = Pack16<T>::runs;
@@ -70,6 +71,8 @@ __global__ void spmv_sched_kernel(int64_t n_heavy, int64_t n, const int64_t* __r
       e1 = __ldg(rp + row + 1);
     }
   }
+  P own{};  // the row's x, when a multiple of it is added to the product
+  if (shift != T(0) && row >= 0 && (!heavy || grp == 0)) own = __ldg(X + row * L + sub);
   T ar[RV], ai[RV];
 #pragma unroll
   for (int q = 0; q < RV; ++q) ar[q] = ai[q] = T(0);
@@ -121,10 +124,11 @@ __global__ void spmv_sched_kernel(int64_t n_heavy, int64_t n, const int64_t* __r
   if (row < 0) return;
   P out;
   T* os = reinterpret_cast<T*>(&out);
+  const T* xo = reinterpret_cast<const T*>(&own);
 #pragma unroll
   for (int q = 0; q < RV; ++q) {
-    os[2 * q] = ar[q];
-    os[2 * q + 1] = ai[q];
+    os[2 * q] = shift != T(0) ? ar[q] + shift * xo[2 * q] : ar[q];
+    os[2 * q + 1] = shift != T(0) ? ai[q] + shift * xo[2 * q + 1] : ai[q];
   }
   __stcs(Y + row * L + sub, out);
 }
@@ -147,10 +151,10 @@ __global__ void spmv_plan_keys_kernel(int64_t n, const int64_t* __restrict__ rp,
 
 template <typename T, bool VALC, int L>
 int launch_sched(const edgpu_csr* h, const T* vals, const int32_t* sched, int64_t n_heavy, int unroll, int block,
-                 const void* x, void* y, cudaStream_t s, int64_t n_rows = -1) {
+                 T shift, const void* x, void* y, cudaStream_t s) {
   using P = typename Pack16<T>::type;
   constexpr int G = 32 / L;
-  const int64_t n = n_rows < 0 ? h->n : n_rows;  // n_rows = n_heavy: the heavy rows only
+  const int64_t n = h->n;
   const int64_t warps = n_heavy + (n - n_heavy + G - 1) / G;
   const int64_t blocks = (warps * 32 + block - 1) / block;
   if (blocks > 0x7fffffffLL) return EDGPU_ERR_ARG;
@@ -158,34 +162,34 @@ int launch_sched(const edgpu_csr* h, const T* vals, const int32_t* sched, int64_
   P* Y = reinterpret_cast<P*>(y);
   if (unroll == 4)
     spmv_sched_kernel<T, VALC, L, 4><<<(unsigned)blocks, block, 0, s>>>(n_heavy, n, h->row_ptr, h->col, vals, sched,
-                                                                        X, Y);
+                                                                        shift, X, Y);
   else if (unroll == 8)
     spmv_sched_kernel<T, VALC, L, 8><<<(unsigned)blocks, block, 0, s>>>(n_heavy, n, h->row_ptr, h->col, vals, sched,
-                                                                        X, Y);
+                                                                        shift, X, Y);
   else
     spmv_sched_kernel<T, VALC, L, 2><<<(unsigned)blocks, block, 0, s>>>(n_heavy, n, h->row_ptr, h->col, vals, sched,
-                                                                        X, Y);
+                                                                        shift, X, Y);
   note_launch();
   return check_launch();
 }
 
 template <typename T, bool VALC>
 int dispatch_lanes(const edgpu_csr* h, const T* vals, const int32_t* sched, int64_t n_heavy, int unroll, int block,
-                   const void* x, void* y, int L, cudaStream_t s, int64_t n_rows = -1) {
+                   T shift, const void* x, void* y, int L, cudaStream_t s) {
   switch (L) {
-    case 1: return launch_sched<T, VALC, 1>(h, vals, sched, n_heavy, unroll, block, x, y, s, n_rows);
-    case 2: return launch_sched<T, VALC, 2>(h, vals, sched, n_heavy, unroll, block, x, y, s, n_rows);
-    case 4: return launch_sched<T, VALC, 4>(h, vals, sched, n_heavy, unroll, block, x, y, s, n_rows);
-    case 8: return launch_sched<T, VALC, 8>(h, vals, sched, n_heavy, unroll, block, x, y, s, n_rows);
-    case 16: return launch_sched<T, VALC, 16>(h, vals, sched, n_heavy, unroll, block, x, y, s, n_rows);
-    case 32: return launch_sched<T, VALC, 32>(h, vals, sched, n_heavy, unroll, block, x, y, s, n_rows);
+    case 1: return launch_sched<T, VALC, 1>(h, vals, sched, n_heavy, unroll, block, shift, x, y, s);
+    case 2: return launch_sched<T, VALC, 2>(h, vals, sched, n_heavy, unroll, block, shift, x, y, s);
+    case 4: return launch_sched<T, VALC, 4>(h, vals, sched, n_heavy, unroll, block, shift, x, y, s);
+    case 8: return launch_sched<T, VALC, 8>(h, vals, sched, n_heavy, unroll, block, shift, x, y, s);
+    case 16: return launch_sched<T, VALC, 16>(h, vals, sched, n_heavy, unroll, block, shift, x, y, s);
+    case 32: return launch_sched<T, VALC, 32>(h, vals, sched, n_heavy, unroll, block, shift, x, y, s);
     default: return EDGPU_ERR_ARG;
   }
 }
 
 template <typename T>
-int spmv_planned(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int unroll, int block, const void* x,
-                 void* y, int R, const T* val_c, const T* val_r, cudaStream_t s) {
+int spmv_planned(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int unroll, int block, T shift,
+                 const void* x, void* y, int R, const T* val_c, const T* val_r, cudaStream_t s) {
   if (!h || !sched || !x || !y || h->n < 1 || R < 1) return EDGPU_ERR_ARG;
   if (n_heavy < 0 || n_heavy > h->n) return EDGPU_ERR_ARG;
   if (unroll != 2 && unroll != 4 && unroll != 8) return EDGPU_ERR_ARG;
@@ -195,8 +199,8 @@ int spmv_planned(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int 
   const int L = R / RV;
   if (L > 32 || (32 % L)) return EDGPU_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) return EDGPU_ERR_ARG;
-  if (val_c) return dispatch_lanes<T, true>(h, val_c, sched, n_heavy, unroll, block, x, y, L, s);
-  if (val_r) return dispatch_lanes<T, false>(h, val_r, sched, n_heavy, unroll, block, x, y, L, s);
+  if (val_c) return dispatch_lanes<T, true>(h, val_c, sched, n_heavy, unroll, block, shift, x, y, L, s);
+  if (val_r) return dispatch_lanes<T, false>(h, val_r, sched, n_heavy, unroll, block, shift, x, y, L, s);
   return EDGPU_ERR_ARG;
 }
 
@@ -261,7 +265,7 @@ constexpr int kPageWarps = 4;  // warps (pages) per block of the paged kernel
 
 template <typename T, bool VALC, int L, int U, int CH, bool PIPE, bool HINT>
 __global__ void __launch_bounds__(32 * kPageWarps) spmv_pages_kernel(int64_t n_pages,
-                                                                     const Ent<T, VALC>* __restrict__ pages,
+                                                                     const Ent<T, VALC>* __restrict__ pages, T shift,
                                                                      const typename Pack16<T>::type* __restrict__ X,
                                                                      typename Pack16<T>::type* __restrict__ Y) {
   using E = Ent<T, VALC>;
@@ -297,6 +301,7 @@ __global__ void __launch_bounds__(32 * kPageWarps) spmv_pages_kernel(int64_t n_p
   for (int q = 0; q < RV; ++q) ar[q] = ai[q] = T(0);
   int64_t row = -1;
   bool heavy = false;
+  P own{};  // the open row's x, when a multiple of it is added to the product
   auto flush = [&]() {  // called by the whole warp at the same column
     if (heavy) {
 #pragma unroll
@@ -310,10 +315,11 @@ __global__ void __launch_bounds__(32 * kPageWarps) spmv_pages_kernel(int64_t n_p
     if (row >= 0 && (!heavy || grp == 0)) {
       P out;
       T* os = reinterpret_cast<T*>(&out);
+      const T* xo = reinterpret_cast<const T*>(&own);
 #pragma unroll
       for (int q = 0; q < RV; ++q) {
-        os[2 * q] = ar[q];
-        os[2 * q + 1] = ai[q];
+        os[2 * q] = shift != T(0) ? ar[q] + shift * xo[2 * q] : ar[q];
+        os[2 * q + 1] = shift != T(0) ? ai[q] + shift * xo[2 * q + 1] : ai[q];
       }
       __stcs(Y + row * L + sub, out);
     }
@@ -352,6 +358,7 @@ __global__ void __launch_bounds__(32 * kPageWarps) spmv_pages_kernel(int64_t n_p
         flush();
         row = c == INT_MIN ? -1 : (int64_t)(-2 - (int64_t)c);
         heavy = e[u].flag() != 0;
+        if (shift != T(0) && row >= 0 && (!heavy || grp == 0)) own = __ldg(X + row * L + sub);
         continue;
       }
       if (c < 0) continue;
@@ -484,7 +491,7 @@ __global__ void pages_fill_kernel(int64_t n_slices, int64_t n_heavy, int64_t n_r
 }
 
 template <typename T, bool VALC, int L, int U, int CH>
-int launch_pages_t(int64_t n_pages, const void* pages, const void* x, void* y, cudaStream_t s, int flags) {
+int launch_pages_t(int64_t n_pages, const void* pages, T shift, const void* x, void* y, cudaStream_t s, int flags) {
   using P = typename Pack16<T>::type;
   using E = Ent<T, VALC>;
   auto kern = (flags & 1) ? ((flags & 2) ? spmv_pages_kernel<T, VALC, L, U, CH, true, true>
@@ -499,7 +506,7 @@ int launch_pages_t(int64_t n_pages, const void* pages, const void* x, void* y, c
   }
   const int64_t blocks = (n_pages + kPageWarps - 1) / kPageWarps;
   if (blocks > 0x7fffffffLL) return EDGPU_ERR_ARG;
-  kern<<<(unsigned)blocks, 32 * kPageWarps, smem, s>>>(n_pages, reinterpret_cast<const E*>(pages),
+  kern<<<(unsigned)blocks, 32 * kPageWarps, smem, s>>>(n_pages, reinterpret_cast<const E*>(pages), shift,
                                                         reinterpret_cast<const P*>(x), reinterpret_cast<P*>(y));
   note_launch();
   return check_launch();
@@ -508,25 +515,25 @@ int launch_pages_t(int64_t n_pages, const void* pages, const void* x, void* y, c
 // unroll: 4 or 8 gathers per lane per batch; flags bit 0: two batches in flight, bit 1: L2
 // eviction hints (x rows evict-last, pages evict-first)
 template <typename T, bool VALC, int L>
-int launch_pages_l(int64_t n_pages, const void* pages, int CH, int unroll, int flags, const void* x, void* y,
+int launch_pages_l(int64_t n_pages, const void* pages, int CH, int unroll, int flags, T shift, const void* x, void* y,
                    cudaStream_t s) {
-  if (CH == 256 && unroll == 4) return launch_pages_t<T, VALC, L, 4, 256>(n_pages, pages, x, y, s, flags);
-  if (CH == 256 && unroll == 8) return launch_pages_t<T, VALC, L, 8, 256>(n_pages, pages, x, y, s, flags);
-  if (CH == 512 && unroll == 4) return launch_pages_t<T, VALC, L, 4, 512>(n_pages, pages, x, y, s, flags);
-  if (CH == 512 && unroll == 8) return launch_pages_t<T, VALC, L, 8, 512>(n_pages, pages, x, y, s, flags);
-  if (CH == 1024 && unroll == 4) return launch_pages_t<T, VALC, L, 4, 1024>(n_pages, pages, x, y, s, flags);
-  if (CH == 1024 && unroll == 8) return launch_pages_t<T, VALC, L, 8, 1024>(n_pages, pages, x, y, s, flags);
+  if (CH == 256 && unroll == 4) return launch_pages_t<T, VALC, L, 4, 256>(n_pages, pages, shift, x, y, s, flags);
+  if (CH == 256 && unroll == 8) return launch_pages_t<T, VALC, L, 8, 256>(n_pages, pages, shift, x, y, s, flags);
+  if (CH == 512 && unroll == 4) return launch_pages_t<T, VALC, L, 4, 512>(n_pages, pages, shift, x, y, s, flags);
+  if (CH == 512 && unroll == 8) return launch_pages_t<T, VALC, L, 8, 512>(n_pages, pages, shift, x, y, s, flags);
+  if (CH == 1024 && unroll == 4) return launch_pages_t<T, VALC, L, 4, 1024>(n_pages, pages, shift, x, y, s, flags);
+  if (CH == 1024 && unroll == 8) return launch_pages_t<T, VALC, L, 8, 1024>(n_pages, pages, shift, x, y, s, flags);
   return EDGPU_ERR_ARG;
 }
 
 template <typename T, bool VALC>
-int launch_pages(int64_t n_pages, const void* pages, int CH, int unroll, int flags, int L, const void* x, void* y,
-                 cudaStream_t s) {
+int launch_pages(int64_t n_pages, const void* pages, int CH, int unroll, int flags, int L, T shift, const void* x,
+                 void* y, cudaStream_t s) {
   switch (L) {
-    case 2: return launch_pages_l<T, VALC, 2>(n_pages, pages, CH, unroll, flags, x, y, s);
-    case 4: return launch_pages_l<T, VALC, 4>(n_pages, pages, CH, unroll, flags, x, y, s);
-    case 8: return launch_pages_l<T, VALC, 8>(n_pages, pages, CH, unroll, flags, x, y, s);
-    case 16: return launch_pages_l<T, VALC, 16>(n_pages, pages, CH, unroll, flags, x, y, s);
+    case 2: return launch_pages_l<T, VALC, 2>(n_pages, pages, CH, unroll, flags, shift, x, y, s);
+    case 4: return launch_pages_l<T, VALC, 4>(n_pages, pages, CH, unroll, flags, shift, x, y, s);
+    case 8: return launch_pages_l<T, VALC, 8>(n_pages, pages, CH, unroll, flags, shift, x, y, s);
+    case 16: return launch_pages_l<T, VALC, 16>(n_pages, pages, CH, unroll, flags, shift, x, y, s);
     default: return EDGPU_ERR_ARG;
   }
 }
@@ -598,13 +605,21 @@ extern "C" int edgpu_spmv_plan(const edgpu_csr* h, int64_t window, int heavy_min
 extern "C" int edgpu_spmv_planned(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int unroll, int block,
                                   const double* x, double* y, int R, void* stream) {
   if (!h) return EDGPU_ERR_ARG;
-  return spmv_planned<double>(h, sched, n_heavy, unroll, block, x, y, R, h->val_c, h->val_r, (cudaStream_t)stream);
+  return spmv_planned<double>(h, sched, n_heavy, unroll, block, 0.0, x, y, R, h->val_c, h->val_r, (cudaStream_t)stream);
 }
 
 extern "C" int edgpu_spmv_planned_c64(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int unroll,
                                       int block, const float* x, float* y, int R, void* stream) {
   if (!h) return EDGPU_ERR_ARG;
-  return spmv_planned<float>(h, sched, n_heavy, unroll, block, x, y, R, h->val_cf, h->val_rf, (cudaStream_t)stream);
+  return spmv_planned<float>(h, sched, n_heavy, unroll, block, 0.f, x, y, R, h->val_cf, h->val_rf,
+                             (cudaStream_t)stream);
+}
+
+extern "C" int edgpu_spmv_planned_shift_c64(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int unroll,
+                                            int block, float shift, const float* x, float* y, int R, void* stream) {
+  if (!h) return EDGPU_ERR_ARG;
+  return spmv_planned<float>(h, sched, n_heavy, unroll, block, shift, x, y, R, h->val_cf, h->val_rf,
+                             (cudaStream_t)stream);
 }
 
 extern "C" size_t edgpu_spmv_pages_workspace(int64_t n, int lanes) {
@@ -688,7 +703,7 @@ extern "C" int edgpu_spmv_pages_build(const edgpu_csr* h, const int32_t* sched, 
 
 template <typename T>
 static int spmv_paged_impl(const edgpu_csr* h, const void* pages, int64_t n_pages, int page_entries, int unroll,
-                           int flags, const void* x, void* y, int R, cudaStream_t s) {
+                           int flags, T shift, const void* x, void* y, int R, cudaStream_t s) {
   if (!h || !x || !y || h->n < 1 || n_pages < 0) return EDGPU_ERR_ARG;
   if (n_pages > 0 && !pages) return EDGPU_ERR_ARG;
   if ((unroll != 4 && unroll != 8) || flags < 0 || flags > 3) return EDGPU_ERR_ARG;
@@ -701,17 +716,26 @@ static int spmv_paged_impl(const edgpu_csr* h, const void* pages, int64_t n_page
   if (sizeof(T) == 8 && (h->val_c || !h->val_r)) return EDGPU_ERR_ARG;  // complex128 values: no paged form
   if (sizeof(T) == 4 && !h->val_cf && !h->val_rf) return EDGPU_ERR_ARG;
   if (n_pages == 0) return EDGPU_OK;
-  if (sizeof(T) == 8) return launch_pages<double, false>(n_pages, pages, page_entries, unroll, flags, L, x, y, s);
-  if (h->val_cf) return launch_pages<float, true>(n_pages, pages, page_entries, unroll, flags, L, x, y, s);
-  return launch_pages<float, false>(n_pages, pages, page_entries, unroll, flags, L, x, y, s);
+  if constexpr (sizeof(T) == 8) {
+    return launch_pages<double, false>(n_pages, pages, page_entries, unroll, flags, L, shift, x, y, s);
+  } else {
+    if (h->val_cf) return launch_pages<float, true>(n_pages, pages, page_entries, unroll, flags, L, shift, x, y, s);
+    return launch_pages<float, false>(n_pages, pages, page_entries, unroll, flags, L, shift, x, y, s);
+  }
 }
 
 extern "C" int edgpu_spmv_paged(const edgpu_csr* h, const void* pages, int64_t n_pages, int page_entries, int unroll,
                                 int flags, const double* x, double* y, int R, void* stream) {
-  return spmv_paged_impl<double>(h, pages, n_pages, page_entries, unroll, flags, x, y, R, (cudaStream_t)stream);
+  return spmv_paged_impl<double>(h, pages, n_pages, page_entries, unroll, flags, 0.0, x, y, R, (cudaStream_t)stream);
 }
 
 extern "C" int edgpu_spmv_paged_c64(const edgpu_csr* h, const void* pages, int64_t n_pages, int page_entries,
                                     int unroll, int flags, const float* x, float* y, int R, void* stream) {
-  return spmv_paged_impl<float>(h, pages, n_pages, page_entries, unroll, flags, x, y, R, (cudaStream_t)stream);
+  return spmv_paged_impl<float>(h, pages, n_pages, page_entries, unroll, flags, 0.f, x, y, R, (cudaStream_t)stream);
+}
+
+extern "C" int edgpu_spmv_paged_shift_c64(const edgpu_csr* h, const void* pages, int64_t n_pages, int page_entries,
+                                          int unroll, int flags, float shift, const float* x, float* y, int R,
+                                          void* stream) {
+  return spmv_paged_impl<float>(h, pages, n_pages, page_entries, unroll, flags, shift, x, y, R, (cudaStream_t)stream);
 }

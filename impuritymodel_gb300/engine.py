@@ -883,13 +883,14 @@ class Engine:
             csr.mixed()
             xr = torch.view_as_real(x.to(torch.complex64).contiguous())
             y = torch.empty((n, r), dtype=torch.complex64, device=self.device)
+            # the float32 copy holds H - shift*I: the kernels add shift*x as they store a row
+            if csr.mixed_shift and n != nx:
+                raise RuntimeError("spmv: a shifted copy needs a square matrix")
             if self.spmv_planned_ok(r, precision) and csr.nnz:
-                self.spmv_into(csr, xr, torch.view_as_real(y), r, precision, mapping)
+                self.spmv_into(csr, xr, torch.view_as_real(y), r, precision, mapping, shift=csr.mixed_shift)
             else:
-                L.check(self.lib.edgpu_spmv_c64(C.byref(csr.struct()), _ptr(xr), _ptr(torch.view_as_real(y)), r,
-                                                self.stream), "spmv_c64")
-            if csr.mixed_shift:
-                y += csr.mixed_shift * x.to(torch.complex64)  # float32 copy holds H - shift*I
+                L.check(self.lib.edgpu_spmv_shift_c64(C.byref(csr.struct()), float(csr.mixed_shift), _ptr(xr),
+                                                      _ptr(torch.view_as_real(y)), r, self.stream), "spmv_c64")
             return y
         xr = torch.view_as_real(x.contiguous())
         y = torch.empty((n, r), dtype=torch.complex128, device=self.device)
@@ -1011,32 +1012,41 @@ class Engine:
         return get_tuner().pick("spmv", self.spmv_key(csr, R, precision), self.spmv_candidates(csr, R, precision),
                                 lambda c: self._spmv_planned(csr, xr, yr, R, precision, c))
 
-    def _spmv_planned(self, csr, xr, yr, R, precision, mapping):
+    def _spmv_planned(self, csr, xr, yr, R, precision, mapping, shift=0.0):
         kernel, w, hm, u, last, flags = mapping
         sched, nh = self.spmv_plan(csr, w, hm)
+        lib, s = self.lib, C.byref(csr.struct())
         if kernel == "tma":
             buf, npg = self.spmv_pages(csr, w, hm, R // 2, last, self._pages_kind(csr, precision))
-            L.check(self.lib.edgpu_spmv_paged_tma_c64(C.byref(csr.struct()), _ptr(buf), npg, int(last), int(u),
-                                                      _ptr(xr), _ptr(yr), int(R), _ptr(self.status), self.stream),
-                    "spmv_paged_tma")
+            L.check(lib.edgpu_spmv_paged_tma_c64(s, _ptr(buf), npg, int(last), int(u), _ptr(xr), _ptr(yr), int(R),
+                                                 _ptr(self.status), self.stream), "spmv_paged_tma")
+            if shift:
+                yr += float(shift) * xr
             return
         if kernel == "pages":
             lanes = R // (2 if precision else 1)
             buf, npg = self.spmv_pages(csr, w, hm, lanes, last, self._pages_kind(csr, precision))
-            fn = self.lib.edgpu_spmv_paged_c64 if precision else self.lib.edgpu_spmv_paged
-            L.check(fn(C.byref(csr.struct()), _ptr(buf), npg, int(last), int(u), int(flags), _ptr(xr), _ptr(yr),
-                       int(R), self.stream), "spmv_paged")
+            args = (s, _ptr(buf), npg, int(last), int(u), int(flags))
+            if precision:
+                rc = lib.edgpu_spmv_paged_shift_c64(*args, float(shift), _ptr(xr), _ptr(yr), int(R), self.stream)
+            else:
+                rc = lib.edgpu_spmv_paged(*args, _ptr(xr), _ptr(yr), int(R), self.stream)
+            L.check(rc, "spmv_paged")
             return
-        fn = self.lib.edgpu_spmv_planned_c64 if precision else self.lib.edgpu_spmv_planned
-        L.check(fn(C.byref(csr.struct()), _ptr(sched), nh, int(u), int(last), _ptr(xr), _ptr(yr), int(R), self.stream),
-                "spmv_planned")
+        args = (s, _ptr(sched), nh, int(u), int(last))
+        if precision:
+            rc = lib.edgpu_spmv_planned_shift_c64(*args, float(shift), _ptr(xr), _ptr(yr), int(R), self.stream)
+        else:
+            rc = lib.edgpu_spmv_planned(*args, _ptr(xr), _ptr(yr), int(R), self.stream)
+        L.check(rc, "spmv_planned")
 
-    def spmv_into(self, csr, xr, yr, R, precision=0, mapping=None):
+    def spmv_into(self, csr, xr, yr, R, precision=0, mapping=None, shift=0.0):
         """yr = csr @ xr on real views of complex [rows][R] buffers (no allocation once the
-        plan exists): the launch the H.v roofline times.  Returns the mapping used."""
+        plan exists): the launch the H.v roofline times.  ``shift`` (complex64 vectors, square
+        matrix): shift * xr is added in the same launch.  Returns the mapping used."""
         if mapping is None:
             mapping = self.spmv_mapping(csr, xr, yr, R, precision)
-        self._spmv_planned(csr, xr, yr, R, precision, tuple(mapping))
+        self._spmv_planned(csr, xr, yr, R, precision, tuple(mapping), shift)
         return tuple(mapping)
 
     def cfrac(self, alpha, beta, k_len, omega, delta, e, scale, precision=0):

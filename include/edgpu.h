@@ -222,6 +222,9 @@ int edgpu_spmv(const edgpu_csr* h, const double* x, double* y, int R, void* stre
 
 /* Same with complex64 vectors and float32 accumulation (mixed-precision form). */
 int edgpu_spmv_c64(const edgpu_csr* h, const float* x, float* y, int R, void* stream);
+/* y = H x + shift x (the float copies hold H minus a multiple of the identity), here and in the
+ * _shift_c64 forms of the scheduled and paged products below; shift = 0 is the plain product. */
+int edgpu_spmv_shift_c64(const edgpu_csr* h, float shift, const float* x, float* y, int R, void* stream);
 
 /*
  * Row schedule for edgpu_spmv_planned (built once per matrix).  sched[n] (device, int32)
@@ -247,6 +250,8 @@ int edgpu_spmv_planned(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy
                        const double* x, double* y, int R, void* stream);
 int edgpu_spmv_planned_c64(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int unroll, int block,
                            const float* x, float* y, int R, void* stream);
+int edgpu_spmv_planned_shift_c64(const edgpu_csr* h, const int32_t* sched, int64_t n_heavy, int unroll, int block,
+                                 float shift, const float* x, float* y, int R, void* stream);
 
 /*
  * Paged copy of a scheduled matrix, for edgpu_spmv_paged[_c64].  In schedule order, each
@@ -279,6 +284,8 @@ int edgpu_spmv_paged(const edgpu_csr* h, const void* pages, int64_t n_pages, int
                      const double* x, double* y, int R, void* stream);
 int edgpu_spmv_paged_c64(const edgpu_csr* h, const void* pages, int64_t n_pages, int page_entries, int unroll,
                          int flags, const float* x, float* y, int R, void* stream);
+int edgpu_spmv_paged_shift_c64(const edgpu_csr* h, const void* pages, int64_t n_pages, int page_entries, int unroll,
+                               int flags, float shift, const float* x, float* y, int R, void* stream);
 
 /*
  * The same product from the same pages with the x rows brought into shared memory by the

@@ -308,3 +308,28 @@ def test_training_step(eng, batch, words):
     bound = depth * float((2.0 / batch * (one.predict(states) - log_w).abs()).sum() + 1.0)
     assert abs(float(one.G[-1] - two.G[-1])) <= bound
     assert len(losses) == 1 and abs(float(losses[0] - loss)) <= depth * abs(float(loss))
+
+
+@pytest.mark.parametrize("R,mapping", [
+    (1, None), (3, None), (5, None),       # odd: a run per thread
+    (10, None), (34, None),                # row kernel, two runs per thread
+    (2, ("sched", 256, 16, 4, 128, 0)), (64, ("sched", 0, 32, 8, 256, 0)),
+    (4, ("pages", 256, 16, 4, 512, 0)), (16, ("pages", 4096, 16, 8, 256, 3)), (32, ("pages", 0, 16, 4, 1024, 1)),
+])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_shifted_product(eng, R, mapping, cplx):
+    """y = H x from the float32 copy of H - shift I, shift x added in the same launch."""
+    n = 1003
+    csr, H = _random_csr(eng, n, R, cplx, heavy=(0, 1, 500))
+    diag = csr.col == torch.repeat_interleave(torch.arange(n, device=eng.device), csr.row_ptr[1:] - csr.row_ptr[:-1])
+    (csr.val_c[:, 0] if cplx else csr.val_r)[diag] -= 700.0
+    H = H - 700.0 * scipy.sparse.identity(n)
+    csr.mixed()
+    assert abs(csr.mixed_shift + 700.0) < 1.0
+    g = np.random.default_rng(R)
+    x = (g.normal(size=(n, R)) + 1j * g.normal(size=(n, R))).astype(np.complex64)
+    y = eng.spmv(csr, torch.from_numpy(x).to(eng.device), precision=1, mapping=mapping).cpu().numpy()
+    # float32: values and products round by 2^-24 each, sums of up to ~90 terms in any order
+    A = abs(H - csr.mixed_shift * scipy.sparse.identity(n))
+    bound = 2.0 ** -24 * (95 * (A @ abs(x)) + 4 * 701.0 * abs(x)) * 2
+    assert (abs(y - H @ x.astype(np.complex128)) <= bound).all()

@@ -94,6 +94,10 @@ SIGNATURES = {
     "edgpu_apply_groups_gather": (_I, [_I, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _I, _P, _SZ, _P]),
     "edgpu_apply_vector": (_I, [_I, _P, _P, _I64, C.POINTER(Terms), C.POINTER(Restrictions), _P, _P, _P, _P, _P]),
     "edgpu_sort_states_workspace": (_SZ, [_I, _I64]),
+    "edgpu_state_stats": (_I, [_I, _P, _I64, _P, _P]),
+    "edgpu_sort_packing": (_I, [_I, C.POINTER(C.c_uint64)]),
+    "edgpu_sort_states_packed_workspace": (_SZ, [_I, _I64]),
+    "edgpu_sort_states_packed": (_I, [_I, _P, _P, _I64, C.POINTER(C.c_uint64), _P, _SZ, _P]),
     "edgpu_sort_states": (_I, [_I, _P, _P, _I64, C.POINTER(C.c_uint64), _P, _SZ, _P]),
     "edgpu_vary_mask": (_I, [_I, _P, _I64, _P, _P]),
     "edgpu_scan_workspace": (_SZ, [_I64]),

@@ -507,3 +507,206 @@ extern "C" int edgpu_lookup_states(int n_words, const uint64_t* basis, int64_t n
   });
   return check_launch();
 }
+
+namespace edgpu {
+
+// ---------------------------------------------------------------------------------------
+// Large inputs of nearly full or nearly empty states (edgpu_sort_states_packed).
+//
+// The states of a sector differ in a few orbitals out of hundreds, spread over every byte: 316
+// spin-orbitals took 40 radix passes of 44 bytes a key (1.3 ms for 438 000 states).  Where every
+// state has at most a few zeros (or ones) among the bits that vary at all, their positions,
+// ascending, are the state: at the first bit in which two states differ one of them has its next
+// zero there and the other one a later zero or none, so comparing the position lists (none = the
+// largest) compares the states; for ones the order of the positions is turned round.  Three
+// positions of 9 bits are four passes of 12 bytes, and one gather of the states at the end
+// (0.12 ms there).
+// ---------------------------------------------------------------------------------------
+
+// out: [0, W) bits that vary, [W] smallest and [W + 1] largest number of ones, [W + 2, 2 W + 2) the
+// first state.
+template <int W>
+__global__ void stats_kernel(const uint64_t* keys, int64_t n, unsigned long long* out) {
+  uint64_t acc[W], k0[W];
+  unsigned lo = 64 * W, hi = 0;
+#pragma unroll
+  for (int q = 0; q < W; ++q) {
+    acc[q] = 0;
+    k0[q] = keys[q];
+  }
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    unsigned c = 0;
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+      const uint64_t k = keys[i * W + q];
+      acc[q] |= k ^ k0[q];
+      c += __popcll(k);
+    }
+    lo = c < lo ? c : lo;
+    hi = c > hi ? c : hi;
+  }
+  __shared__ unsigned long long sv[W];
+  __shared__ unsigned slo, shi;
+  if (threadIdx.x < W) sv[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    slo = 64 * W;
+    shi = 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < W; ++q) {
+    uint64_t v = acc[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0 && v) atomicOr(&sv[q], (unsigned long long)v);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(&slo, lo);
+    atomicMax(&shi, hi);
+  }
+  __syncthreads();
+  if (threadIdx.x < W && sv[threadIdx.x]) atomicOr(out + threadIdx.x, sv[threadIdx.x]);
+  if (threadIdx.x == 0) {
+    atomicMin(out + W, (unsigned long long)slo);
+    atomicMax(out + W + 1, (unsigned long long)shi);
+  }
+  if (blockIdx.x == 0 && threadIdx.x < W) out[W + 2 + threadIdx.x] = keys[threadIdx.x];
+}
+
+struct VaryMask {
+  uint64_t w[EDGPU_MAX_WORDS];
+};
+
+// The positions of the varying zeros (ones) as one key of `count` fields of `bits` bits.
+template <int W>
+__global__ void pack_kernel(const uint64_t* keys, int64_t n, VaryMask vary, int ones, int bits, int count,
+                            uint64_t* packed, uint32_t* idx) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t none = (1ull << bits) - 1;
+    uint64_t key = 0;
+    int used = 0;
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+      const uint64_t k = keys[i * W + q];
+      uint64_t z = (ones ? k : ~k) & vary.w[q];
+      while (z && used < count) {
+        const int p = __clzll(z);
+        z &= ~(1ull << (63 - p));
+        const uint64_t pos = (uint64_t)(64 * q + p);
+        key = (key << bits) | (ones ? none - pos : pos);
+        ++used;
+      }
+    }
+    for (; used < count; ++used) key = (key << bits) | (ones ? 0ull : none);
+    packed[i] = key;
+    idx[i] = (uint32_t)i;
+  }
+}
+
+template <int W>
+__global__ void gather_states_kernel(const uint64_t* src, const uint32_t* psrc, const uint32_t* idx, uint64_t* dst,
+                                     uint32_t* pdst, int64_t n) {
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n * W; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = t / W;
+    const int q = (int)(t - i * W);
+    const uint32_t from = idx[i];
+    dst[t] = src[(int64_t)from * W + q];
+    if (q == 0) pdst[i] = psrc[from];
+  }
+}
+
+// How states with these statistics are packed: fields of `bits` bits, `count` of them (0: not at all).
+struct Packing {
+  int ones, bits, count;
+};
+
+Packing choose_packing(int W, const uint64_t* stats) {
+  int fixed_ones = 0, vary_bytes = 0;
+  for (int q = 0; q < W; ++q) {
+    fixed_ones += __builtin_popcountll(stats[W + 2 + q] & ~stats[q]);
+    for (int b = 0; b < 8; ++b) vary_bytes += ((stats[q] >> (8 * b)) & 0xFF) != 0;
+  }
+  int varying = 0;
+  for (int q = 0; q < W; ++q) varying += __builtin_popcountll(stats[q]);
+  Packing best{0, 0, 0};
+  int bits = 1;
+  while ((1 << bits) - 1 < 64 * W) ++bits;  // every position and "none"
+  for (int ones = 0; ones < 2; ++ones) {
+    // most ones (zeros) a state has among the varying bits
+    const int count = ones ? (int)stats[W + 1] - fixed_ones : varying - ((int)stats[W] - fixed_ones);
+    if (count < 1 || count * bits > 64) continue;
+    if (best.count == 0 || count < best.count) best = Packing{ones, bits, count};
+  }
+  // passes of 12 bytes a key and a gather (three times the state) against passes of the whole state
+  if (best.count && (best.count * best.bits + 7) / 8 * 12 + 3 * (8 * W + 4) >= vary_bytes * (8 * W + 4)) best.count = 0;
+  return best;
+}
+
+}  // namespace edgpu
+
+extern "C" int edgpu_state_stats(int n_words, const uint64_t* keys, int64_t n, uint64_t* stats, void* stream) {
+  if (n_words < 1 || n_words > EDGPU_MAX_WORDS || !keys || !stats || n < 1) return EDGPU_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (cudaMemsetAsync(stats, 0, sizeof(uint64_t) * (2 * (size_t)n_words + 2), s) != cudaSuccess ||
+      cudaMemsetAsync(stats + n_words, 0xFF, sizeof(uint64_t), s) != cudaSuccess)
+    return EDGPU_ERR_CUDA;
+  EDGPU_DISPATCH_W(n_words, {
+    stats_kernel<W><<<grid_for(n, 1024), 256, 0, s>>>(keys, n, reinterpret_cast<unsigned long long*>(stats)); note_launch();
+  });
+  return check_launch();
+}
+
+extern "C" int edgpu_sort_packing(int n_words, const uint64_t* stats) {
+  if (n_words < 1 || n_words > EDGPU_MAX_WORDS || !stats) return -1;
+  const Packing p = choose_packing(n_words, stats);
+  return p.count * p.bits;
+}
+
+extern "C" size_t edgpu_sort_states_packed_workspace(int n_words, int64_t n) {
+  const size_t a = edgpu_sort_states_workspace(n_words, n);
+  const size_t b = ((size_t)n * (8 + 4 + 8 * (size_t)n_words + 4) + 1024) + edgpu_sort_states_workspace(1, n);
+  return a > b ? a : b;
+}
+
+extern "C" int edgpu_sort_states_packed(int n_words, uint64_t* keys, uint32_t* payload, int64_t n,
+                                        const uint64_t* stats, void* workspace, size_t workspace_bytes, void* stream) {
+  if (n_words < 1 || n_words > EDGPU_MAX_WORDS || n < 0) return EDGPU_ERR_ARG;
+  if (n <= 1) return EDGPU_OK;
+  if (!keys || !payload || !stats) return EDGPU_ERR_ARG;
+  const Packing pk = choose_packing(n_words, stats);
+  // small inputs are sorted in one CTA's shared memory whatever their bits
+  if (pk.count == 0 || n >= (1ll << 32) || small_sort_fits(n_words, n) || small_sort_fits(1, n))
+    return edgpu_sort_states(n_words, keys, payload, n, stats, workspace, workspace_bytes, stream);
+  if (workspace_bytes < edgpu_sort_states_packed_workspace(n_words, n)) return EDGPU_ERR_WORKSPACE;
+  cudaStream_t s = (cudaStream_t)stream;
+  unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
+  size_t off = 0;
+  auto carve = [&](size_t bytes) {
+    unsigned char* p = ws + off;
+    off += (bytes + 255) & ~(size_t)255;
+    return p;
+  };
+  uint64_t* packed = reinterpret_cast<uint64_t*>(carve(8 * (size_t)n));
+  uint64_t* src = reinterpret_cast<uint64_t*>(carve(8 * (size_t)n * n_words));
+  uint32_t* idx = reinterpret_cast<uint32_t*>(carve(4 * (size_t)n));
+  uint32_t* psrc = reinterpret_cast<uint32_t*>(carve(4 * (size_t)n));
+  VaryMask vary{};
+  for (int q = 0; q < n_words; ++q) vary.w[q] = stats[q];
+  EDGPU_DISPATCH_W(n_words, {
+    pack_kernel<W><<<grid_for(n, 256), 256, 0, s>>>(keys, n, vary, pk.ones, pk.bits, pk.count, packed, idx); note_launch();
+  });
+  int rc = check_launch();
+  if (rc) return rc;
+  const int total = pk.bits * pk.count;
+  const uint64_t mask = total >= 64 ? ~0ull : (1ull << total) - 1;
+  if ((rc = edgpu_sort_states(1, packed, idx, n, &mask, ws + off, workspace_bytes - off, stream))) return rc;
+  if (cudaMemcpyAsync(src, keys, 8 * (size_t)n * n_words, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+      cudaMemcpyAsync(psrc, payload, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+    return EDGPU_ERR_CUDA;
+  EDGPU_DISPATCH_W(n_words, {
+    gather_states_kernel<W><<<grid_for(n * W, 256), 256, 0, s>>>(src, psrc, idx, keys, payload, n); note_launch();
+  });
+  return check_launch();
+}

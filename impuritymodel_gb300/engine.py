@@ -409,12 +409,11 @@ class Engine:
             L.check(self.lib.edgpu_sort_states(w, _ptr(keys), _ptr(payload), m, None, C.c_void_p(0), 0,
                                                self.stream), "sort")
             return keys, payload
-        vary = torch.empty(w, dtype=torch.int64, device=self.device)
-        L.check(self.lib.edgpu_vary_mask(w, _ptr(keys), m, _ptr(vary), self.stream), "vary_mask")
-        vm = vary.cpu().numpy().view(np.uint64).copy()
-        arr = (C.c_uint64 * w)(*[int(x) for x in vm])
-        ws, wsn = self.workspace(self.lib.edgpu_sort_states_workspace(w, m))
-        L.check(self.lib.edgpu_sort_states(w, _ptr(keys), _ptr(payload), m, arr, ws, wsn, self.stream), "sort")
+        stats = torch.empty(2 * w + 2, dtype=torch.int64, device=self.device)
+        L.check(self.lib.edgpu_state_stats(w, _ptr(keys), m, _ptr(stats), self.stream), "state_stats")
+        arr = (C.c_uint64 * (2 * w + 2))(*[int(x) for x in stats.cpu().numpy().view(np.uint64)])
+        ws, wsn = self.workspace(self.lib.edgpu_sort_states_packed_workspace(w, m))
+        L.check(self.lib.edgpu_sort_states_packed(w, _ptr(keys), _ptr(payload), m, arr, ws, wsn, self.stream), "sort")
         return keys, payload
 
     def unique_sorted(self, keys, payload=None, vals=None):

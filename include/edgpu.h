@@ -176,6 +176,18 @@ int edgpu_apply_vector(int n_words, const uint64_t* states, const double* amps, 
 size_t edgpu_sort_states_workspace(int n_words, int64_t n);
 int edgpu_sort_states(int n_words, uint64_t* keys, uint32_t* payload, int64_t n, const uint64_t* vary_mask,
                       void* workspace, size_t workspace_bytes, void* stream);
+/* Statistics of the keys for edgpu_sort_states_packed: stats [2 n_words + 2] (device) receives the
+ * bits that vary, the smallest and the largest number of ones and the first key.
+ */
+int edgpu_state_stats(int n_words, const uint64_t* keys, int64_t n, uint64_t* stats, void* stream);
+/* edgpu_sort_states (the same stable order) for keys of known statistics (host array): keys that
+ * differ in the positions of a few zeros or ones are sorted by those positions instead of byte by
+ * byte.  edgpu_sort_packing: bits of the packed key (0: sorted byte by byte).
+ */
+int edgpu_sort_packing(int n_words, const uint64_t* stats);
+size_t edgpu_sort_states_packed_workspace(int n_words, int64_t n);
+int edgpu_sort_states_packed(int n_words, uint64_t* keys, uint32_t* payload, int64_t n, const uint64_t* stats,
+                             void* workspace, size_t workspace_bytes, void* stream);
 
 /* OR over rows of (row XOR row 0) into vary_out[n_words] (device). */
 int edgpu_vary_mask(int n_words, const uint64_t* keys, int64_t n, uint64_t* vary_out, void* stream);

@@ -333,3 +333,35 @@ def test_shifted_product(eng, R, mapping, cplx):
     A = abs(H - csr.mixed_shift * scipy.sparse.identity(n))
     bound = 2.0 ** -24 * (95 * (A @ abs(x)) + 4 * 701.0 * abs(x)) * 2
     assert (abs(y - H @ x.astype(np.complex128)) <= bound).all()
+
+
+@pytest.mark.parametrize("n,words,flips,ones,packs", [
+    (8193, 5, 3, False, True),     # a few zeros in full states, the smallest size beyond one CTA
+    (50001, 5, 3, True, True),     # a few ones in empty states
+    (20000, 1, 2, False, True),    # one word: two passes and a gather instead of eight passes
+    (20000, 8, 6, False, True),    # the widest fields: 60 bits
+    (20000, 8, 7, True, False),    # too many positions for one key
+    (9001, 2, 40, False, False),   # dense states
+])
+def test_sort_of_sparse_states(eng, n, words, flips, ones, packs):
+    import ctypes as C
+
+    g = np.random.default_rng(n + words)
+    bits = np.zeros((n, 64 * words), dtype=np.uint8)
+    for _ in range(flips):  # fewer positions where some coincide; a third of the states twice
+        bits[np.arange(n), g.integers(3, 64 * words - 2, size=n)] = 1
+    bits[: n // 3] = bits[n - n // 3:]
+    bits[:, :3] = (1, 0, 1)
+    if not ones:
+        bits[:, 3:] ^= 1
+    keys = np.packbits(bits, axis=1).view(">u8").astype(np.uint64).reshape(n, words)
+    t = eng.upload_states(keys)
+    payload = torch.arange(n, dtype=torch.int32, device=eng.device) * 3
+    stats = torch.empty(2 * words + 2, dtype=torch.int64, device=eng.device)
+    eng.lib.edgpu_state_stats(words, t.data_ptr(), n, stats.data_ptr(), eng.stream)
+    arr = (C.c_uint64 * (2 * words + 2))(*[int(x) for x in stats.cpu().numpy().view(np.uint64)])
+    assert (eng.lib.edgpu_sort_packing(words, arr) > 0) == packs
+    eng.sort_states(t, payload)
+    order = np.lexsort(keys.T[::-1])  # stable, first word most significant
+    assert np.array_equal(t.cpu().numpy().view(np.uint64), keys[order])
+    assert np.array_equal(payload.cpu().numpy(), 3 * order)

@@ -1232,11 +1232,17 @@ namespace edgpu {
 constexpr int kSmallThreads = 512;
 constexpr int kSmallBatch = 8;  // CSR entries loaded together per row
 
-// Deterministic block sum (fixed thread -> partial mapping and fixed tree).
-__device__ __forceinline__ double block_sum(double v, double* red) {
+// Deterministic block sum (fixed thread -> partial mapping and fixed tree).  The first `active`
+// threads may hold a value; the other warps keep off the FP64 pipe (their sum is 0).  ROOT: one
+// thread turns the sum into its root, returned instead, and red[33] into the root's reciprocal (0
+// for 0 and NaN) -- by every thread of 16 warps these two took 6 400 cycles of FP64 issue.
+template <bool ROOT>
+__device__ __forceinline__ double block_sum(double v, double* red, int active) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (32 * warp < active) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  }
   __syncthreads();
   if (lane == 0) red[warp] = v;
   __syncthreads();
@@ -1245,7 +1251,15 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
     double t = lane < nw ? red[lane] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (lane == 0) red[32] = t;
+    if (lane == 0) {
+      if (ROOT) {
+        const double b = sqrt(t);
+        red[32] = b;
+        red[33] = b > 0.0 ? 1.0 / b : 0.0;
+      } else {
+        red[32] = t;
+      }
+    }
   }
   __syncthreads();
   return red[32];
@@ -1256,11 +1270,23 @@ __device__ __forceinline__ float2 to_v(double2 a, float) { return make_float2((f
 
 // Upstream's Lanczos recurrence (finite.py:1974-1992) for run r entirely in shared memory:
 // x = v_j, p = v_{j-1}, y = H v_j then w.  One CTA per run, persistent over runs.
-template <typename T, bool VALC>
+//
+// Bound by FP64 issue (~16 cycles a warp instruction; two CTAs share an SM's pipe).  SLICED (real H):
+// the products walk the rows by length on the sliced copy (slices_kernel), a warp's rows of nearly
+// equal lengths and their entries side by side in memory, instead of 32 consecutive rows whose
+// longest sets the pace (1.52 issue slots an entry on the 1770-row sector, 1.03 sliced).  Every row
+// still adds its entries in their order, and alpha's per-thread sums run over the rows i = tid,
+// tid + 512, ... after a barrier, so the bits are those of the unsliced form: a recurrence without
+// reorthogonalisation turns rounding into visible changes.  750 runs x 150 steps of the 1770-row
+// sector: 17.6 ms (19.2 from the CSR rows with the root in every thread; the 46.6 operations a row
+// and step that these bits need issue in 15.9); 750 runs of a 200-row
+// matrix 6.4 -> 4.3 ms, 9 runs of 600 rows 2.96 -> 2.46.
+template <typename T, bool VALC, bool SLICED>
 __global__ void __launch_bounds__(kSmallThreads) lanczos_small_kernel(
-    int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ col, const T* __restrict__ vals, int R,
-    const double2* __restrict__ v0, const int32_t* __restrict__ k_max, int K, double* __restrict__ alpha,
-    double* __restrict__ beta, int32_t* status) {
+    int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ col, const T* __restrict__ vals,
+    const int32_t* __restrict__ sinfo, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
+    const T* __restrict__ eval, int R, const double2* __restrict__ v0, const int32_t* __restrict__ k_max, int K,
+    double* __restrict__ alpha, double* __restrict__ beta, int32_t* status) {
   using V = typename Cx<T>::V;
   extern __shared__ __align__(16) unsigned char sm[];
   V* A = reinterpret_cast<V*>(sm);
@@ -1268,6 +1294,9 @@ __global__ void __launch_bounds__(kSmallThreads) lanczos_small_kernel(
   V* Cv = B + n;
   double* red = reinterpret_cast<double*>(Cv + n);
   const int tid = threadIdx.x, bs = blockDim.x;
+  const int active = n < bs ? (int)n : bs;
+  const bool sliced = SLICED && soff[0] >= 0;
+  const int npad = (int)((n + 31) & ~(int64_t)31);
   for (int r = blockIdx.x; r < R; r += gridDim.x) {
     const int km = k_max[r];
     if (km <= 0) continue;
@@ -1282,29 +1311,67 @@ __global__ void __launch_bounds__(kSmallThreads) lanczos_small_kernel(
     double bprev = 0.0;
     for (int j = 0; j < km; ++j) {
       double acc = 0.0;
-      for (int64_t i = tid; i < n; i += bs) {
-        T yr = 0, yi = 0;
-        const int64_t e1 = rp[i + 1];
-        for (int64_t e = rp[i]; e < e1; ++e) {
-          const V xv = x[col[e]];
-          if (VALC) {
-            const T hr = vals[2 * e], hi = vals[2 * e + 1];
-            yr += hr * xv.x - hi * xv.y;
-            yi += hr * xv.y + hi * xv.x;
-          } else {
-            const T h = vals[e];
-            yr += h * xv.x;
-            yi += h * xv.y;
+      if (SLICED && sliced) {
+        for (int q = tid; q < npad; q += bs) {
+          const int info = __ldg(sinfo + q);
+          if (info < 0) continue;
+          const int len = info >> 16;
+          const int32_t* c = ecol + __ldg(soff + (q >> 5)) + (q & 31);
+          const T* h = eval + (c - ecol);
+          T yr = 0, yi = 0;
+          for (int e = 0; e < len; e += kSmallBatch) {
+            int cc[kSmallBatch];
+            T hh[kSmallBatch];
+#pragma unroll
+            for (int u = 0; u < kSmallBatch; ++u) {
+              const bool ok = e + u < len;
+              cc[u] = ok ? __ldg(c + 32 * (e + u)) : 0;
+              hh[u] = ok ? __ldg(h + 32 * (e + u)) : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < kSmallBatch; ++u) {
+              if (e + u < len) {
+                const V xv = x[cc[u]];
+                yr += hh[u] * xv.x;
+                yi += hh[u] * xv.y;
+              }
+            }
           }
+          V yv;
+          yv.x = yr;
+          yv.y = yi;
+          y[info & 0xffff] = yv;
         }
-        V yv;
-        yv.x = yr;
-        yv.y = yi;
-        y[i] = yv;
-        const V xi = x[i];
-        acc += (double)yr * (double)xi.x + (double)yi * (double)xi.y;
+        __syncthreads();
+        for (int64_t i = tid; i < n; i += bs) {
+          const V yv = y[i], xi = x[i];
+          acc += (double)yv.x * (double)xi.x + (double)yv.y * (double)xi.y;
+        }
+      } else {
+        for (int64_t i = tid; i < n; i += bs) {
+          T yr = 0, yi = 0;
+          const int64_t e1 = rp[i + 1];
+          for (int64_t e = rp[i]; e < e1; ++e) {
+            const V xv = x[col[e]];
+            if (VALC) {
+              const T hr = vals[2 * e], hi = vals[2 * e + 1];
+              yr += hr * xv.x - hi * xv.y;
+              yi += hr * xv.y + hi * xv.x;
+            } else {
+              const T h = vals[e];
+              yr += h * xv.x;
+              yi += h * xv.y;
+            }
+          }
+          V yv;
+          yv.x = yr;
+          yv.y = yi;
+          y[i] = yv;
+          const V xi = x[i];
+          acc += (double)yr * (double)xi.x + (double)yi * (double)xi.y;
+        }
       }
-      const double a = block_sum(acc, red);
+      const double a = block_sum<false>(acc, red, active);
       if (tid == 0) alpha[(int64_t)r * K + j] = a;
       if (j + 1 == km) break;
       acc = 0.0;
@@ -1318,12 +1385,12 @@ __global__ void __launch_bounds__(kSmallThreads) lanczos_small_kernel(
         y[i] = w;
         acc += (double)w.x * (double)w.x + (double)w.y * (double)w.y;
       }
-      const double b = sqrt(block_sum(acc, red));
+      const double b = block_sum<true>(acc, red, active);
       if (tid == 0) {
         beta[(int64_t)r * K + j] = b;
         if (!(b > 0.0)) atomicExch(status, (int32_t)(b == 0.0 ? EDGPU_ERR_BREAKDOWN : EDGPU_ERR_NAN));
       }
-      const T inv = b > 0.0 ? (T)(1.0 / b) : (T)0;
+      const T inv = (T)red[33];
       for (int64_t i = tid; i < n; i += bs) {
         const V w = y[i];
         V o;
@@ -1457,11 +1524,14 @@ __global__ void __launch_bounds__(THREADS, MINB) lanczos_small_df_kernel(
 // placement by warp 0 with __match_any_sync ranks, then the fill by every thread.  When the
 // slices would need more than `cap` entries (possible only for rows with repeated columns)
 // every slot gets length 0 and *status EDGPU_ERR_WORKSPACE, so nothing reads past the arrays.
-__global__ void __launch_bounds__(1024) df_slices_kernel(int64_t n, const int64_t* __restrict__ rp,
-                                                         const int32_t* __restrict__ col,
-                                                         const float2* __restrict__ hv, int32_t* __restrict__ sinfo,
-                                                         int32_t* __restrict__ soff, int32_t* __restrict__ ecol,
-                                                         float2* __restrict__ eval, int64_t cap, int32_t* status) {
+// SLOTS = false (the FP64 kernel, which keeps its vectors in row order): stored columns are rows, and
+// where the slices do not fit soff[0] becomes -1 and the caller's kernel reads the CSR arrays.
+template <typename E, bool SLOTS>
+__global__ void __launch_bounds__(1024) slices_kernel(int64_t n, const int64_t* __restrict__ rp,
+                                                      const int32_t* __restrict__ col, const E* __restrict__ hv,
+                                                      int32_t* __restrict__ sinfo, int32_t* __restrict__ soff,
+                                                      int32_t* __restrict__ ecol, E* __restrict__ eval, int64_t cap,
+                                                      int32_t* status) {
   extern __shared__ int32_t hist[];  // [n + 1] bucket offsets (row lengths 0..n)
   __shared__ int32_t s_max;
   __shared__ int32_t s_over;
@@ -1476,6 +1546,10 @@ __global__ void __launch_bounds__(1024) df_slices_kernel(int64_t n, const int64_
   for (int64_t i = tid; i < n; i += blockDim.x) lmax = max(lmax, (int)(rp[i + 1] - rp[i]));
   atomicMax(&s_max, lmax);
   __syncthreads();
+  if (!SLOTS && s_max > n) {
+    if (tid == 0) soff[0] = -1;
+    return;
+  }
   if (s_max > n) {  // repeated columns: no sliced layout
     for (int q = tid; q < npad; q += blockDim.x) sinfo[q] = q < n ? q : -1;
     for (int q = tid; q <= nslices; q += blockDim.x) soff[q] = 0;
@@ -1525,6 +1599,10 @@ __global__ void __launch_bounds__(1024) df_slices_kernel(int64_t n, const int64_
     if (off > cap) s_over = 1;
   }
   __syncthreads();
+  if (!SLOTS && s_over) {
+    if (tid == 0) soff[0] = -1;
+    return;
+  }
   if (s_over) {
     for (int q = tid; q < npad; q += blockDim.x) sinfo[q] = sinfo[q] < 0 ? -1 : (sinfo[q] & 0xffff);
     for (int q = tid; q <= nslices; q += blockDim.x) soff[q] = 0;
@@ -1539,8 +1617,8 @@ __global__ void __launch_bounds__(1024) df_slices_kernel(int64_t n, const int64_
     const int len = info < 0 ? 0 : (info >> 16);
     const int64_t e0 = info < 0 ? 0 : rp[info & 0xffff];
     for (int e = 0; e < m; ++e) {
-      ecol[base + 32 * e] = e < len ? hist[col[e0 + e]] : 0;
-      eval[base + 32 * e] = e < len ? hv[e0 + e] : make_float2(0.f, 0.f);
+      ecol[base + 32 * e] = e < len ? (SLOTS ? hist[col[e0 + e]] : col[e0 + e]) : 0;
+      eval[base + 32 * e] = e < len ? hv[e0 + e] : E{};
     }
   }
 }
@@ -1676,19 +1754,54 @@ static size_t small_df_smem_bytes(int64_t n) {
 
 bool small_fits(int64_t n, int precision) { return small_smem_bytes(n, precision) <= 200 * 1024; }
 
+static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// Entries the sliced copy of a real H is given in the FP64 form's workspace (beside its slot table);
+// 0 where the smallest workspace edgpu_lanczos accepts for (n, R) cannot hold it, and for calls of
+// fewer than eight steps a CTA slot, which do not repay the one-CTA launch that makes the copy:
+// 152 runs of 1770 rows take 193 us sliced and 166 from the CSR rows at 2 steps, 434 and 447 at 8,
+// 933 and 998 at 20; 750 runs of 2 steps 414 and 451.
+static int64_t fp64_slices_cap(int64_t n, int64_t nnz, int R, int K) {
+  const int64_t npad = (n + 31) & ~(int64_t)31, cap = nnz + nnz / 4 + 32 * 64;
+  const size_t need = 256 + align256(4 * (size_t)npad) + align256(4 * (size_t)(npad / 32 + 1)) + align256(4 * (size_t)cap) +
+                      align256(8 * (size_t)cap);
+  const int64_t waves = (R + grid_cap() - 1) / grid_cap();
+  return waves * K >= 8 && need <= 3 * sizeof(double2) * (size_t)n * R ? cap : 0;
+}
+
 template <typename T, bool VALC>
 int launch_small(const edgpu_csr* h, const T* vals, const double* v0, int R, const int32_t* k_max, int K,
-                 double* alpha, double* beta, int32_t* status, int precision, cudaStream_t s) {
-  const size_t smem = small_smem_bytes(h->n, precision);
-  auto kern = lanczos_small_kernel<T, VALC>;
+                 double* alpha, double* beta, int32_t* status, int precision, void* ws, cudaStream_t s) {
+  const int64_t n = h->n;
+  const size_t smem = small_smem_bytes(n, precision);
+  int32_t *sinfo = nullptr, *soff = nullptr, *ecol = nullptr;
+  T* eval = nullptr;
+  auto kern = lanczos_small_kernel<T, VALC, false>;
+  if constexpr (sizeof(T) == 8 && !VALC) {
+    const int64_t cap = ws ? fp64_slices_cap(n, h->nnz, R, K) : 0;
+    if (cap > 0) {
+      unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
+      const int64_t npad = (n + 31) & ~(int64_t)31;
+      eval = reinterpret_cast<T*>(base);
+      ecol = reinterpret_cast<int32_t*>(base + align256(8 * (size_t)cap));
+      sinfo = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(ecol) + align256(4 * (size_t)cap));
+      soff = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(sinfo) + align256(4 * (size_t)npad));
+      const size_t hist_bytes = sizeof(int32_t) * (size_t)(n + 1);
+      auto slices = slices_kernel<double, false>;
+      cudaFuncSetAttribute(slices, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes);
+      slices<<<1, 1024, hist_bytes, s>>>(n, h->row_ptr, h->col, vals, sinfo, soff, ecol, eval, cap, status);
+      note_launch();
+      kern = lanczos_small_kernel<T, VALC, true>;
+    }
+  }
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSmallThreads, smem);
   if (per_sm < 1) per_sm = 1;
   int grid = grid_cap() * per_sm;
   if (grid > R) grid = R;
-  kern<<<grid, kSmallThreads, smem, s>>>(h->n, h->row_ptr, h->col, vals, R, reinterpret_cast<const double2*>(v0), k_max,
-                                         K, alpha, beta, status);
+  kern<<<grid, kSmallThreads, smem, s>>>(n, h->row_ptr, h->col, vals, sinfo, soff, ecol, eval, R,
+                                         reinterpret_cast<const double2*>(v0), k_max, K, alpha, beta, status);
   note_launch();
   return check_launch();
 }
@@ -1749,8 +1862,6 @@ static int pick_df_config(const void* const* kerns, size_t smem, int R, int* per
   return best;
 }
 
-static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
-
 int launch_small_df(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, double* alpha,
                     double* beta, int32_t* status, void* ws, cudaStream_t s) {
   static const SmallDfKern csr_kerns[5] = {lanczos_small_df_kernel<512, 2>, lanczos_small_df_kernel<256, 4>,
@@ -1785,8 +1896,9 @@ int launch_small_df(const edgpu_csr* h, const double* v0, int R, const int32_t* 
         int32_t* ecol = reinterpret_cast<int32_t*>(base + b_p + b_info + b_off);
         float2* eval = reinterpret_cast<float2*>(base + b_p + b_info + b_off + b_col);
         const size_t hist_bytes = sizeof(int32_t) * (size_t)(n + 1);
-        cudaFuncSetAttribute(df_slices_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes);
-        df_slices_kernel<<<1, 1024, hist_bytes, s>>>(n, h->row_ptr, h->col, reinterpret_cast<const float2*>(h->val_df),
+        auto slices = slices_kernel<float2, true>;
+        cudaFuncSetAttribute(slices, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes);
+        slices<<<1, 1024, hist_bytes, s>>>(n, h->row_ptr, h->col, reinterpret_cast<const float2*>(h->val_df),
                                                      sinfo, soff, ecol, eval, cap, status);
         note_launch();
         sl_kerns[c]<<<grid, kDfThreads[c], smem, s>>>(n, sinfo, soff, ecol, eval, R,
@@ -1817,12 +1929,12 @@ int lanczos_small(const edgpu_csr* h, const double* v0, int R, const int32_t* k_
     precision = 0;  // complex H: FP64
   }
   if (precision == 0) {
-    if (h->val_c) return launch_small<double, true>(h, h->val_c, v0, R, k_max, K, alpha, beta, status, 0, s);
-    return launch_small<double, false>(h, h->val_r, v0, R, k_max, K, alpha, beta, status, 0, s);
+    if (h->val_c) return launch_small<double, true>(h, h->val_c, v0, R, k_max, K, alpha, beta, status, 0, ws, s);
+    return launch_small<double, false>(h, h->val_r, v0, R, k_max, K, alpha, beta, status, 0, ws, s);
   }
-  if (h->val_cf) return launch_small<float, true>(h, h->val_cf, v0, R, k_max, K, alpha, beta, status, 1, s);
+  if (h->val_cf) return launch_small<float, true>(h, h->val_cf, v0, R, k_max, K, alpha, beta, status, 1, ws, s);
   if (!h->val_rf) return EDGPU_ERR_ARG;
-  return launch_small<float, false>(h, h->val_rf, v0, R, k_max, K, alpha, beta, status, 1, s);
+  return launch_small<float, false>(h, h->val_rf, v0, R, k_max, K, alpha, beta, status, 1, ws, s);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -326,8 +326,10 @@ int edgpu_spmv_paged_tma_c64(const edgpu_csr* h, const void* pages, int64_t n_pa
  * float64 alpha/beta reductions, for real H in the shared-memory path; precision 3
  * anywhere else runs as 0.  Breakdown (beta == 0 before k_max) sets
  * *status_dev = EDGPU_ERR_BREAKDOWN.  Sectors whose three Krylov vectors fit in shared
- * memory run as one persistent launch with one CTA per run; larger ones as three
- * grid-wide kernels per step.  In the double-float form the CTA keeps one vector in shared
+ * memory run as one persistent launch with one CTA per run; larger ones as two
+ * grid-wide kernels per step.  In the FP64 form with real H, from eight steps a wave of CTAs on,
+ * one extra launch builds a sliced copy of H in the workspace where it fits (rows that repeat a
+ * column are read from the CSR arrays as before).  In the double-float form the CTA keeps one vector in shared
  * memory and the previous one in the workspace, and, when the workspace size returned for
  * (n, R, K) also holds it, reads H through a sliced copy (rows sorted by length in 32-row
  * column-major slices) that one extra launch builds in the workspace; a matrix whose rows
@@ -356,7 +358,7 @@ long long edgpu_launch_count(void);
  * the whole GPU and forbids cudaMalloc, or a solver loop embedded in another program where
  * an allocation would synchronise the device between time steps.  The caller passes the
  * inputs and outputs of edgpu_lanczos (no workspace); this always runs the grid-wide
- * batched Lanczos (three kernels per step) and keeps its scratch (three [n][R] vectors
+ * batched Lanczos (two kernels per step) and keeps its scratch (three [n][R] vectors
  * and partial sums, size edgpu_lanczos_workspace(n, R, K, precision)) in a static
  * device array of EDGPU_LANCZOS_NOALLOC_BYTES inside the library, which every GPU that
  * loads the library holds until the process exits.  Larger problems are rejected with

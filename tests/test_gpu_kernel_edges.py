@@ -365,3 +365,52 @@ def test_sort_of_sparse_states(eng, n, words, flips, ones, packs):
     order = np.lexsort(keys.T[::-1])  # stable, first word most significant
     assert np.array_equal(t.cpu().numpy().view(np.uint64), keys[order])
     assert np.array_equal(payload.cpu().numpy(), 3 * order)
+
+
+@pytest.mark.parametrize("n,extra,K", [
+    (9, 0, 7),       # less than a warp of rows
+    (33, 0, 20),     # fewer rows than threads, one row in the second slice
+    (513, 0, 40),    # a second pass of one row
+    (1770, 0, 40),
+    (4240, 0, 24),   # near the largest sector that fits
+    (700, 40, 24),   # rows of 40 more entries: several lengths
+    (60, 90, 24),    # a row longer than the sector (repeated columns): no sliced copy
+])
+def test_runs_on_sliced_rows(eng, n, extra, K):
+    """Long calls (sliced rows) give every run the bits that it has in a short call (CSR rows)."""
+    from impuritymodel_gb300.engine import CsrMatrix
+
+    rng = np.random.default_rng(n + extra)
+    rows, cols = [np.arange(n)], [np.arange(n)]
+    for _ in range(2):
+        i, j = rng.integers(0, n, size=(2, n))
+        rows += [i, j]
+        cols += [j, i]
+    for i in (0, n // 2):
+        j = rng.integers(0, n, size=extra)
+        rows += [np.full(extra, i), j]
+        cols += [j, np.full(extra, i)]
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    o = np.argsort(rows, kind="stable")
+    rows, cols = rows[o], cols[o]
+    vals = np.cos(1.0 + 7.0 * np.minimum(rows, cols) + 3.0 * np.maximum(rows, cols)) + 4.0 * (rows == cols)
+    rp = torch.from_numpy(np.searchsorted(rows, np.arange(n + 1)).astype(np.int64)).to(eng.device)
+    csr = CsrMatrix(rp, torch.from_numpy(cols.astype(np.int32)).to(eng.device),
+                    val_r=torch.from_numpy(vals).to(eng.device))
+    R = torch.cuda.get_device_properties(eng.device).multi_processor_count + 5
+    v = rng.normal(size=(n, R)) + 1j * rng.normal(size=(n, R))
+    v = torch.from_numpy(v / np.linalg.norm(v, axis=0)).to(eng.device)
+    k = np.full(R, K, dtype=np.int32)
+    k[1], k[2] = 0, max(1, K // 2)
+    a, b = eng.lanczos(csr, v, k, precision=0)
+    some = [0, 1, 2, R // 2, R - 1]
+    k1 = np.minimum(k[some], 7)
+    a1, b1 = eng.lanczos(csr, v[:, some].contiguous(), k1, precision=0)
+    for q, r in enumerate(some):
+        assert torch.equal(a[r, :k1[q]], a1[q, :k1[q]])
+        assert torch.equal(b[r, :max(k1[q] - 1, 0)], b1[q, :max(k1[q] - 1, 0)])
+    H = scipy.sparse.csr_matrix((vals, (rows, cols)), shape=(n, n))
+    ar, br = _recurrence(H, v[:, 0].cpu().numpy(), min(K, 12))
+    m = min(K, 12)
+    # a dozen steps of an unconverged recurrence amplify rounding by less than 1e3
+    assert np.abs(a[0, :m].cpu().numpy() - ar[:m]).max() < 1e-12 * max(abs(H).sum(1).max(), 1.0)

@@ -13,8 +13,12 @@
 #include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "df64.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace edgpu {
 
@@ -2205,6 +2209,314 @@ __global__ void __launch_bounds__(kShiftMaxThreads) shifted_small_kernel(Shifted
   }
 }
 
+// The same recurrence with a right-hand side on a cluster of 2, 4 or 8 CTAs, for calls whose
+// right-hand sides leave SMs idle (15 RIXS intermediate states on 152 SMs).
+//
+// On one CTA a step is bound by that SM's FP64 issue (16 cycles a warp instruction, of one lane or of
+// 32).  Here the rows, sorted by length, are dealt to the row CTAs one by one; every CTA keeps the whole
+// vector in shared memory for its gather and sends its rows of the next one to the others
+// (distributed shared memory).  Few shifts (kOwnTrackers) are tracked by a CTA of their own, more of
+// them by warps of every CTA.  What is left is latency, so a step has two cluster barriers and no more:
+//   1  y = H w on the unscaled w = beta_{j-1} v_j, SUB lanes a row, a component per half of them,
+//      and the partials of <w, y>, a partial per warp sent to every CTA.  Meanwhile a warp of the last
+//      CTA takes the root of |w|^2 and its reciprocal, and the trackers the pivots of step j - 1.
+//   2  one warp adds up alpha_j while the others form v_j and y - beta_{j-1} v_{j-1}; then
+//      w' = y - alpha_j v_j - beta_{j-1} v_{j-1}, sent to every row CTA, and the partials of |w'|^2,
+//      sent to the last CTA.  The trackers' verdict on step j - 1 arrives with them.
+// Roots and reciprocals (~1500 dependent cycles each) and the trackers' ~3000 thus stay off the
+// chain.  Every warp that adds up partials takes them in the same order, so that all CTAs take identical
+// branches around the barriers.
+// 15 right-hand sides, 50 shifts, ~480 steps: 360 states (15 RIXS intermediate states) 4.3 -> 2.9 ms for
+// the whole solve; a random H of 3500 rows 38 -> 20; 70 right-hand sides of 360 rows (pairs) 6.1 -> 4.9.  A
+// step of the 360 states is ~7000 cycles of latencies: 2 barriers of ~600, two sums over all lanes of
+// ~1200 each, some 30 dependent FP64 operations of 64 and more.
+constexpr int kClusterMax = 8;
+constexpr int kOwnTrackers = 64;                                         // shifts of a tracking CTA at most
+constexpr int kClusterWarps = kSmallThreads / 32;                        // main warps at most
+constexpr int kClusterThreads = kSmallThreads + 32 + kSmallThreads / 2;  // and the sums', and the trackers
+
+struct ClusterArgs {
+  ShiftedArgs a;
+  int passes;   // rounds of main_threads / SUB rows
+  int rows_on;  // row CTAs: all of the cluster, or all but the last
+};
+
+// barrier of the first `threads` threads (the main warps and the one that sums)
+__device__ __forceinline__ void cluster_bar(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+
+template <bool VALC, int SUB>
+__global__ void __launch_bounds__(kClusterThreads) shifted_cluster_kernel(ClusterArgs ca) {
+  const ShiftedArgs& g = ca.a;
+  cg::cluster_group cl = cg::this_cluster();
+  const int CL = (int)cl.num_blocks(), rank = (int)cl.block_rank(), RC = ca.rows_on;
+  const int n = (int)g.n, M = g.main_threads, mw = M >> 5, nz = g.nz, k_cap = g.k_cap;
+  constexpr int spw = 32 / SUB;  // rows of a warp
+  const int passes = ca.passes, rpp = M / SUB, nsl = passes * mw;
+  extern __shared__ __align__(16) unsigned char sm[];
+  double2* A = reinterpret_cast<double2*>(sm);
+  double2* B = A + n;
+  double* own_y = reinterpret_cast<double*>(B + n);  // [passes][M] of this thread's components
+  double* own_p = own_y + (size_t)passes * M;
+  double* sval = own_p + (size_t)passes * M;
+  uint16_t* scol = reinterpret_cast<uint16_t*>(sval + (size_t)g.ent_cap * (VALC ? 2 : 1));
+  uint16_t* len = scol + g.ent_cap;  // [n]
+  uint16_t* order = len + n;         // [passes * rpp] this CTA's rows, 0xFFFF past the last
+  __shared__ double s_alpha[kClusterMax * kClusterWarps], s_norm[kClusterMax * kClusterWarps];
+  __shared__ int s_ok[kClusterMax * kClusterWarps];
+  __shared__ int soff[2 * kSmallThreads];
+  __shared__ double s_a, s_b, s_ib, s_ib2;
+  __shared__ int sliced;
+  const int tid = threadIdx.x, bs = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const bool row_cta = rank < RC, last_cta = rank == CL - 1;
+  const bool is_main = tid < M, is_sum = warp == mw;
+  // trackers: every CTA's where they share the row CTAs, else the last CTA's
+  const int tz = tid - M - 32, tw = (bs - M - 32) >> 5;
+  const int tcs = RC == CL ? CL : 1, trank = RC == CL ? rank : 0;
+  const bool is_track = tz >= 0 && (RC == CL || last_cta);
+  const int zi = tz * tcs + trank;
+  const int comp = SUB == 4 ? (lane >> 1) & 1 : lane & 1;            // 0: real part, 1: imaginary part
+  const int d0 = SUB == 4 ? lane & 1 : 0, dstep = SUB == 4 ? 2 : 1;  // the CTAs this lane sends to
+
+  // rows by length, longest first, equal lengths in order; slot s is row s / RC of CTA s % RC
+  for (int i = tid; i < n; i += bs) {
+    const int64_t l = g.rp[i + 1] - g.rp[i];
+    len[i] = (uint16_t)(l < 0xFFFF ? l : 0xFFFF);
+  }
+  for (int q = tid; q < passes * rpp; q += bs) order[q] = 0xFFFF;
+  cl.sync();
+  for (int i = rank + CL * tid; i < n; i += CL * bs) {
+    const int l = len[i];
+    int at = 0;
+    for (int q = 0; q < n; ++q) at += len[q] > l || (len[q] == l && q < i);
+    cl.map_shared_rank(order, at % RC)[at / RC] = (uint16_t)i;
+  }
+  cl.sync();
+  if (tid == 0) {
+    int at = 0;
+    for (int s = 0; s < nsl; ++s) {
+      const int row = order[s * spw];
+      soff[s] = at;
+      if (row != 0xFFFF) at += 32 * ((len[row] + SUB - 1) / SUB);
+      if (at > g.ent_cap) break;
+    }
+    soff[nsl] = at;
+    sliced = at <= g.ent_cap;
+  }
+  __syncthreads();
+  if (sliced) {
+    for (int q = tid; q < 32 * nsl; q += bs) {
+      const int s = q >> 5, row = order[s * spw + (q & 31) / SUB], width = (soff[s + 1] - soff[s]) >> 5;
+      const int l = row == 0xFFFF ? 0 : len[row];
+      const int64_t e0 = row == 0xFFFF ? 0 : g.rp[row];
+      for (int e = 0; e < width; ++e) {
+        const int at = soff[s] + 32 * e + (q & 31), k = e * SUB + q % SUB;
+        scol[at] = k < l ? (uint16_t)g.col[e0 + k] : 0;
+        if (VALC) {
+          sval[2 * at] = k < l ? g.vals[2 * (e0 + k)] : 0.0;
+          sval[2 * at + 1] = k < l ? g.vals[2 * (e0 + k) + 1] : 0.0;
+        } else {
+          sval[at] = k < l ? g.vals[e0 + k] : 0.0;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // a thread's row of the first pass
+  const int row0 = is_main ? order[tid / SUB] : 0xFFFF;
+  const int len0 = row0 != 0xFFFF ? len[row0] : 0, at0 = is_main && sliced ? soff[warp] + lane : 0;
+
+  // the sum of a main warp's components (the lanes of one component carry equal values)
+  auto warp_part = [&](double v) -> double {
+#pragma unroll
+    for (int o = 16; o >= (SUB == 4 ? 2 : 1); o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  auto total = [&](const double* slots) -> double {
+    double v = 0.0;
+    for (int k = lane; k < RC * mw; k += 32) v += slots[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  // |w| and its reciprocal, from the last CTA to every CTA: the root from the reciprocal by one
+  // Newton step
+  auto roots = [&](double* out) {
+    const double w2 = total(s_norm);
+    const double ib = w2 > 0.0 ? rsqrt(w2) : 0.0, h = w2 * ib;
+    const double b = w2 < HUGE_VAL ? fma(fma(-h, h, w2), 0.5 * ib, h) : w2;
+    if (lane < CL) {
+      *cl.map_shared_rank(&s_ib, lane) = ib;
+      *cl.map_shared_rank(&s_ib2, lane) = ib * ib;
+      *cl.map_shared_rank(&s_b, lane) = b;
+    }
+    if (lane == 0) *out = b;
+  };
+
+  for (int r = blockIdx.x / CL; r < g.n_rhs; r += gridDim.x / CL) {
+    double2* Vr = g.V + (size_t)r * k_cap * n;
+    const double2* y = g.Y + (size_t)r * n;
+    double2 *cur = A, *nxt = B;
+    cl.sync();  // every CTA is done with the slots of the last right-hand side
+    for (int i = tid; i < n; i += bs) cur[i] = y[i];
+    if (is_main && row_cta) {
+      double acc = 0.0;
+      for (int ps = 0; ps < passes; ++ps) {
+        const int row = ps ? order[ps * rpp + tid / SUB] : row0;
+        if (row == 0xFFFF) continue;
+        const double v = comp ? y[row].y : y[row].x;
+        own_p[ps * M + tid] = 0.0;
+        acc = fma(v, v, acc);
+      }
+      acc = warp_part(acc);
+      if (lane == 0) cl.map_shared_rank(s_norm, CL - 1)[rank * mw + warp] = acc;
+    }
+    cl.sync();
+    if (is_sum && last_cta) roots(g.ynorm + r);
+    cl.sync();
+    if (!(s_b > 0.0)) {
+      if (rank == 0 && tid == 0) g.m_out[r] = 0;
+      continue;
+    }
+    const double iyn = s_ib;
+    for (int i = tid; i < n; i += bs) cur[i] = make_double2(cur[i].x * iyn, cur[i].y * iyn);
+    __syncthreads();
+    double2 z = make_double2(0.0, 0.0), id = make_double2(0.0, 0.0), q = make_double2(1.0, 0.0);
+    if (is_track && zi < nz) z = g.zs[(size_t)r * nz + zi];
+    double bt = 0.0;  // a tracker's beta_{j-2}
+    int m = k_cap;
+    for (int j = 0;; ++j) {
+      // ---- 1
+      if (is_main) {
+        if (row_cta && j < k_cap) {
+          double acc = 0.0;
+          for (int ps = 0; ps < passes; ++ps) {
+            const int row = ps ? order[ps * rpp + tid / SUB] : row0;
+            double yr = 0.0, yi = 0.0, x = 0.0;
+            if (row != 0xFFFF) {
+              x = reinterpret_cast<const double*>(cur)[2 * row + comp];
+              if (sliced) {
+                const int l = ps ? len[row] : len0;
+                int at = ps ? soff[ps * mw + warp] + lane : at0;
+#pragma unroll 4
+                for (int k = tid % SUB; k < l; k += SUB, at += 32) {
+                  const double2 xv = cur[scol[at]];
+                  const double hr = sval[VALC ? 2 * at : at];
+                  yr = fma(hr, xv.x, yr);
+                  yi = fma(hr, xv.y, yi);
+                  if (VALC) {
+                    const double hi = sval[2 * at + 1];
+                    yr = fma(-hi, xv.y, yr);
+                    yi = fma(hi, xv.x, yi);
+                  }
+                }
+              } else {
+                const int64_t e1 = g.rp[row + 1];
+#pragma unroll 4
+                for (int64_t e = g.rp[row] + tid % SUB; e < e1; e += SUB) {
+                  const double2 xv = cur[g.col[e]];
+                  const double hr = g.vals[VALC ? 2 * e : e];
+                  yr = fma(hr, xv.x, yr);
+                  yi = fma(hr, xv.y, yi);
+                  if (VALC) {
+                    const double hi = g.vals[2 * e + 1];
+                    yr = fma(-hi, xv.y, yr);
+                    yi = fma(hi, xv.x, yi);
+                  }
+                }
+              }
+            }
+            double v = (comp ? yi : yr) + __shfl_xor_sync(0xffffffffu, comp ? yr : yi, SUB >> 1);
+            if (SUB == 4) v += __shfl_xor_sync(0xffffffffu, v, 1);
+            own_y[ps * M + tid] = v;
+            acc = fma(v, x, acc);
+          }
+          acc = warp_part(acc);
+          if (lane < CL) cl.map_shared_rank(s_alpha, lane)[rank * mw + warp] = acc;
+        }
+      } else if (is_sum) {
+        if (last_cta && j > 0) roots(g.beta + (size_t)r * k_cap + j - 1);
+      } else if (is_track && j > 0 && zi < nz) {
+        // the shift's pivot and residual estimate for step j - 1, but for the factor beta_{j-1}
+        double2 d = make_double2(z.x - s_a, z.y), qn = make_double2(1.0, 0.0);
+        if (j > 1) {
+          const double b2 = bt * bt;
+          d.x -= b2 * id.x;
+          d.y -= b2 * id.y;
+          qn = make_double2(q.x * bt, q.y * bt);
+        }
+        const double rd = 1.0 / (d.x * d.x + d.y * d.y);
+        id = make_double2(d.x * rd, -d.y * rd);
+        q = make_double2(qn.x * id.x - qn.y * id.y, qn.x * id.y + qn.y * id.x);
+      }
+      cl.sync();
+      const double b = s_b, ib = j > 0 ? s_ib : 1.0;  // beta_{j-1} and its reciprocal
+      if (!(b > 0.0)) {  // the space is exhausted, or a NaN
+        m = j;
+        if (rank == 0 && tid == 0 && !(b >= 0.0)) atomicExch(g.status, (int32_t)EDGPU_ERR_NAN);
+        break;
+      }
+      // ---- 2
+      if (is_main) {
+        if (row_cta && j < k_cap) {
+          const double nb = j > 0 ? -b : 0.0;
+          double* vj = reinterpret_cast<double*>(Vr + (size_t)j * n);
+          for (int ps = 0; ps < passes; ++ps) {
+            const int row = ps ? order[ps * rpp + tid / SUB] : row0, at = ps * M + tid;
+            if (row == 0xFFFF) continue;
+            const double v = reinterpret_cast<const double*>(cur)[2 * row + comp] * ib;
+            own_y[at] = fma(nb, own_p[at], own_y[at] * ib);
+            own_p[at] = v;
+            if (d0 == 0) vj[2 * row + comp] = v;
+          }
+          cluster_bar(M + 32);
+          const double na = -s_a;
+          double acc = 0.0;
+          for (int ps = 0; ps < passes; ++ps) {
+            const int row = ps ? order[ps * rpp + tid / SUB] : row0, at = ps * M + tid;
+            if (row == 0xFFFF) continue;
+            const double w = fma(na, own_p[at], own_y[at]);
+            acc = fma(w, w, acc);
+            for (int d = d0; d < RC; d += dstep)
+              reinterpret_cast<double*>(cl.map_shared_rank(nxt, d))[2 * row + comp] = w;
+          }
+          acc = warp_part(acc);
+          if (lane == 0) cl.map_shared_rank(s_norm, CL - 1)[rank * mw + warp] = acc;
+        }
+      } else if (is_sum) {
+        if (j < k_cap) {
+          double a = total(s_alpha);
+          if (j > 0) a *= s_ib2;
+          if (lane == 0) {
+            s_a = a;
+            if (rank == 0) g.alpha[(size_t)r * k_cap + j] = a;
+          }
+          if (row_cta) cluster_bar(M + 32);
+        }
+      } else if (is_track && j > 0) {
+        bt = b;
+        const bool ok = __all_sync(0xffffffffu, zi >= nz || b * sqrt(q.x * q.x + q.y * q.y) <= g.tol);
+        if (lane < CL) cl.map_shared_rank(s_ok, lane)[trank * tw + (tz >> 5)] = ok;
+      }
+      cl.sync();
+      if (j > 0) {
+        bool ok = true;
+        for (int k = lane; k < tcs * tw; k += 32) ok = ok && s_ok[k];
+        const bool conv = __all_sync(0xffffffffu, ok);
+        if (conv || j == k_cap) {  // step j - 1 was the last
+          m = j;
+          if (rank == 0 && tid == 0 && !conv) atomicExch(g.status, (int32_t)EDGPU_ERR_NOCONV);
+          break;
+        }
+      }
+      double2* t = cur;
+      cur = nxt;
+      nxt = t;
+    }
+    if (rank == 0 && tid == 0) g.m_out[r] = m;
+  }
+  cl.sync();
+}
+
 // The same shifted solves in double-float arithmetic for a real H (values as hi/lo float
 // pairs), two vectors per right-hand side as in lanczos_small_df_kernel, each v_j written
 // to V[rhs][j] as float4 (re.hi, re.lo, im.hi, im.lo).  The residual estimate only decides
@@ -2568,6 +2880,58 @@ extern "C" size_t edgpu_shifted_solve_workspace(int64_t n, int n_rhs, int nz, in
 
 namespace {
 
+// Launches the clusters where one of the sizes holds every right-hand side at once: the size, 0 where
+// none does (the caller's one-CTA form, which keeps every SM busy then), -1 on an error.  A warp's worth of
+// rows has nothing to share: 1 row takes 130 us on one CTA and 145 on a cluster, 33 rows 342 and 327.
+int launch_shifted_cluster(edgpu::ShiftedArgs g, bool cplx, int64_t nnz, cudaStream_t s) {
+  using namespace edgpu;
+  if (g.n <= 32) return 0;
+  const size_t per_entry = (cplx ? 16 : 8) + 2;
+  for (int cl = kClusterMax; cl > 1; cl >>= 1) {
+    if ((int64_t)g.n_rhs * cl > grid_cap()) continue;
+    ClusterArgs c{};
+    c.a = g;
+    c.rows_on = cl > 2 && g.nz <= kOwnTrackers ? cl - 1 : cl;
+    const int rows = (int)((g.n + c.rows_on - 1) / c.rows_on);
+    const int sub = 4 * rows <= kSmallThreads ? 4 : 2;
+    auto kern = sub == 4 ? (cplx ? shifted_cluster_kernel<true, 4> : shifted_cluster_kernel<false, 4>)
+                         : (cplx ? shifted_cluster_kernel<true, 2> : shifted_cluster_kernel<false, 2>);
+    c.a.main_threads = std::min(kSmallThreads, (sub * rows + 31) / 32 * 32);
+    c.passes = (sub * rows + c.a.main_threads - 1) / c.a.main_threads;
+    const int threads = c.a.main_threads + 32 + ((c.rows_on < cl ? g.nz : (g.nz + cl - 1) / cl) + 31) / 32 * 32;
+    const size_t fixed = 2 * sizeof(double2) * (size_t)g.n + 2 * sizeof(double) * (size_t)c.passes * c.a.main_threads +
+                         sizeof(uint16_t) * (size_t)(g.n + (int64_t)c.passes * c.a.main_threads / sub) + 16;
+    if (fixed > 200 * 1024) continue;
+    // a warp's rows have nearly equal lengths: room for half as many lanes without an entry again
+    const int64_t want = (nnz / c.rows_on + 1) * 3 / 2 + (int64_t)sub * rows + 32;
+    c.a.ent_cap = fixed + per_entry * (size_t)want <= 216 * 1024 ? (int)((want + 3) & ~(int64_t)3) : 0;
+    const size_t bytes = fixed + per_entry * (size_t)c.a.ent_cap;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = cl;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(cl * g.n_rhs));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    if (fit < g.n_rhs) continue;
+    return cudaLaunchKernelEx(&cfg, kern, c) == cudaSuccess ? cl : -1;
+  }
+  return 0;
+}
+
 int shifted_solve_impl(const edgpu_csr* h, const double* Y, int n_rhs, const double* zs, int nz, int k_cap, double tol,
                        double* X, int32_t* m_out, int32_t* status_dev, void* workspace, size_t workspace_bytes,
                        cudaStream_t s, bool df) {
@@ -2630,19 +2994,23 @@ int shifted_solve_impl(const edgpu_csr* h, const double* Y, int n_rhs, const dou
     g.m_out = m_out;
     g.ynorm = yn;
     g.status = status_dev;
-    g.main_threads = std::min(kSmallThreads, npad);
-    const int threads = g.main_threads + (nz + 31) / 32 * 32;
-    // shared memory: vectors, sums, slots; the sliced entries when a third more than nnz of them fit
-    const size_t fixed = 3 * sizeof(double2) * (size_t)n + 34 * sizeof(double) + 2 * sizeof(uint16_t) * (size_t)npad + 16;
     const size_t per_entry = (h->val_c ? 16 : 8) + 2;
-    const int64_t want = h->nnz + h->nnz / 3 + 32;
-    g.ent_cap = fixed + per_entry * (size_t)want <= 220 * 1024 ? (int)((want + 3) & ~(int64_t)3) : 0;
-    const size_t bytes = fixed + per_entry * (size_t)g.ent_cap;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes);
-    if (per_sm < 1) per_sm = 1;
-    const int grid = std::min(grid_cap() * per_sm, n_rhs);
-    kern<<<grid, threads, bytes, s>>>(g);
+    const int cl = launch_shifted_cluster(g, h->val_c != nullptr, h->nnz, s);
+    if (cl < 0) return EDGPU_ERR_CUDA;
+    if (cl == 0) {
+      g.main_threads = std::min(kSmallThreads, npad);
+      const int threads = g.main_threads + (nz + 31) / 32 * 32;
+      // shared memory: vectors, sums, slots; the sliced entries when a third more than nnz of them fit
+      const size_t fixed = 3 * sizeof(double2) * (size_t)n + 34 * sizeof(double) + 2 * sizeof(uint16_t) * (size_t)npad + 16;
+      const int64_t want = h->nnz + h->nnz / 3 + 32;
+      g.ent_cap = fixed + per_entry * (size_t)want <= 220 * 1024 ? (int)((want + 3) & ~(int64_t)3) : 0;
+      const size_t bytes = fixed + per_entry * (size_t)g.ent_cap;
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes);
+      if (per_sm < 1) per_sm = 1;
+      const int grid = std::min(grid_cap() * per_sm, n_rhs);
+      kern<<<grid, threads, bytes, s>>>(g);
+    }
   }
   note_launch();
   int rc = check_launch();

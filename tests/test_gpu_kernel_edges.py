@@ -281,6 +281,28 @@ def test_shifted_solves(eng, n, nz, cplx, precision):
             assert np.linalg.norm(X[r, q] - x) <= 4e-10 * np.linalg.norm(Y[r])
 
 
+@pytest.mark.parametrize("n,R,nz,cplx", [
+    (65, 30, 65, True),    # clusters of 4, as many shifts as their CTAs share
+    (300, 70, 7, False),   # clusters of 2
+    (1300, 60, 2, False),  # clusters of 2, several rows a thread
+    (90, 160, 3, False),   # a CTA a right-hand side
+])
+def test_shifted_solves_on_clusters(eng, n, R, nz, cplx):
+    csr, _ = _random_csr(eng, n, n + R, cplx, heavy=(0, n // 3))
+    g = np.random.default_rng(R)
+    Y = g.normal(size=(R, n)) + 1j * g.normal(size=(R, n))
+    Y[R // 2] = 0.0
+    zs = g.uniform(-8.0, 8.0, size=(R, nz)) + 0.5j
+    X, m = eng.shifted_solve(csr, torch.from_numpy(Y).to(eng.device), zs, 1e-10, min(6 * n + 50, 2000), 0)
+    some = [0, 1, R // 2, R - 1]
+    X1, m1 = eng.shifted_solve(csr, torch.from_numpy(Y[some]).to(eng.device), zs[some], 1e-10, min(6 * n + 50, 2000), 0)
+    X, X1 = X.cpu().numpy()[some], X1.cpu().numpy()
+    assert int(m[R // 2]) == 0 and not X[2].any() and not X1[2].any()
+    for q in (0, 1, 3):
+        # either residual is below 1e-10 |y|, and |(z - H)^{-1}| <= 1 / Im z; as much again for the rounding
+        assert np.linalg.norm(X[q] - X1[q], axis=-1).max() <= 8e-10 * np.linalg.norm(Y[some[q]])
+
+
 @pytest.mark.parametrize("batch,words", [(128, 5), (384, 2), (4096, 5)])
 def test_training_step(eng, batch, words):
     """One fused step against the layer-by-layer calls."""

@@ -927,6 +927,310 @@ struct KernelTimer {
   }
 };
 
+// The same recurrence in FP64 as one cooperative launch, for sectors whose rows fit in the SMs' shared
+// memory.  A block of 1024 threads per SM takes the rows b, b + B, ... (the long ones are neighbours in
+// the basis), sorts them by length and keeps their entries, y, w and v_{j-1} in shared memory for all
+// steps; only the unscaled w = beta_{j-1} v_j goes through L2, for the other blocks' gathers.  Two or four
+// threads per row and run; a warp's rows have nearly equal lengths.  Two grid barriers a step (after the partials of alpha_j and of beta_j^2), the sums of
+// the blocks' partials by a warp per run in one fixed order.
+// Bound by FP64 issue in the products (16 cycles a warp instruction: 9.4 us a step for 3 runs of 47 895
+// rows) and the latency of the barriers and sums.
+// 47 895 rows, 0.93 M entries, 100 steps: 3 runs 4.0 -> 2.56 ms (two launches a step pay their gaps, read
+// H and the vectors again and wait for the long rows); 40 steps of 1 run 1.21 -> 0.81, of 8 2.35 -> 1.82.
+constexpr int kGridThreads = 1024;
+constexpr int kGridRuns = kGridThreads / 32;
+constexpr int kGridRows = 2048;  // rows of a block at most (their ranks take rows^2 / 1024 steps)
+
+struct GridArgs {
+  int64_t n;
+  const int64_t* rp;
+  const int32_t* col;
+  const double* vals;
+  const double2* v0;
+  int R, K;
+  int sub;      // threads per row and run
+  int ent_cap;  // entries a block has room for
+  double2 *A, *B;
+  double *pa, *pb;
+  const int32_t* k_max;
+  double *alpha, *beta;
+  int32_t* status;
+};
+
+// Shared memory of a block without the entries.
+inline size_t grid_fixed_bytes(int64_t rows, int R) {
+  return 3 * sizeof(double2) * (size_t)rows * R + sizeof(double) * kGridThreads +
+         (sizeof(int) + 2 * sizeof(uint16_t)) * (size_t)rows + 16;
+}
+
+template <bool VALC>
+__global__ void __launch_bounds__(kGridThreads, 1) lanczos_grid_kernel(GridArgs g) {
+  cg::grid_group grid = cg::this_grid();
+  const int B = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R = g.R, K = g.K;
+  const int mine = (int)((g.n - b + B - 1) / B), items = mine * R;
+  const int most = (int)((g.n + B - 1) / B);
+  extern __shared__ __align__(16) unsigned char sm[];
+  double2* y = reinterpret_cast<double2*>(sm);  // [slot][run], as w and p
+  double2* w = y + (size_t)most * R;
+  double2* p = w + (size_t)most * R;
+  double* red = reinterpret_cast<double*>(p + (size_t)most * R);
+  double* eval = red + kGridThreads;
+  int* ecol = reinterpret_cast<int*>(eval + (size_t)g.ent_cap * (VALC ? 2 : 1));
+  int* eoff = ecol + g.ent_cap;                               // [mine] a slot's first entry
+  uint16_t* len = reinterpret_cast<uint16_t*>(eoff + most);   // [mine]
+  uint16_t* order = len + most;                               // [mine] slot's row b + B * order
+  __shared__ double s_ib[kGridRuns], s_cy[kGridRuns], s_cw[kGridRuns], s_cp[kGridRuns], s_b[kGridRuns];
+  __shared__ int s_fits;
+
+  for (int k = tid; k < mine; k += kGridThreads) {
+    const int64_t i = b + (int64_t)B * k, l = g.rp[i + 1] - g.rp[i];
+    len[k] = (uint16_t)(l < 0xFFFF ? l : 0xFFFF);
+  }
+  __syncthreads();
+  for (int k = tid; k < mine; k += kGridThreads) {
+    const int l = len[k];
+    int at = 0;
+    for (int q = 0; q < mine; ++q) at += len[q] > l || (len[q] == l && q < k);
+    order[at] = (uint16_t)k;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int at = 0;
+    bool fits = true;
+    for (int q0 = 0; q0 < mine; q0 += 32) {
+      const int l = q0 + lane < mine ? len[order[q0 + lane]] : 0;
+      int end = l;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += o;
+      }
+      if (q0 + lane < mine) eoff[q0 + lane] = at + end - l;
+      at += __shfl_sync(0xffffffffu, end, 31);
+      fits = fits && at <= g.ent_cap;
+      if (!fits) break;
+    }
+    if (lane == 0) s_fits = fits;
+  }
+  __syncthreads();
+  const bool fits = s_fits;
+  if (!fits) {
+    for (int s = tid; s < mine; s += kGridThreads) eoff[s] = 0;
+  } else {
+    for (int s = warp; s < mine; s += kGridThreads / 32) {
+      const int64_t e0 = g.rp[b + (int64_t)B * order[s]];
+      const int l = len[order[s]], at = eoff[s];
+      for (int e = lane; e < l; e += 32) {
+        ecol[at + e] = g.col[e0 + e];
+        if (VALC) {
+          eval[2 * (at + e)] = g.vals[2 * (e0 + e)];
+          eval[2 * (at + e) + 1] = g.vals[2 * (e0 + e) + 1];
+        } else {
+          eval[at + e] = g.vals[e0 + e];
+        }
+      }
+    }
+  }
+  // dense loops: a run per thread whatever the pass
+  const int dense = kGridThreads / R * R, dr = tid % R;
+  if (tid < dense)
+    for (int q = tid; q < items; q += dense) {
+      w[q] = g.v0[(b + (int64_t)B * order[q / R]) * R + dr];
+      p[q] = make_double2(0.0, 0.0);
+    }
+  if (tid < R) {
+    s_ib[tid] = 1.0;
+    s_b[tid] = 0.0;
+  }
+  __syncthreads();
+
+  // products: g.sub threads per row and run
+  const int sub = g.sub, per = kGridThreads / (R * sub) * R, gi = tid / sub, gs = tid % sub;
+  const int slot0 = gi / R, gr = gi % R, slots = per / R;
+
+  // sums of a run: the last warps, whose rows are the shortest
+  const int run = kGridThreads / 32 - 1 - warp;
+  // this block's partial of a dense sum, a warp per run
+  auto partial = [&](double v, double* out) {
+    red[tid] = v;
+    __syncthreads();
+    if (run < R) {
+      const int lim = items < dense ? items : dense;
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k = run + R * lane; k < lim; k += 128 * R) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (k + 32 * R * u < lim) s[u] += red[k + 32 * R * u];
+      }
+      double t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) out[(int64_t)b * R + run] = t;
+    }
+    grid.sync();
+  };
+  // the sum of all blocks' partials of `run`
+  auto total = [&](const double* part) -> double {
+    double s = 0.0;
+    for (int q = lane; q < B; q += 32) s += part[(int64_t)q * R + run];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  };
+
+  const double2* cur = g.v0;
+  for (int j = 0; j < K; ++j) {
+    // ---- y = H w, alpha_j
+    if (gi < per) {
+      const double2* x = cur + gr;
+      for (int slot = slot0; slot < mine; slot += slots) {
+        const int k0 = order[slot];
+        int l = len[k0];
+        const int* ec = ecol + eoff[slot];
+        const double* ev = eval + (VALC ? 2 : 1) * eoff[slot];
+        if (!fits) {
+          const int64_t i = b + (int64_t)B * k0, e0 = g.rp[i];
+          l = (int)(g.rp[i + 1] - e0);
+          ec = g.col + e0;
+          ev = g.vals + (VALC ? 2 : 1) * e0;
+        }
+        double yr = 0.0, yi = 0.0;
+        for (int e = gs; e < l; e += 4 * sub) {
+          double2 xv[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (e + u * sub < l) xv[u] = x[(int64_t)ec[e + u * sub] * R];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int k = e + u * sub;
+            if (k < l) {
+              const double hr = ev[VALC ? 2 * k : k];
+              yr = fma(hr, xv[u].x, yr);
+              yi = fma(hr, xv[u].y, yi);
+              if (VALC) {
+                const double hi = ev[2 * k + 1];
+                yr = fma(-hi, xv[u].y, yr);
+                yi = fma(hi, xv[u].x, yi);
+              }
+            }
+          }
+        }
+        // the threads of a row and run: neighbours in a warp
+        const unsigned group = ((1u << sub) - 1u) << (lane & ~(sub - 1));
+        for (int o = sub >> 1; o > 0; o >>= 1) {
+          yr += __shfl_xor_sync(group, yr, o);
+          yi += __shfl_xor_sync(group, yi, o);
+        }
+        if (gs == 0) y[slot * R + gr] = make_double2(yr, yi);
+      }
+    }
+    __syncthreads();
+    double acc = 0.0;
+    if (tid < dense)
+      for (int q = tid; q < items; q += dense) acc = fma(y[q].y, w[q].y, fma(y[q].x, w[q].x, acc));
+    partial(acc, g.pa);
+    if (run < R) {
+      const double ib = s_ib[run], a = total(g.pa) * ib * ib;
+      if (lane == 0) {
+        if (b == 0) g.alpha[(int64_t)run * K + j] = a;
+        s_cy[run] = ib;
+        s_cw[run] = -a * ib;
+        s_cp[run] = -s_b[run];
+      }
+    }
+    if (j + 1 >= K) break;  // identical in every block
+    __syncthreads();
+    // ---- w' = y / beta_{j-1} - alpha_j v_j - beta_{j-1} v_{j-1}, beta_j
+    double2* nxt = j & 1 ? g.B : g.A;
+    acc = 0.0;
+    if (tid < dense) {
+      const double cy = s_cy[dr], cw = s_cw[dr], cp = s_cp[dr];
+      for (int q = tid, s = tid / R; q < items; q += dense, s += dense / R) {
+        const double2 v = w[q], h = y[q], o = p[q];
+        double2 x;
+        x.x = fma(cp, o.x, fma(cw, v.x, cy * h.x));
+        x.y = fma(cp, o.y, fma(cw, v.y, cy * h.y));
+        p[q] = make_double2(v.x * cy, v.y * cy);
+        w[q] = x;
+        nxt[(b + (int64_t)B * order[s]) * R + dr] = x;
+        acc = fma(x.y, x.y, fma(x.x, x.x, acc));
+      }
+    }
+    partial(acc, g.pb);
+    if (run < R) {
+      const double t = total(g.pb);
+      if (lane == 0) {
+        const double bt = sqrt(t);
+        s_b[run] = bt;
+        s_ib[run] = bt > 0.0 ? 1.0 / bt : 0.0;  // a run whose beta is 0 has ended: its vector stays 0
+        if (b == 0) {
+          g.beta[(int64_t)run * K + j] = bt;
+          if (g.k_max[run] > j + 1 && !(bt > 0.0))
+            atomicExch(g.status, (int32_t)(bt == 0.0 ? EDGPU_ERR_BREAKDOWN : EDGPU_ERR_NAN));
+        }
+      }
+    }
+    cur = nxt;
+  }
+}
+
+// Launches the cooperative form where the sector's vectors and entries fit in shared memory (without the
+// entries 40 steps of 300 000 rows take 3.4 ms against 2.4 in two launches a step): 1 when it ran, 0 when the caller's two
+// launches a step take the call, -1 on an error.
+static int launch_grid(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, double* alpha,
+                       double* beta, int32_t* status, unsigned char* ws, cudaStream_t s) {
+  if (R > kGridRuns || (!h->val_c && !h->val_r)) return 0;
+  const int blocks = grid_cap();
+  const int64_t most = (h->n + blocks - 1) / blocks;
+  const bool cplx = h->val_c != nullptr;
+  const size_t limit = 220 * 1024, per_entry = (cplx ? 16 : 8) + sizeof(int);
+  if (h->n < blocks || most > kGridRows || grid_fixed_bytes(most, R) > limit) return 0;
+  GridArgs g{};
+  const size_t room = (limit - grid_fixed_bytes(most, R)) / per_entry;
+  if (room < (size_t)(h->nnz / blocks + h->nnz / blocks / 8 + 64)) return 0;
+  g.ent_cap = (int)std::min<size_t>(room, (size_t)(2 * (h->nnz / blocks) + 256)) & ~1;
+  const size_t bytes = grid_fixed_bytes(most, R) + per_entry * (size_t)g.ent_cap;
+  auto kern = cplx ? lanczos_grid_kernel<true> : lanczos_grid_kernel<false>;
+  int dev = 0, coop = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGridThreads, bytes) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  // the same places in the workspace as the two launches a step: two vectors, the partials behind the third
+  const size_t vec = (sizeof(double2) * (size_t)h->n * R + 255) & ~(size_t)255;
+  const size_t part = (sizeof(double) * (size_t)blocks * R + 255) & ~(size_t)255;
+  if (2 * part > vec) return 0;  // pa and pb share the third vector's place
+  g.n = h->n;
+  g.rp = h->row_ptr;
+  g.col = h->col;
+  g.vals = cplx ? h->val_c : h->val_r;
+  g.v0 = reinterpret_cast<const double2*>(v0);
+  g.R = R;
+  g.K = K;
+  // The few long rows of a sector (65 entries of 19 on average) set the products' length: 40 steps of the
+  // 316-spin-orbital sector take 1143, 864, 808 us with 1, 2, 4 threads a row for one run, 1349, 1114,
+  // 1286 for 3 runs and 1930, 1822, 2542 for 8.
+  g.sub = most * R <= 320 ? 4 : 2;
+  g.A = reinterpret_cast<double2*>(ws);
+  g.B = reinterpret_cast<double2*>(ws + vec);
+  g.pa = reinterpret_cast<double*>(ws + 2 * vec);
+  g.pb = reinterpret_cast<double*>(ws + 2 * vec + part);
+  g.k_max = k_max;
+  g.alpha = alpha;
+  g.beta = beta;
+  g.status = status;
+  void* args[] = {&g};
+  if (cudaLaunchCooperativeKernel((const void*)kern, blocks, kGridThreads, args, bytes, s) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  note_launch();
+  return 1;
+}
+
 template <typename T>
 int lanczos_impl(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, double* alpha, double* beta,
                  int32_t* status, unsigned char* ws, size_t ws_bytes, cudaStream_t s, double* kernel_ms = nullptr) {
@@ -1049,9 +1353,12 @@ extern "C" int edgpu_lanczos(const edgpu_csr* h, const double* v0, int R, const 
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
   if (small_fits(h->n, precision))
     return lanczos_small(h, v0, R, k_max, K, precision, alpha, beta, status_dev, ws, (cudaStream_t)stream);
-  if (precision == 0)
+  if (precision == 0) {
+    const int ran = launch_grid(h, v0, R, k_max, K, alpha, beta, status_dev, ws, (cudaStream_t)stream);
+    if (ran != 0) return ran > 0 ? check_launch() : EDGPU_ERR_CUDA;
     return lanczos_impl<double>(h, v0, R, k_max, K, alpha, beta, status_dev, ws, workspace_bytes,
                                 (cudaStream_t)stream);
+  }
   return lanczos_impl<float>(h, v0, R, k_max, K, alpha, beta, status_dev, ws, workspace_bytes, (cudaStream_t)stream);
 }
 

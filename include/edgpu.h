@@ -327,7 +327,8 @@ int edgpu_spmv_paged_tma_c64(const edgpu_csr* h, const void* pages, int64_t n_pa
  * anywhere else runs as 0.  Breakdown (beta == 0 before k_max) sets
  * *status_dev = EDGPU_ERR_BREAKDOWN.  Sectors whose three Krylov vectors fit in shared
  * memory run as one persistent launch with one CTA per run; larger ones as two
- * grid-wide kernels per step.  In the FP64 form with real H, from eight steps a wave of CTAs on,
+ * grid-wide kernels per step, or in FP64 as one cooperative launch for all steps where the rows and
+ * entries of H fit in the SMs' shared memory.  In the FP64 form with real H, from eight steps a wave of CTAs on,
  * one extra launch builds a sliced copy of H in the workspace where it fits (rows that repeat a
  * column are read from the CSR arrays as before).  In the double-float form the CTA keeps one vector in shared
  * memory and the previous one in the workspace, and, when the workspace size returned for

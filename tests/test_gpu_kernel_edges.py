@@ -436,3 +436,48 @@ def test_runs_on_sliced_rows(eng, n, extra, K):
     m = min(K, 12)
     # a dozen steps of an unconverged recurrence amplify rounding by less than 1e3
     assert np.abs(a[0, :m].cpu().numpy() - ar[:m]).max() < 1e-12 * max(abs(H).sum(1).max(), 1.0)
+
+
+@pytest.mark.parametrize("n,R,K,cplx,extra", [
+    (4267, 1, 12, False, 0),      # four threads a row, most of the block idle
+    (4300, 32, 12, False, 0),     # as many runs as a block sums
+    (30000, 2, 12, True, 0),      # two threads a row
+    (47895, 8, 12, False, 0),     # several rows a thread
+    (47895, 3, 12, False, 3000),  # a block's entries beyond its shared memory, repeated columns
+    (20000, 5, 1, False, 0),      # a single step: alpha only
+])
+def test_grid_wide_lanczos_in_one_launch(eng, n, R, K, cplx, extra):
+    """The cooperative form against the two launches a step (which the timed entry point keeps)."""
+    from impuritymodel_gb300.engine import CsrMatrix
+
+    rng = np.random.default_rng(n + R)
+    rows, cols = [np.arange(0, n, 2)], [np.arange(0, n, 2)]  # odd diagonals are 0, some rows empty
+    for _ in range(2):
+        i, j = rng.integers(0, n, size=(2, n // 2))
+        rows += [i, j]
+        cols += [j, i]
+    for i in (0, n // 3):
+        j = rng.integers(0, n // 8, size=extra) * 8 % n
+        rows += [np.full(extra, i), j]
+        cols += [j, np.full(extra, i)]
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    o = np.argsort(rows, kind="stable")
+    rows, cols = rows[o], cols[o]
+    lo, hi = np.minimum(rows, cols), np.maximum(rows, cols)
+    vals = np.cos(1.0 + 7.0 * lo + 3.0 * hi) / (1.0 + extra ** 0.5) + 4.0 * (rows == cols)
+    rp = torch.from_numpy(np.searchsorted(rows, np.arange(n + 1)).astype(np.int64)).to(eng.device)
+    col = torch.from_numpy(cols.astype(np.int32)).to(eng.device)
+    if cplx:
+        im = np.sign(cols - rows) * np.sin(5.0 * lo + hi)
+        csr = CsrMatrix(rp, col, val_c=torch.from_numpy(np.stack([vals, im], 1)).to(eng.device).contiguous())
+    else:
+        csr = CsrMatrix(rp, col, val_r=torch.from_numpy(vals).to(eng.device))
+    v = rng.normal(size=(n, R)) + 1j * rng.normal(size=(n, R))
+    v = torch.from_numpy(v / np.linalg.norm(v, axis=0)).to(eng.device)
+    k = np.full(R, K, dtype=np.int32)
+    a, b = eng.lanczos(csr, v, k, precision=0)
+    a1, b1 = eng.lanczos(csr, v, k, precision=0, timing=[])
+    norm = np.bincount(rows, weights=np.abs(vals) + (np.abs(im) if cplx else 0.0)).max()
+    # a dozen steps of an unconverged recurrence amplify rounding by less than 1e3
+    assert (a - a1).abs().max().item() < 1e-12 * norm
+    assert K == 1 or (b - b1)[:, :K - 1].abs().max().item() < 1e-12 * norm

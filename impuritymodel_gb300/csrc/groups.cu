@@ -14,7 +14,7 @@
 // Against the two-pass form (a count and a fill launch that each did all of the work; per state an
 // emission buffer with an O(m^2) ordered merge, ~19 dependent reads for every basis lookup, a
 // double-precision hypot per output) the application launches of the 316-orbital photoemission
-// sector's construction (462 120 states, 2542 terms) take 3.7 ms instead of 71.  What the one pass is
+// sector's construction (462 120 states, 2542 terms) take 3.9 ms instead of 71.  What the one pass is
 // made of there: some 80 candidate groups a state tested against occupations and restrictions (61
 // of them hops out of a full bath that the restrictions drop; the counts of all restrictions change by
 // bit-sliced sums), ~8 that survive, finished 32 at a time.

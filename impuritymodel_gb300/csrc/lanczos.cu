@@ -108,6 +108,8 @@ __global__ void spmm_alpha_kernel(int64_t n, const int64_t* __restrict__ rp, con
 
 // ---------------------------------------------------------------------------------------
 // Grid-wide batched Lanczos (lanczos_impl): two launches per step on vectors kept unnormalised.
+// Serves complex64 vectors, more runs or larger sectors than lanczos_grid_kernel below, the timed and the
+// allocation-free entry points.
 //
 // w_j is stored as it leaves the three-term update and v_j = w_j / beta_{j-1} is never formed:
 // the first launch takes y = H w_j and the partial sums of <y, w_j>, the second
@@ -931,8 +933,9 @@ struct KernelTimer {
 // memory.  A block of 1024 threads per SM takes the rows b, b + B, ... (the long ones are neighbours in
 // the basis), sorts them by length and keeps their entries, y, w and v_{j-1} in shared memory for all
 // steps; only the unscaled w = beta_{j-1} v_j goes through L2, for the other blocks' gathers.  Two or four
-// threads per row and run; a warp's rows have nearly equal lengths.  Two grid barriers a step (after the partials of alpha_j and of beta_j^2), the sums of
-// the blocks' partials by a warp per run in one fixed order.
+// threads per row and run; a warp's rows have nearly equal lengths.  Two grid barriers a step (after the
+// partials of alpha_j and of beta_j^2), the sums of the blocks' partials by a warp per run in one
+// fixed order.
 // Bound by FP64 issue in the products (16 cycles a warp instruction: 9.4 us a step for 3 runs of 47 895
 // rows) and the latency of the barriers and sums.
 // 47 895 rows, 0.93 M entries, 100 steps: 3 runs 4.0 -> 2.56 ms (two launches a step pay their gaps, read

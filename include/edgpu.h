@@ -343,8 +343,9 @@ int edgpu_lanczos(const edgpu_csr* h, const double* v0, int R, const int32_t* k_
 
 /*
  * edgpu_lanczos with CUDA-event timing of its kernels on the launching stream:
- * kernel_ms (host, 3 doubles) receives the summed milliseconds of the SpMM + alpha,
- * axpy + beta and normalise launches.  Synchronises on the last event before returning.
+ * kernel_ms (host, 3 doubles) receives the summed milliseconds of the products, of the
+ * vector updates and 0 (sectors that do not fit in one SM: always the two launches per step), or the
+ * whole of a small sector's launch and two zeros.  Synchronises on the last event before returning.
  */
 int edgpu_lanczos_timed(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, int precision,
                         double* alpha, double* beta, int32_t* status_dev, void* workspace, size_t workspace_bytes,

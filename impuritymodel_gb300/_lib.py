@@ -102,6 +102,8 @@ SIGNATURES = {
     "edgpu_vary_mask": (_I, [_I, _P, _I64, _P, _P]),
     "edgpu_scan_workspace": (_SZ, [_I64]),
     "edgpu_scan_i64": (_I, [_P, _P, _I64, _P, _SZ, _P]),
+    "edgpu_sort_unique_fits": (_I, [_I, _I64]),
+    "edgpu_sort_unique": (_I, [_I, _P, _I64, _P, _P, _P]),
     "edgpu_segment_heads": (_I, [_I, _P, _I64, _P, _P]),
     "edgpu_segment_reduce": (_I, [_I, _P, _P, _I64, _P, _P, _P, _P, _P, _P]),
     "edgpu_merge_states": (_I, [_I, _P, _I64, _P, _I64, _P, _P]),

@@ -453,6 +453,13 @@ class Engine:
 
     def sort_unique(self, keys):
         """Sorted unique rows of ``keys`` (copy)."""
+        m, w = keys.shape
+        if m > 1 and self.lib.edgpu_sort_unique_fits(w, m):
+            out = torch.empty((m, w), dtype=torch.int64, device=self.device)
+            count = torch.empty(1, dtype=torch.int64, device=self.device)
+            src = keys.contiguous()
+            L.check(self.lib.edgpu_sort_unique(w, _ptr(src), m, _ptr(out), _ptr(count), self.stream), "sort_unique")
+            return out[: int(count.item())]
         k = keys.clone()
         p = torch.arange(k.shape[0], dtype=torch.int32, device=self.device)
         self.sort_states(k, p)

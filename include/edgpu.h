@@ -189,6 +189,12 @@ size_t edgpu_sort_states_packed_workspace(int n_words, int64_t n);
 int edgpu_sort_states_packed(int n_words, uint64_t* keys, uint32_t* payload, int64_t n, const uint64_t* stats,
                              void* workspace, size_t workspace_bytes, void* stream);
 
+/* Sorted unique rows of keys (left as they are) into out (room for n rows), their number into count
+ * (device), in one launch; for the sizes that edgpu_sort_unique_fits accepts (those one CTA sorts).
+ */
+int edgpu_sort_unique_fits(int n_words, int64_t n);
+int edgpu_sort_unique(int n_words, const uint64_t* keys, int64_t n, uint64_t* out, int64_t* count, void* stream);
+
 /* OR over rows of (row XOR row 0) into vary_out[n_words] (device). */
 int edgpu_vary_mask(int n_words, const uint64_t* keys, int64_t n, uint64_t* vary_out, void* stream);
 

@@ -481,3 +481,27 @@ def test_grid_wide_lanczos_in_one_launch(eng, n, R, K, cplx, extra):
     # a dozen steps of an unconverged recurrence amplify rounding by less than 1e3
     assert (a - a1).abs().max().item() < 1e-12 * norm
     assert K == 1 or (b - b1)[:, :K - 1].abs().max().item() < 1e-12 * norm
+
+
+@pytest.mark.parametrize("n,words,kinds", [
+    (2, 1, 1),       # one key twice
+    (33, 2, 20),     # a ragged second warp
+    (1025, 5, 700),  # a network of 2048 keys, several blocks of heads
+    (2048, 8, 2048),  # the longest keys
+    (8192, 2, 5000),  # the largest that one CTA sorts
+])
+def test_sorted_unique_in_one_launch(eng, n, words, kinds):
+    """Against the separate sort and compaction."""
+    g = torch.Generator(device=eng.device)
+    g.manual_seed(n)
+    pool = torch.randint(-(1 << 62), 1 << 62, (kinds, words), device=eng.device, generator=g) * 2
+    pool[0] = -1  # the padding's key
+    keys = pool[torch.randint(0, kinds, (n,), device=eng.device, generator=g)]
+    assert eng.lib.edgpu_sort_unique_fits(words, n) == 1
+    wide = torch.cat([keys, keys], 1)
+    k, p = keys.clone(), torch.arange(n, dtype=torch.int32, device=eng.device)
+    eng.sort_states(k, p)
+    want, _, _ = eng.unique_sorted(k, p)
+    before = keys.clone()
+    assert torch.equal(eng.sort_unique(keys), want) and torch.equal(keys, before)
+    assert torch.equal(eng.sort_unique(wide[:, :words]), want)  # strided rows

@@ -505,3 +505,14 @@ def test_sorted_unique_in_one_launch(eng, n, words, kinds):
     before = keys.clone()
     assert torch.equal(eng.sort_unique(keys), want) and torch.equal(keys, before)
     assert torch.equal(eng.sort_unique(wide[:, :words]), want)  # strided rows
+
+
+@pytest.mark.parametrize("n,n_orb,n_terms,cplx,filled", [
+    (19501, 130, 400, False, 0.95),  # four states a batch, the last ones ragged
+    (20000, 200, 2500, True, 0.97),  # complex operator
+    (20500, 26, 900, False, 0.4),    # more outputs than a batch's scratch holds: one by one
+])
+def test_candidates_of_several_states(eng, n, n_orb, n_terms, cplx, filled, monkeypatch):
+    if n_orb == 26:
+        monkeypatch.setattr(eng, "scratch_entries", 64)
+    test_one_pass_application(eng, n, n_orb, n_terms, cplx, filled)

@@ -1402,8 +1402,8 @@ extern "C" int edgpu_lanczos_timed(const edgpu_csr* h, const double* v0, int R, 
 namespace edgpu {
 size_t reorth_coop_scratch_bytes();
 int lanczos_reorth_coop(const edgpu_csr* h, const double* v0, int j0, int j1, int K_cap, double* Vd, double* wd,
-                        double* alpha, double* beta, int32_t* status_dev, double* scratch, double2* y, double2* pd,
-                        double2* hc, cudaStream_t s);
+                        double* alpha, double* beta, int32_t* status_dev, double* scratch, double2* hc,
+                        cudaStream_t s);
 }  // namespace edgpu
 static std::atomic<int> g_reorth_fused{1};
 
@@ -1448,10 +1448,9 @@ extern "C" int edgpu_lanczos_reorth(const edgpu_csr* h, const double* v0, int j0
   double2* hc = reinterpret_cast<double2*>(carve(sizeof(double2) * (size_t)(K_cap + 1)));
   double* pnp = reinterpret_cast<double*>(carve(sizeof(double) * (size_t)((n + 31) / 32 + 1)));
   double* coop = reinterpret_cast<double*>(carve(reorth_coop_scratch_bytes()));
-  double2* y = reinterpret_cast<double2*>(carve(sizeof(double2) * (size_t)n));
   if (off > workspace_bytes) return EDGPU_ERR_WORKSPACE;
   if (g_reorth_fused.load()) {
-    const int rcc = lanczos_reorth_coop(h, v0, j0, j1, K_cap, Vd, wd, alpha, beta, status_dev, coop, y, pd, hc, s);
+    const int rcc = lanczos_reorth_coop(h, v0, j0, j1, K_cap, Vd, wd, alpha, beta, status_dev, coop, hc, s);
     if (rcc >= 0) return rcc;
   }
   if (j0 == 0) {

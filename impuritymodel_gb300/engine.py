@@ -471,12 +471,15 @@ class Engine:
 
     def _plan(self, dop, w):
         """The operator's terms sorted into groups for states of ``w`` words (edgpu_apply_plan), made
-        on first use and kept with the operator (made again when its tables were written since).
+        on first use and kept with the operator (made again when its tables were written since, and on
+        every call for tables made under inference mode, which count no versions).
         Another stream than the one that made it waits for it, and the memory is kept until that
         stream's work on it is done."""
         plans = dop.__dict__.setdefault("_plans", {})
         stream = torch.cuda.current_stream(self.device)
-        version = (dop.ops._version, dop.coeff._version)
+        version = None
+        if not (dop.ops.is_inference() or dop.coeff.is_inference()):
+            version = (dop.ops._version, dop.coeff._version)
         hit = plans.get(w)
         if hit is not None and hit[3] != version:
             hit = None
@@ -484,6 +487,8 @@ class Engine:
             size = self.lib.edgpu_apply_plan_bytes(dop.n_terms)
             plan = torch.empty(size, dtype=torch.uint8, device=self.device)
             L.check(self.lib.edgpu_apply_plan(w, C.byref(dop.terms), _ptr(plan), size, self.stream), "apply_plan")
+            if version is None:
+                return plan
             hit = plans[w] = (plan, stream.record_event(), stream.cuda_stream, version)
         elif hit[2] != stream.cuda_stream:
             stream.wait_event(hit[1])

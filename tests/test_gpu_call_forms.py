@@ -28,3 +28,48 @@ def test_reorthogonalised_steps_of_any_chunk(eng, n, K, cplx, locked):
         W, c, d = eng.krylov_reorth(csr, v0, K, chunk=chunk, locked=lock)
         assert (a == c).all() and (b == d).all()
         assert torch.equal(torch.view_as_real(V), torch.view_as_real(W))
+
+
+def _hopping(n_orb, value=0.3):
+    """A ring of hops and a density-density term per neighbour."""
+    op = {}
+    for i in range(n_orb):
+        j = (i + 1) % n_orb
+        op[((i, "c"), (i, "a"))] = 0.1 * i
+        op[((i, "c"), (j, "a"))] = value
+        op[((j, "c"), (i, "a"))] = value
+        op[((i, "c"), (j, "c"), (j, "a"), (i, "a"))] = 0.7
+    return op
+
+
+def _start(eng, words=(0b1011 << 60,)):
+    import numpy as np
+
+    return eng.upload_states(np.array([words], dtype=np.uint64))
+
+
+def test_application_of_tables_from_inference_mode(eng):
+    """Tensors made there count no versions; a plan of them is not kept."""
+    from impuritymodel_gb300 import ops as _ops  # noqa: F401  (registers torch.ops.edgpu)
+    from impuritymodel_gb300.engine import DeviceOp
+
+    b0 = _start(eng)
+    plain = DeviceOp(_hopping(9), eng.device)
+    basis, order = eng.expand(b0, plain, None)
+    csr = eng.build_csr(basis, plain, None)
+    with torch.inference_mode():
+        dop = DeviceOp(_hopping(9), eng.device)
+        inside = eng.expand(b0, dop, None) + tuple(getattr(eng.build_csr(basis, dop, None), k)
+                                                   for k in ("row_ptr", "col", "val_r"))
+        none = torch.zeros(0, dtype=torch.int32, device=eng.device)
+        mask = torch.zeros((0, 8), dtype=torch.int64, device=eng.device)
+        ops = torch.ops.edgpu.build_csr(basis, dop.ops, dop.coeff, dop.flags, none, none, mask, 1e-12)
+    outside = eng.build_csr(basis, dop, None)  # the same tensors after the mode has ended
+    again = eng.build_csr(basis, plain, None)  # a plan made outside, read again
+    with torch.inference_mode():
+        again_inside = eng.build_csr(basis, plain, None)
+    assert torch.equal(inside[0], basis) and torch.equal(inside[1], order)
+    for got in (inside[2:], ops, (outside.row_ptr, outside.col, outside.val_r), (again.row_ptr, again.col, again.val_r),
+                (again_inside.row_ptr, again_inside.col, again_inside.val_r)):
+        for x, y in zip(got, (csr.row_ptr, csr.col, csr.val_r)):
+            assert torch.equal(x, y)

@@ -517,23 +517,29 @@ class Engine:
         rp = C.byref(restr) if restr is not None else None
         entry = lib.edgpu_apply_groups_entry_bytes()
         cap = min(16 * n + 4096, n * dop.n_terms) if want else 0
+        # outputs of a state that a warp holds, up to one for every term; what an operator was found to
+        # need stays with it (a large buffer leaves an SM few warps)
+        most = lib.edgpu_apply_groups_max_terms()
+        scratch = min(max(self.scratch_entries, dop.__dict__.get("_scratch", 0)), most)
         scan_ws, scan_n = self.workspace(lib.edgpu_scan_workspace(n))
         while True:
             arena = torch.empty(cap * entry, dtype=torch.uint8, device=dev) if want else None
             L.check(
                 lib.edgpu_apply_groups(w, _ptr(states), n, _ptr(plan), dop.n_terms, int(dop.is_real), rp, weight_min,
                                        _ptr(basis), nb, _ptr(table), 0 if table is None else table.numel(), filt,
-                                       _ptr(buf[n + 1:]), _ptr(arena), cap, self.scratch_entries, _ptr(ws), wsn,
+                                       _ptr(buf[n + 1:]), _ptr(arena), cap, scratch, _ptr(ws), wsn,
                                        self.stream),
                 "apply_groups",
             )
             L.check(lib.edgpu_scan_i64(_ptr(buf[n + 3:]), _ptr(offsets), n, scan_ws, scan_n, self.stream), "scan")
             total, st, need = buf[n: n + 3].tolist()  # an overflowed pass is discarded
-            if st == L.EDGPU_ERR_OVERFLOW and self.scratch_entries < 8192:
-                self.scratch_entries *= 4
+            if st == L.EDGPU_ERR_OVERFLOW and scratch < most:
+                scratch = min(4 * scratch, most)
                 continue
             if st != L.EDGPU_OK:
                 raise L.EdgpuError(st, "apply_groups")
+            if scratch > self.scratch_entries:
+                dop.__dict__["_scratch"] = scratch
             if want and need > cap:
                 cap = need
                 continue

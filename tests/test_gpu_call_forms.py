@@ -73,3 +73,35 @@ def test_application_of_tables_from_inference_mode(eng):
                 (again_inside.row_ptr, again_inside.col, again_inside.val_r)):
         for x, y in zip(got, (csr.row_ptr, csr.col, csr.val_r)):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("full,empty", [(16, 17), (64, 64), (70, 70), (64, 128)])  # outputs: 272, 4096, 4900, 8192
+def test_application_of_more_outputs_than_the_scratch(eng, full, empty, cplx):
+    """Hops from `full` to `empty` orbitals: as many outputs of one state as terms, in their order."""
+    import numpy as np
+
+    from impuritymodel_gb300.engine import DeviceOp
+
+    hops = [(i, j) for i in range(full, full + empty) for j in range(full)]
+    amp = [0.5 + k + (0.25j * k if cplx else 0.0) for k in range(len(hops))]
+    dop = DeviceOp({((i, "c"), (j, "a")): v for (i, j), v in zip(hops, amp)}, eng.device)
+    occ = np.zeros((1, 256), dtype=np.uint8)
+    occ[0, :full] = 1
+    words = lambda o: np.packbits(o, axis=1).view(">u8").astype(np.uint64)  # noqa: E731
+    state = eng.upload_states(words(occ))
+    before = eng.scratch_entries
+    offs, out, _, vals = eng.apply_columns(state, dop, None, 0.0, want_states=True, want_vals=True)
+    want = np.repeat(occ, len(hops), axis=0)
+    for k, (i, j) in enumerate(hops):
+        want[k, i], want[k, j] = 1, 0
+    # j orbitals below the annihilated one, then full - 1 below the created one
+    sign = np.array([(-1.0) ** (j + full - 1) for _, j in hops])
+    assert offs.tolist() == [0, len(hops)]
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), words(want))
+    v = vals.cpu().numpy()
+    assert np.array_equal(v[:, 0] + 1j * v[:, 1], sign * np.array(amp))
+    # what that call needed is no other call's
+    assert eng.scratch_entries == before
+    basis, _ = eng.expand(_start(eng), DeviceOp(_hopping(9), eng.device), None)
+    assert basis.shape == (84, 1)  # three particles on nine orbitals

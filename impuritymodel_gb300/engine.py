@@ -31,6 +31,26 @@ def _ptr(t):
 _TERM_ENCODING = {}
 
 
+def _table_versions(op):
+    """Versions of an operator's device tables, which count the writes to them; None for tables made
+    under inference mode, which count none."""
+    if op.ops.is_inference() or op.coeff.is_inference():
+        return None
+    return op.ops._version, op.coeff._version
+
+
+def read_tables(op):
+    """Sets what the host has to know of an operator's device tables, from one read of them: whether
+    every coefficient is real, and the largest orbital of any slot in use."""
+    op.is_real, op.max_orbital = True, -1
+    if op.n_terms:
+        slots = torch.stack([(op.ops >> (16 * k)) & 0xFFFF for k in range(4)])
+        orb = torch.where((slots & 0x8000) != 0, slots & 0x3FF, -1)
+        cplx, top = torch.stack([(op.coeff[:, 1] != 0).any().to(torch.int64), orb.max()]).tolist()
+        op.is_real, op.max_orbital = not cplx, int(top)
+    op.tables_read = _table_versions(op)
+
+
 class DeviceOp:
     """Operator dict compiled to the device term table of ``edgpu_terms``.
 
@@ -99,6 +119,7 @@ class DeviceOp:
         self.ops = torch.from_numpy(ops.view(np.int64)).to(device)
         self.coeff = torch.from_numpy(coeff).to(device)
         self.flags = torch.from_numpy(flags.view(np.int32)).to(device)
+        self.tables_read = _table_versions(self)  # is_real and max_orbital hold for these
         self.terms = L.Terms(self.ops.data_ptr() if t else 0, self.coeff.data_ptr() if t else 0,
                              self.flags.data_ptr() if t else 0, t)
 
@@ -477,9 +498,7 @@ class Engine:
         stream's work on it is done."""
         plans = dop.__dict__.setdefault("_plans", {})
         stream = torch.cuda.current_stream(self.device)
-        version = None
-        if not (dop.ops.is_inference() or dop.coeff.is_inference()):
-            version = (dop.ops._version, dop.coeff._version)
+        version = _table_versions(dop)
         hit = plans.get(w)
         if hit is not None and hit[3] != version:
             hit = None
@@ -515,6 +534,8 @@ class Engine:
             L.check(lib.edgpu_state_hash_build(w, _ptr(basis), nb, _ptr(table), table.numel(), self.stream),
                     "state_hash")
         rp = C.byref(restr) if restr is not None else None
+        # writes to tables that count none go unseen: their imaginary parts are always added up
+        real = int(dop.is_real and dop.tables_read is not None)
         entry = lib.edgpu_apply_groups_entry_bytes()
         cap = min(16 * n + 4096, n * dop.n_terms) if want else 0
         # outputs of a state that a warp holds, up to one for every term; what an operator was found to
@@ -525,7 +546,7 @@ class Engine:
         while True:
             arena = torch.empty(cap * entry, dtype=torch.uint8, device=dev) if want else None
             L.check(
-                lib.edgpu_apply_groups(w, _ptr(states), n, _ptr(plan), dop.n_terms, int(dop.is_real), rp, weight_min,
+                lib.edgpu_apply_groups(w, _ptr(states), n, _ptr(plan), dop.n_terms, real, rp, weight_min,
                                        _ptr(basis), nb, _ptr(table), 0 if table is None else table.numel(), filt,
                                        _ptr(buf[n + 1:]), _ptr(arena), cap, scratch, _ptr(ws), wsn,
                                        self.stream),
@@ -555,6 +576,8 @@ class Engine:
         return offsets, out
 
     def _groups_ok(self, dop, w):
+        if dop.n_terms and dop.tables_read != _table_versions(dop):
+            read_tables(dop)  # written since
         return 0 < dop.n_terms <= self.lib.edgpu_apply_groups_max_terms() and dop.max_orbital < 64 * w
 
     def apply_columns(self, states, dop, restr, weight_min, basis=None, filt=L.FILTER_NONE, want_states=False,

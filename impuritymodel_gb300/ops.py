@@ -40,15 +40,11 @@ class _TermView:
     """An operator given as term-table tensors, shaped like DeviceOp for the engine."""
 
     def __init__(self, ops, coeff, flags):
+        from .engine import read_tables
+
         self.ops, self.coeff, self.flags = ops, coeff, flags
         self.n_terms = int(ops.numel())
-        self.is_real, self.max_orbital = True, -1
-        if self.n_terms:
-            # one read: imaginary parts present, largest orbital of any slot in use
-            slots = torch.stack([(ops >> (16 * k)) & 0xFFFF for k in range(4)])
-            orb = torch.where((slots & 0x8000) != 0, slots & 0x3FF, -1)
-            cplx, top = torch.stack([(coeff[:, 1] != 0).any().to(torch.int64), orb.max()]).tolist()
-            self.is_real, self.max_orbital = not cplx, int(top)
+        read_tables(self)
         self.terms = L.Terms(ops.data_ptr() if self.n_terms else 0, coeff.data_ptr() if self.n_terms else 0,
                              flags.data_ptr() if self.n_terms else 0, self.n_terms)
 

@@ -105,3 +105,31 @@ def test_application_of_more_outputs_than_the_scratch(eng, full, empty, cplx):
     assert eng.scratch_entries == before
     basis, _ = eng.expand(_start(eng), DeviceOp(_hopping(9), eng.device), None)
     assert basis.shape == (84, 1)  # three particles on nine orbitals
+
+
+def test_application_follows_its_tables(eng):
+    """Tables written in place between two applications: coefficients that become complex, orbitals
+    beyond the states' words."""
+    from impuritymodel_gb300.engine import DeviceOp
+
+    b0 = _start(eng, (0b1011 << 60, 0))  # two words
+    dop = DeviceOp(_hopping(9), eng.device)
+    cols = lambda d: eng.apply_columns(b0, d, None, 0.0, want_states=True, want_vals=True)  # noqa: E731
+    cols(dop)
+    dop.coeff[:, 1] = 0.5 * dop.coeff[:, 0]
+    want = DeviceOp({k: v * (1 + 0.5j) for k, v in _hopping(9).items()}, eng.device)
+    for x, y in zip(cols(dop), cols(want)):
+        assert x is None and y is None or torch.equal(x, y)
+    basis, _ = eng.expand(b0, want, None)
+    one, two = eng.build_csr(basis, dop, None), eng.build_csr(basis, want, None)
+    assert torch.equal(one.val_c, two.val_c) and torch.equal(one.col, two.col)
+    dop.coeff[:, 1] = 0.0  # real again
+    one, two = eng.build_csr(basis, dop, None), eng.build_csr(basis, DeviceOp(_hopping(9), eng.device), None)
+    assert torch.equal(one.val_r, two.val_r) and torch.equal(one.col, two.col)
+    # a hop to an orbital that the words do not hold: the kernel for general tables only empties the
+    # other one, and the plan has no group for it
+    near, far = ((1, "c"), (0, "a")), ((200, "c"), (0, "a"))
+    dop.ops[list(_hopping(9)).index(near)] = DeviceOp({far: 0.3}, eng.device).ops[0]
+    moved = DeviceOp({(far if t == near else t): v for t, v in _hopping(9).items()}, eng.device)
+    for x, y in zip(cols(dop), cols(moved)):
+        assert x is None and y is None or torch.equal(x, y)

@@ -157,9 +157,17 @@ class BasisNet:
         gen.manual_seed(int(seed))
         e, lib = self.eng, self._lib()
         dev = e.device
-        states, log_w = states.contiguous(), log_w.contiguous()
         steps = n // batch
         loss = torch.empty(max(1, epochs * steps), dtype=torch.float32, device=dev)
+        if steps:
+            # the kernels gather rows of both by the shuffled positions, through plain pointers
+            if states.dim() != 2 or states.element_size() != 8:
+                raise ValueError("train: states as [N, W] 64-bit words required")
+            if log_w.shape[0] < n:
+                raise ValueError("train: %d weights for %d states" % (log_w.shape[0], n))
+            if states.device != loss.device or log_w.device != loss.device:
+                raise ValueError("train: states and weights on the engine's device required")
+        states, log_w = states.contiguous(), log_w.to(torch.float32).contiguous()
         wsn = lib.edgpu_mlp_step_workspace(batch)
         ws = torch.empty(wsn if steps else 1, dtype=torch.uint8, device=dev)
         k = 0

@@ -1178,19 +1178,20 @@ __global__ void __launch_bounds__(kGridThreads, 1) lanczos_grid_kernel(GridArgs 
 }
 
 // Launches the cooperative form where the sector's vectors and entries fit in shared memory (without the
-// entries 40 steps of 300 000 rows take 3.4 ms against 2.4 in two launches a step): 1 when it ran, 0 when the caller's two
-// launches a step take the call, -1 on an error.
-static int launch_grid(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, double* alpha,
+// entries 40 steps of 300 000 rows take 3.4 ms against 2.4 in two launches a step): false when the caller's two
+// launches a step take the call, also where the launch is refused (a program that has only a part of the
+// SMs cannot hold all blocks at once).
+static bool launch_grid(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, double* alpha,
                        double* beta, int32_t* status, unsigned char* ws, cudaStream_t s) {
-  if (R > kGridRuns || (!h->val_c && !h->val_r)) return 0;
+  if (R > kGridRuns || (!h->val_c && !h->val_r)) return false;
   const int blocks = grid_cap();
   const int64_t most = (h->n + blocks - 1) / blocks;
   const bool cplx = h->val_c != nullptr;
   const size_t limit = 220 * 1024, per_entry = (cplx ? 16 : 8) + sizeof(int);
-  if (h->n < blocks || most > kGridRows || grid_fixed_bytes(most, R) > limit) return 0;
+  if (h->n < blocks || most > kGridRows || grid_fixed_bytes(most, R) > limit) return false;
   GridArgs g{};
   const size_t room = (limit - grid_fixed_bytes(most, R)) / per_entry;
-  if (room < (size_t)(h->nnz / blocks + h->nnz / blocks / 8 + 64)) return 0;
+  if (room < (size_t)(h->nnz / blocks + h->nnz / blocks / 8 + 64)) return false;
   g.ent_cap = (int)std::min<size_t>(room, (size_t)(2 * (h->nnz / blocks) + 256)) & ~1;
   const size_t bytes = grid_fixed_bytes(most, R) + per_entry * (size_t)g.ent_cap;
   auto kern = cplx ? lanczos_grid_kernel<true> : lanczos_grid_kernel<false>;
@@ -1200,12 +1201,12 @@ static int launch_grid(const edgpu_csr* h, const double* v0, int R, const int32_
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGridThreads, bytes) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
-    return 0;
+    return false;
   }
   // the same places in the workspace as the two launches a step: two vectors, the partials behind the third
   const size_t vec = (sizeof(double2) * (size_t)h->n * R + 255) & ~(size_t)255;
   const size_t part = (sizeof(double) * (size_t)blocks * R + 255) & ~(size_t)255;
-  if (2 * part > vec) return 0;  // pa and pb share the third vector's place
+  if (2 * part > vec) return false;  // pa and pb share the third vector's place
   g.n = h->n;
   g.rp = h->row_ptr;
   g.col = h->col;
@@ -1228,10 +1229,10 @@ static int launch_grid(const edgpu_csr* h, const double* v0, int R, const int32_
   void* args[] = {&g};
   if (cudaLaunchCooperativeKernel((const void*)kern, blocks, kGridThreads, args, bytes, s) != cudaSuccess) {
     cudaGetLastError();
-    return -1;
+    return false;
   }
   note_launch();
-  return 1;
+  return true;
 }
 
 template <typename T>
@@ -1357,8 +1358,7 @@ extern "C" int edgpu_lanczos(const edgpu_csr* h, const double* v0, int R, const 
   if (small_fits(h->n, precision))
     return lanczos_small(h, v0, R, k_max, K, precision, alpha, beta, status_dev, ws, (cudaStream_t)stream);
   if (precision == 0) {
-    const int ran = launch_grid(h, v0, R, k_max, K, alpha, beta, status_dev, ws, (cudaStream_t)stream);
-    if (ran != 0) return ran > 0 ? check_launch() : EDGPU_ERR_CUDA;
+    if (launch_grid(h, v0, R, k_max, K, alpha, beta, status_dev, ws, (cudaStream_t)stream)) return check_launch();
     return lanczos_impl<double>(h, v0, R, k_max, K, alpha, beta, status_dev, ws, workspace_bytes,
                                 (cudaStream_t)stream);
   }
@@ -3189,12 +3189,12 @@ extern "C" size_t edgpu_shifted_solve_workspace(int64_t n, int n_rhs, int nz, in
 
 namespace {
 
-// Launches the clusters where one of the sizes holds every right-hand side at once: the size, 0 where
-// none does (the caller's one-CTA form, which keeps every SM busy then), -1 on an error.  A warp's worth of
+// Launches the clusters where one of the sizes holds every right-hand side at once; false where
+// none does (the caller's one-CTA form, which keeps every SM busy then) or is accepted.  A warp's worth of
 // rows has nothing to share: 1 row takes 130 us on one CTA and 145 on a cluster, 33 rows 342 and 327.
-int launch_shifted_cluster(edgpu::ShiftedArgs g, bool cplx, int64_t nnz, cudaStream_t s) {
+bool launch_shifted_cluster(edgpu::ShiftedArgs g, bool cplx, int64_t nnz, cudaStream_t s) {
   using namespace edgpu;
-  if (g.n <= 32) return 0;
+  if (g.n <= 32) return false;
   const size_t per_entry = (cplx ? 16 : 8) + 2;
   for (int cl = kClusterMax; cl > 1; cl >>= 1) {
     if ((int64_t)g.n_rhs * cl > grid_cap()) continue;
@@ -3236,9 +3236,10 @@ int launch_shifted_cluster(edgpu::ShiftedArgs g, bool cplx, int64_t nnz, cudaStr
       continue;
     }
     if (fit < g.n_rhs) continue;
-    return cudaLaunchKernelEx(&cfg, kern, c) == cudaSuccess ? cl : -1;
+    if (cudaLaunchKernelEx(&cfg, kern, c) == cudaSuccess) return true;
+    cudaGetLastError();
   }
-  return 0;
+  return false;
 }
 
 int shifted_solve_impl(const edgpu_csr* h, const double* Y, int n_rhs, const double* zs, int nz, int k_cap, double tol,
@@ -3304,9 +3305,7 @@ int shifted_solve_impl(const edgpu_csr* h, const double* Y, int n_rhs, const dou
     g.ynorm = yn;
     g.status = status_dev;
     const size_t per_entry = (h->val_c ? 16 : 8) + 2;
-    const int cl = launch_shifted_cluster(g, h->val_c != nullptr, h->nnz, s);
-    if (cl < 0) return EDGPU_ERR_CUDA;
-    if (cl == 0) {
+    if (!launch_shifted_cluster(g, h->val_c != nullptr, h->nnz, s)) {
       g.main_threads = std::min(kSmallThreads, npad);
       const int threads = g.main_threads + (nz + 31) / 32 * 32;
       // shared memory: vectors, sums, slots; the sliced entries when a third more than nnz of them fit

@@ -133,3 +133,72 @@ def test_application_follows_its_tables(eng):
     moved = DeviceOp({(far if t == near else t): v for t, v in _hopping(9).items()}, eng.device)
     for x, y in zip(cols(dop), cols(moved)):
         assert x is None and y is None or torch.equal(x, y)
+
+
+@pytest.fixture(scope="module")
+def refusing(eng, tmp_path_factory):
+    """A copy of the library whose cooperative and cluster launches are refused, by the linker's
+    stand-ins for the two runtime calls, as where a program holds only a part of the SMs."""
+    import glob
+    import os
+    import subprocess
+
+    from impuritymodel_gb300 import _lib as L
+    from impuritymodel_gb300 import nvcc_build
+
+    out = tmp_path_factory.mktemp("refusing")
+    src = out / "refuse.cu"
+    src.write_text("""
+#include <cuda_runtime.h>
+static int refused = 0;
+extern "C" cudaError_t __wrap_cudaLaunchCooperativeKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) {
+  ++refused;
+  return cudaErrorCooperativeLaunchTooLarge;
+}
+extern "C" cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) {
+  ++refused;
+  return cudaErrorInvalidClusterSize;
+}
+extern "C" int launches_refused() { return refused; }
+""")
+    so = str(out / "librefusing.so")
+    objs = glob.glob(os.path.join(nvcc_build.BUILD_DIR, "*.o"))
+    subprocess.run([nvcc_build._nvcc(), *nvcc_build.ARCH, "-Xcompiler", "-fPIC", "-shared", "-o", so, str(src), *objs,
+                    "-cudart", "static", "-Xlinker", "--wrap=cudaLaunchCooperativeKernel", "-Xlinker",
+                    "--wrap=cudaLaunchKernelExC"], check=True, capture_output=True)
+    return L.load(so)
+
+
+@pytest.mark.parametrize("n,R,K,cplx", [(4300, 1, 12, False), (20000, 3, 12, True), (47895, 8, 9, False)])
+def test_large_sectors_where_cooperative_launches_are_refused(eng, refusing, monkeypatch, n, R, K, cplx):
+    """The two launches a step take the call, to the rounding of another order of sums."""
+    csr, H = _random_csr(eng, n, n + R, cplx, heavy=(0, 1, n // 2))
+    g = torch.Generator(device=eng.device)
+    g.manual_seed(R)
+    v = torch.randn((n, R), dtype=torch.complex128, device=eng.device, generator=g)
+    v /= torch.linalg.vector_norm(v, dim=0)
+    a, b = eng.lanczos(csr, v, [K] * R)
+    before = refusing.launches_refused()
+    monkeypatch.setattr(eng, "lib", refusing)
+    a1, b1 = eng.lanczos(csr, v, [K] * R)
+    assert refusing.launches_refused() == before + 1
+    # a dozen steps of an unconverged recurrence amplify rounding by less than 1e3
+    tol = 1e-12 * abs(H).sum(1).max()
+    assert (a - a1).abs().max().item() < tol and (b - b1)[:, :K - 1].abs().max().item() < tol
+
+
+@pytest.mark.parametrize("n,R,cplx", [(40, 2, False), (360, 15, False), (360, 70, True)])
+def test_shifted_solves_where_cluster_launches_are_refused(eng, refusing, monkeypatch, n, R, cplx):
+    csr, _ = _random_csr(eng, n, n + R, cplx, heavy=(0,))
+    g = torch.Generator(device=eng.device)
+    g.manual_seed(n)
+    y = torch.randn((R, n), dtype=torch.complex128, device=eng.device, generator=g)
+    y /= torch.linalg.vector_norm(y, dim=1, keepdim=True)
+    zs = torch.linspace(-8.0, 8.0, 3 * R, dtype=torch.float64).view(R, 3).numpy() + 0.5j
+    X, _ = eng.shifted_solve(csr, y, zs, 1e-10, min(6 * n + 50, 2000))
+    before = refusing.launches_refused()
+    monkeypatch.setattr(eng, "lib", refusing)
+    X1, _ = eng.shifted_solve(csr, y, zs, 1e-10, min(6 * n + 50, 2000))
+    assert refusing.launches_refused() > before
+    # either residual is below 1e-10, and |(z - H)^{-1}| <= 1 / Im z; as much again for the rounding
+    assert torch.linalg.vector_norm(X - X1, dim=2).max().item() <= 8e-10

@@ -108,8 +108,8 @@ __global__ void spmm_alpha_kernel(int64_t n, const int64_t* __restrict__ rp, con
 
 // ---------------------------------------------------------------------------------------
 // Grid-wide batched Lanczos (lanczos_impl): two launches per step on vectors kept unnormalised.
-// Serves complex64 vectors, more runs or larger sectors than lanczos_grid_kernel below, the timed and the
-// allocation-free entry points.
+// Serves complex64 vectors, more runs or larger sectors than lanczos_grid_kernel below, and the
+// allocation-free entry point (whose callers forbid what a cooperative launch might allocate in the driver).
 //
 // w_j is stored as it leaves the three-term update and v_j = w_j / beta_{j-1} is never formed:
 // the first launch takes y = H w_j and the partial sums of <y, w_j>, the second
@@ -1302,6 +1302,37 @@ int lanczos_impl(const edgpu_csr* h, const double* v0, int R, const int32_t* k_m
   return EDGPU_OK;
 }
 
+// The milliseconds of what run() launches into kernel_ms[0] (the others 0) where kernel_ms is given.
+template <typename F>
+auto timed_whole(double* kernel_ms, cudaStream_t s, F&& run) {
+  if (!kernel_ms) return run();
+  cudaEvent_t e0, e1;
+  cudaEventCreate(&e0);
+  cudaEventCreate(&e1);
+  cudaEventRecord(e0, s);
+  const auto rc = run();
+  cudaEventRecord(e1, s);
+  cudaEventSynchronize(e1);
+  float ms = 0.f;
+  cudaEventElapsedTime(&ms, e0, e1);
+  kernel_ms[0] = ms;
+  kernel_ms[1] = kernel_ms[2] = 0.0;
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  return rc;
+}
+
+// Sectors beyond one SM's shared memory, the same for the timed entry point and the plain one: a timed run
+// has the other's bits, and its time is of the kernels that the other runs.
+static int lanczos_large(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, int precision,
+                         double* alpha, double* beta, int32_t* status, unsigned char* ws, size_t ws_bytes,
+                         cudaStream_t s, double* kernel_ms = nullptr) {
+  if (precision != 0) return lanczos_impl<float>(h, v0, R, k_max, K, alpha, beta, status, ws, ws_bytes, s, kernel_ms);
+  if (timed_whole(kernel_ms, s, [&] { return launch_grid(h, v0, R, k_max, K, alpha, beta, status, ws, s); }))
+    return check_launch();
+  return lanczos_impl<double>(h, v0, R, k_max, K, alpha, beta, status, ws, ws_bytes, s, kernel_ms);
+}
+
 }  // namespace edgpu
 
 using namespace edgpu;
@@ -1357,12 +1388,8 @@ extern "C" int edgpu_lanczos(const edgpu_csr* h, const double* v0, int R, const 
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
   if (small_fits(h->n, precision))
     return lanczos_small(h, v0, R, k_max, K, precision, alpha, beta, status_dev, ws, (cudaStream_t)stream);
-  if (precision == 0) {
-    if (launch_grid(h, v0, R, k_max, K, alpha, beta, status_dev, ws, (cudaStream_t)stream)) return check_launch();
-    return lanczos_impl<double>(h, v0, R, k_max, K, alpha, beta, status_dev, ws, workspace_bytes,
-                                (cudaStream_t)stream);
-  }
-  return lanczos_impl<float>(h, v0, R, k_max, K, alpha, beta, status_dev, ws, workspace_bytes, (cudaStream_t)stream);
+  return lanczos_large(h, v0, R, k_max, K, precision, alpha, beta, status_dev, ws, workspace_bytes,
+                       (cudaStream_t)stream);
 }
 
 extern "C" int edgpu_lanczos_timed(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K,
@@ -1374,29 +1401,12 @@ extern "C" int edgpu_lanczos_timed(const edgpu_csr* h, const double* v0, int R, 
   precision = effective_precision(h, precision);
   if (workspace_bytes < edgpu_lanczos_workspace(h->n, R, K, precision)) return EDGPU_ERR_WORKSPACE;
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
-  if (small_fits(h->n, precision)) {
-    cudaStream_t s = (cudaStream_t)stream;
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, s);
-    int rc = lanczos_small(h, v0, R, k_max, K, precision, alpha, beta, status_dev, ws, s);
-    cudaEventRecord(e1, s);
-    cudaEventSynchronize(e1);
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    kernel_ms[0] = ms;  // whole fused Krylov loop (SpMV, reductions, axpy) in one launch
-    kernel_ms[1] = 0.0;
-    kernel_ms[2] = 0.0;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    return rc;
-  }
-  if (precision == 0)
-    return lanczos_impl<double>(h, v0, R, k_max, K, alpha, beta, status_dev, ws, workspace_bytes,
-                                (cudaStream_t)stream, kernel_ms);
-  return lanczos_impl<float>(h, v0, R, k_max, K, alpha, beta, status_dev, ws, workspace_bytes, (cudaStream_t)stream,
-                             kernel_ms);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (small_fits(h->n, precision))  // the whole recurrence (products, sums, updates) in one launch
+    return timed_whole(kernel_ms, s, [&] {
+      return lanczos_small(h, v0, R, k_max, K, precision, alpha, beta, status_dev, ws, s);
+    });
+  return lanczos_large(h, v0, R, k_max, K, precision, alpha, beta, status_dev, ws, workspace_bytes, s, kernel_ms);
 }
 
 namespace edgpu {

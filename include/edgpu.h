@@ -348,10 +348,10 @@ int edgpu_lanczos(const edgpu_csr* h, const double* v0, int R, const int32_t* k_
                   void* stream);
 
 /*
- * edgpu_lanczos with CUDA-event timing of its kernels on the launching stream:
+ * edgpu_lanczos (the same kernels, the same bits) with CUDA-event timing on the launching stream:
  * kernel_ms (host, 3 doubles) receives the summed milliseconds of the products, of the
- * vector updates and 0 (sectors that do not fit in one SM: always the two launches per step), or the
- * whole of a small sector's launch and two zeros.  Synchronises on the last event before returning.
+ * vector updates and 0 where a step is two launches, or the whole and two zeros where one launch takes
+ * all steps.  Synchronises on the last event before returning.
  */
 int edgpu_lanczos_timed(const edgpu_csr* h, const double* v0, int R, const int32_t* k_max, int K, int precision,
                         double* alpha, double* beta, int32_t* status_dev, void* workspace, size_t workspace_bytes,
@@ -366,7 +366,8 @@ long long edgpu_launch_count(void);
  * the whole GPU and forbids cudaMalloc, or a solver loop embedded in another program where
  * an allocation would synchronise the device between time steps.  The caller passes the
  * inputs and outputs of edgpu_lanczos (no workspace); this always runs the grid-wide
- * batched Lanczos (two kernels per step) and keeps its scratch (three [n][R] vectors
+ * batched Lanczos (two kernels per step; in FP64 its sums round in another order than the one launch
+ * of edgpu_lanczos) and keeps its scratch (three [n][R] vectors
  * and partial sums, size edgpu_lanczos_workspace(n, R, K, precision)) in a static
  * device array of EDGPU_LANCZOS_NOALLOC_BYTES inside the library, which every GPU that
  * loads the library holds until the process exits.  Larger problems are rejected with

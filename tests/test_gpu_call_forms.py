@@ -202,3 +202,23 @@ def test_shifted_solves_where_cluster_launches_are_refused(eng, refusing, monkey
     assert refusing.launches_refused() > before
     # either residual is below 1e-10, and |(z - H)^{-1}| <= 1 / Im z; as much again for the rounding
     assert torch.linalg.vector_norm(X - X1, dim=2).max().item() <= 8e-10
+
+
+@pytest.mark.parametrize("n,R,K,precision", [
+    (1770, 3, 40, 0),    # one SM
+    (4300, 2, 25, 0),    # one cooperative launch
+    (47895, 3, 30, 0),
+    (5000, 33, 10, 0),   # two launches a step
+    (5000, 40, 10, 1),
+])
+def test_timed_lanczos_is_the_plain_one(eng, n, R, K, precision):
+    csr, _ = _random_csr(eng, n, n + R, heavy=(0, n // 2))
+    g = torch.Generator(device=eng.device)
+    g.manual_seed(n)
+    v = torch.randn((n, R), dtype=torch.complex128, device=eng.device, generator=g)
+    v /= torch.linalg.vector_norm(v, dim=0)
+    a, b = eng.lanczos(csr, v, [K] * R, precision=precision)
+    timing = []
+    a1, b1 = eng.lanczos(csr, v, [K] * R, precision=precision, timing=timing)
+    assert torch.equal(a, a1) and torch.equal(b, b1)
+    assert timing[0]["spmm_ms"] > 0.0 and timing[0]["axpy_ms"] >= 0.0 and timing[0]["normalize_ms"] == 0.0

@@ -812,7 +812,9 @@ __global__ void __launch_bounds__(kRankThreads, 1)
         part[quarter - 1][kBM + row] = zz.x + zz.y;
         mbar_arrive(&quarter_sums);
       } else {
-        ok = mbar_wait(&quarter_sums, pass_phase);
+        // one answer for the warp here too: a lane that gave up alone would be missing from the next vote
+        ok = __all_sync(0xffffffffu, mbar_wait(&quarter_sums, pass_phase));
+        if (!ok) break;
         const float b3 = __ldg(g.b3);
         if (base + row < g.n) g.y[base + row] = ((ss.x + ss.y) + part[0][row]) + (part[1][row] + part[2][row]) + b3;
         if (two && base + kBM + row < g.n)

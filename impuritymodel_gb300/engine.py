@@ -383,6 +383,7 @@ class Engine:
     def read_status(self, where):
         st = int(self.status.item())
         if st != L.EDGPU_OK:
+            self.reset_status()  # spent: the next reader asks for its own call's
             raise L.EdgpuError(st, where)
 
     def upload_states(self, words):
@@ -1187,6 +1188,8 @@ class Engine:
             ev_next = enqueue(j1, jn) if jn > j1 else None  # speculative next chunk
             st = int(host[0])
             ah, bh = host[1:1 + j1], host[1 + j1:]
+            if st != L.EDGPU_OK:
+                self.reset_status()  # behind the chunk already queued, which sets it again
             if st == L.EDGPU_ERR_BREAKDOWN:
                 # invariant subspace: the Krylov space is exact at the first zero beta
                 kb = int(np.argmax(bh == 0.0)) + 1
@@ -1228,6 +1231,8 @@ class Engine:
 
         def finish():
             st = int(status.item())
+            if st != L.EDGPU_OK:
+                status.zero_()
             if st == L.EDGPU_ERR_NOCONV:
                 # upstream only prints when BiCGSTAB misses its tolerance (spectra.py:963-971)
                 warnings.warn("shifted solve: residual tolerance %g not reached in %d Krylov steps" % (tol, k_cap))

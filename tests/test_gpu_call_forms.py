@@ -222,3 +222,36 @@ def test_timed_lanczos_is_the_plain_one(eng, n, R, K, precision):
     a1, b1 = eng.lanczos(csr, v, [K] * R, precision=precision, timing=timing)
     assert torch.equal(a, a1) and torch.equal(b, b1)
     assert timing[0]["spmm_ms"] > 0.0 and timing[0]["axpy_ms"] >= 0.0 and timing[0]["normalize_ms"] == 0.0
+
+
+def test_a_read_status_is_spent(eng):
+    """What one call set and answered for is no later call's error."""
+    import numpy as np
+
+    from impuritymodel_gb300 import _lib as L
+    from impuritymodel_gb300.engine import CsrMatrix, DeviceOp
+    from impuritymodel_gb300.pruning import BasisNet
+
+    n = 12
+    csr = CsrMatrix(torch.arange(n + 1, device=eng.device), torch.arange(n, dtype=torch.int32, device=eng.device),
+                    val_r=torch.arange(n, dtype=torch.float64, device=eng.device))
+    v = torch.zeros(n, dtype=torch.complex128, device=eng.device)
+    v[3] = 1.0
+    net, dop = BasisNet(eng, seed=0), DeviceOp(_hopping(9), eng.device)
+    eng.reset_status()
+
+    def rank():
+        basis, _ = eng.expand(_start(eng, (0b1011 << 60, 0, 0, 0, 0)), dop, None)
+        assert net.predict(basis).shape == (84,)
+
+    V, a, b = eng.krylov_reorth(csr, v, 8, chunk=2)  # an eigenvector: the space is exhausted at once
+    assert len(a) == 1 and a[0] == 3.0 and b[0] == 0.0
+    rank()
+    with pytest.raises(L.EdgpuError):
+        eng.lanczos(csr, v.view(n, 1), [4])
+    rank()
+    zs = np.full((1, 1), 3.5 + 0.1j)
+    y = torch.ones((1, n), dtype=torch.complex128, device=eng.device)
+    with pytest.warns(UserWarning):
+        eng.shifted_solve(csr, y, zs, 1e-13, 2)
+    rank()

@@ -517,7 +517,8 @@ class Engine:
 
     def _apply_groups(self, states, dop, restr, weight_min, basis, filt, want, conj):
         """H|b> of every state in one pass (edgpu_apply_groups).  ``want``: names of the outputs
-        ("states", "index", "vals", "col", "real"); none: counts only.  Returns (offsets, dict)."""
+        ("states", "index", "vals", "col", "real"); none: counts only.  Returns (offsets, dict), or None
+        where memory does not hold the outputs twice (32 bytes each in the arena)."""
         n, w = states.shape
         dev, lib = self.device, self.lib
         plan = self._plan(dop, w)
@@ -544,8 +545,14 @@ class Engine:
         most = lib.edgpu_apply_groups_max_terms()
         scratch = min(max(self.scratch_entries, dop.__dict__.get("_scratch", 0)), most)
         scan_ws, scan_n = self.workspace(lib.edgpu_scan_workspace(n))
+        arena = None
         while True:
-            arena = torch.empty(cap * entry, dtype=torch.uint8, device=dev) if want else None
+            if want and (arena is None or arena.numel() < cap * entry):
+                arena = None
+                try:
+                    arena = torch.empty(cap * entry, dtype=torch.uint8, device=dev)
+                except torch.cuda.OutOfMemoryError:
+                    return None
             L.check(
                 lib.edgpu_apply_groups(w, _ptr(states), n, _ptr(plan), dop.n_terms, real, rp, weight_min,
                                        _ptr(basis), nb, _ptr(table), 0 if table is None else table.numel(), filt,
@@ -568,7 +575,10 @@ class Engine:
             break
         kinds = {"states": ((total, w), torch.int64), "index": ((total,), torch.int64), "col": ((total,), torch.int32),
                  "vals": ((total, 2), torch.float64), "real": ((total,), torch.float64)}
-        out = {k: torch.empty(kinds[k][0], dtype=kinds[k][1], device=dev) for k in want}
+        try:
+            out = {k: torch.empty(kinds[k][0], dtype=kinds[k][1], device=dev) for k in want}
+        except torch.cuda.OutOfMemoryError:
+            return None
         if total and want:
             L.check(
                 lib.edgpu_apply_groups_gather(w, _ptr(states), n, _ptr(offsets), _ptr(arena),
@@ -587,9 +597,12 @@ class Engine:
         n, w = states.shape
         if n and self._groups_ok(dop, w):
             want = [k for k, on in (("states", want_states), ("index", want_index), ("vals", want_vals)) if on]
-            offsets, out = self._apply_groups(states, dop, restr, weight_min, basis, filt, want, conj)
-            return offsets, out.get("states"), out.get("index"), out.get("vals")
-        # operators of more terms, or with orbitals beyond the states' words: a count and a fill pass
+            got = self._apply_groups(states, dop, restr, weight_min, basis, filt, want, conj)
+            if got is not None:
+                offsets, out = got
+                return offsets, out.get("states"), out.get("index"), out.get("vals")
+        # operators of more terms, or with orbitals beyond the states' words, or outputs that only just fit in
+        # memory: a count and a fill pass
         offsets = torch.zeros(n + 1, dtype=torch.int64, device=self.device)
         empty = torch.empty((0, w), dtype=torch.int64, device=self.device)
         if n == 0 or dop.n_terms == 0:
@@ -787,11 +800,13 @@ class Engine:
         n, w = basis_sorted.shape
         if n and self._groups_ok(dop, w):
             val = "real" if dop.is_real else "vals"
-            offsets, out = self._apply_groups(basis_sorted, dop, restr, weight_min, basis_sorted, L.FILTER_IN_BASIS,
-                                              ("col", val), True)
-            if dop.is_real:
-                return CsrMatrix(offsets, out["col"], val_r=out["real"])
-            return CsrMatrix(offsets, out["col"], val_c=out["vals"])
+            got = self._apply_groups(basis_sorted, dop, restr, weight_min, basis_sorted, L.FILTER_IN_BASIS,
+                                     ("col", val), True)
+            if got is not None:
+                offsets, out = got
+                if dop.is_real:
+                    return CsrMatrix(offsets, out["col"], val_r=out["real"])
+                return CsrMatrix(offsets, out["col"], val_c=out["vals"])
         offsets, _, idx, vals = self.apply_columns(basis_sorted, dop, restr, weight_min, basis=basis_sorted,
                                                    filt=L.FILTER_IN_BASIS, want_index=True, want_vals=True, conj=True)
         col = idx.to(torch.int32)

@@ -255,3 +255,36 @@ def test_a_read_status_is_spent(eng):
     with pytest.warns(UserWarning):
         eng.shifted_solve(csr, y, zs, 1e-13, 2)
     rank()
+
+
+@pytest.mark.parametrize("grown", [False, True])
+def test_application_without_room_for_its_arena(eng, monkeypatch, grown):
+    """The two passes, which keep nothing but the outputs, take the call."""
+    from impuritymodel_gb300 import _lib as L
+    from impuritymodel_gb300.engine import DeviceOp
+
+    op = _hopping(26)
+    # without `grown` the first arena is refused, with it the one for 45 outputs a state that follows
+    op.update({((i, "c"), (j, "a")): 0.01 * (i + 1) * (j + 1) for i in range(26) for j in range(26) if (i - j) % 26 > 1})
+    dop = DeviceOp(op, eng.device)
+    basis, _ = eng.expand(_start(eng, (0b1011 << 60,)), dop, None)
+    assert basis.shape == (2600, 1)
+    want_c = eng.apply_columns(basis, dop, None, 0.0, want_states=True, want_vals=True)
+    want = eng.build_csr(basis, dop, None)
+    entry, first = eng.lib.edgpu_apply_groups_entry_bytes(), 16 * 2600 + 4096
+    assert want.nnz > first
+    empty = torch.empty
+
+    def refuse(*size, **kw):
+        if kw.get("dtype") == torch.uint8 and size[0] >= entry * (first + 1 if grown else first):
+            raise torch.cuda.OutOfMemoryError("refused")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", refuse)
+    got = eng.build_csr(basis, dop, None)
+    got_c = eng.apply_columns(basis, dop, None, 0.0, want_states=True, want_vals=True)
+    for k in ("row_ptr", "col", "val_r"):
+        assert torch.equal(getattr(got, k), getattr(want, k))
+    for x, y in zip(got_c, want_c):
+        assert x is None and y is None or torch.equal(x, y)
+    assert L.EDGPU_OK == int(eng.status.item())

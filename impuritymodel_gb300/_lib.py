@@ -85,6 +85,7 @@ SIGNATURES = {
     "edgpu_apply_groups_max_terms": (_I, []),
     "edgpu_apply_plan_bytes": (_SZ, [_I]),
     "edgpu_apply_plan": (_I, [_I, C.POINTER(Terms), _P, _SZ, _P]),
+    "edgpu_term_info": (_I, [C.POINTER(Terms), _P, _P]),
     "edgpu_apply_groups_workspace": (_SZ, [_I64]),
     "edgpu_apply_groups_entry_bytes": (_SZ, []),
     "edgpu_apply_groups": (

@@ -233,6 +233,34 @@ __global__ void __launch_bounds__(kPlanThreads) apply_plan_kernel(const uint64_t
   }
 }
 
+// Whether any coefficient has an imaginary part, and the largest orbital of any slot in use (-1: none): one
+// launch for some 18 tensor operations on every call with a caller's own tables (torch.ops.edgpu.build_csr of
+// 1 to 700 states: 410-500 us by two passes, 560-590 with the tensor operations, 290-330 so).
+__global__ void __launch_bounds__(kPlanThreads) term_info_kernel(const uint64_t* __restrict__ ops,
+                                                                 const double2* __restrict__ coeff, int T,
+                                                                 int32_t* __restrict__ info) {
+  __shared__ int top[kPlanThreads / 32];
+  int cplx = 0, orb = -1;
+  for (int t = threadIdx.x; t < T; t += kPlanThreads) {
+    cplx |= coeff[t].y != 0.0;
+    const uint64_t o = ops[t];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t op = (uint32_t)(o >> (16 * k)) & 0xFFFFu;
+      if (op & 0x8000u) orb = max(orb, (int)(op & 0x3FFu));
+    }
+  }
+  orb = __reduce_max_sync(0xffffffffu, orb);
+  if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = orb;
+  cplx = __syncthreads_or(cplx);
+  if (threadIdx.x >= 32) return;
+  orb = __reduce_max_sync(0xffffffffu, top[threadIdx.x]);
+  if (threadIdx.x == 0) {
+    info[0] = cplx != 0;
+    info[1] = orb;
+  }
+}
+
 // Outputs of a state in the arena, in upstream's order of first occurrence.
 struct Entry {
   uint64_t key;   // flipped orbitals (Plan::gkey)
@@ -844,6 +872,14 @@ extern "C" int edgpu_apply_plan(int n_words, const edgpu_terms* terms, void* pla
     return EDGPU_ERR_CUDA;
   apply_plan_kernel<<<1, kPlanThreads, smem, (cudaStream_t)stream>>>(
       terms->ops, reinterpret_cast<const double2*>(terms->coeff), terms->n_terms, N, 64 * n_words, plan);
+  note_launch();
+  return check_launch();
+}
+
+extern "C" int edgpu_term_info(const edgpu_terms* terms, int32_t* info, void* stream) {
+  if (!terms || !info || terms->n_terms < 1 || !terms->ops || !terms->coeff) return EDGPU_ERR_ARG;
+  term_info_kernel<<<1, kPlanThreads, 0, (cudaStream_t)stream>>>(
+      terms->ops, reinterpret_cast<const double2*>(terms->coeff), terms->n_terms, info);
   note_launch();
   return check_launch();
 }

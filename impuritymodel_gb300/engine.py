@@ -39,18 +39,6 @@ def _table_versions(op):
     return op.ops._version, op.coeff._version
 
 
-def read_tables(op):
-    """Sets what the host has to know of an operator's device tables, from one read of them: whether
-    every coefficient is real, and the largest orbital of any slot in use."""
-    op.is_real, op.max_orbital = True, -1
-    if op.n_terms:
-        slots = torch.stack([(op.ops >> (16 * k)) & 0xFFFF for k in range(4)])
-        orb = torch.where((slots & 0x8000) != 0, slots & 0x3FF, -1)
-        cplx, top = torch.stack([(op.coeff[:, 1] != 0).any().to(torch.int64), orb.max()]).tolist()
-        op.is_real, op.max_orbital = not cplx, int(top)
-    op.tables_read = _table_versions(op)
-
-
 class DeviceOp:
     """Operator dict compiled to the device term table of ``edgpu_terms``.
 
@@ -491,6 +479,17 @@ class Engine:
     # -- operator application -------------------------------------------------------------
     TABLE_MIN_BASIS = 4096  # basis lookups through a hash table from this size on
 
+    def read_tables(self, op):
+        """Sets what the host has to know of an operator's device tables, from one read of them: whether
+        every coefficient is real, and the largest orbital of any slot in use."""
+        op.is_real, op.max_orbital = True, -1
+        if op.n_terms:
+            info = torch.empty(2, dtype=torch.int32, device=self.device)
+            L.check(self.lib.edgpu_term_info(C.byref(op.terms), _ptr(info), self.stream), "term_info")
+            cplx, op.max_orbital = info.tolist()
+            op.is_real = not cplx
+        op.tables_read = _table_versions(op)
+
     def _plan(self, dop, w):
         """The operator's terms sorted into groups for states of ``w`` words (edgpu_apply_plan), made
         on first use and kept with the operator (made again when its tables were written since, and on
@@ -588,7 +587,7 @@ class Engine:
 
     def _groups_ok(self, dop, w):
         if dop.n_terms and dop.tables_read != _table_versions(dop):
-            read_tables(dop)  # written since
+            self.read_tables(dop)  # written since
         return 0 < dop.n_terms <= self.lib.edgpu_apply_groups_max_terms() and dop.max_orbital < 64 * w
 
     def apply_columns(self, states, dop, restr, weight_min, basis=None, filt=L.FILTER_NONE, want_states=False,

@@ -39,14 +39,12 @@ def _csr(row_ptr, col, val, ncols=None):
 class _TermView:
     """An operator given as term-table tensors, shaped like DeviceOp for the engine."""
 
-    def __init__(self, ops, coeff, flags):
-        from .engine import read_tables
-
+    def __init__(self, eng, ops, coeff, flags):
         self.ops, self.coeff, self.flags = ops, coeff, flags
         self.n_terms = int(ops.numel())
-        read_tables(self)
         self.terms = L.Terms(ops.data_ptr() if self.n_terms else 0, coeff.data_ptr() if self.n_terms else 0,
                              flags.data_ptr() if self.n_terms else 0, self.n_terms)
+        eng.read_tables(self)
 
 
 def _restr(lo, hi, mask):
@@ -117,7 +115,7 @@ def build_csr(basis: Tensor, ops: Tensor, coeff: Tensor, flags: Tensor, lo: Tens
     """Sector Hamiltonian on a sorted basis [n, W]: (row_ptr, col, val); val float64 [nnz] when
     every coefficient is real, else [nnz, 2]."""
     eng = _engine()
-    csr = eng.build_csr(basis.contiguous(), _TermView(ops, coeff, flags), _restr(lo, hi, mask), weight_min)
+    csr = eng.build_csr(basis.contiguous(), _TermView(eng, ops, coeff, flags), _restr(lo, hi, mask), weight_min)
     val = csr.val_r if csr.val_r is not None else csr.val_c
     return csr.row_ptr, csr.col, val
 
@@ -134,7 +132,7 @@ def expand(basis0: Tensor, ops: Tensor, coeff: Tensor, flags: Tensor, lo: Tensor
            weight_min: float) -> tuple[Tensor, Tensor]:
     """Closure of basis0 [n0, W]: (sorted basis, upstream's layered order), both [N, W]."""
     eng = _engine()
-    return eng.expand(basis0.contiguous(), _TermView(ops, coeff, flags), _restr(lo, hi, mask), weight_min)
+    return eng.expand(basis0.contiguous(), _TermView(eng, ops, coeff, flags), _restr(lo, hi, mask), weight_min)
 
 
 @expand.register_fake

@@ -139,6 +139,8 @@ int edgpu_apply_columns(int n_words, const uint64_t* states, int64_t n_states, c
 int edgpu_apply_groups_max_terms(void);
 size_t edgpu_apply_plan_bytes(int n_terms);
 int edgpu_apply_plan(int n_words, const edgpu_terms* terms, void* plan, size_t bytes, void* stream);
+/* info [2] (device): whether any coefficient has an imaginary part, and the largest orbital in use. */
+int edgpu_term_info(const edgpu_terms* terms, int32_t* info, void* stream);
 size_t edgpu_apply_groups_workspace(int64_t n_states);
 size_t edgpu_apply_groups_entry_bytes(void);
 int edgpu_apply_groups(int n_words, const uint64_t* states, int64_t n_states, const void* plan, int n_terms,

@@ -288,3 +288,26 @@ def test_application_without_room_for_its_arena(eng, monkeypatch, grown):
     for x, y in zip(got_c, want_c):
         assert x is None and y is None or torch.equal(x, y)
     assert L.EDGPU_OK == int(eng.status.item())
+
+
+@pytest.mark.parametrize("terms", [1, 33, 1025, 9000])
+@pytest.mark.parametrize("cplx,top", [(False, -1), (True, 700), (False, 1023)])
+def test_what_the_host_reads_of_tables(eng, terms, cplx, top):
+    """Imaginary parts and the largest orbital, the last term alone deciding; unused slots hold none."""
+    from types import SimpleNamespace
+
+    from impuritymodel_gb300 import _lib as L
+
+    ops = torch.zeros(terms, dtype=torch.int64, device=eng.device)
+    ops[:-1] = 0x0000_03FF_8005_C007  # orbital 1023 in a slot that is not in use
+    coeff = torch.zeros((terms, 2), dtype=torch.float64, device=eng.device)
+    coeff[:, 0], coeff[:, 1] = 1.0, -0.0
+    flags = torch.zeros(terms, dtype=torch.int32, device=eng.device)
+    if top >= 0:
+        ops[-1] = (0x8000 | top) << 32
+    if cplx:
+        coeff[-1, 1] = float("nan") if terms == 33 else 1e-300
+    op = SimpleNamespace(ops=ops, coeff=coeff, flags=flags, n_terms=terms,
+                         terms=L.Terms(ops.data_ptr(), coeff.data_ptr(), flags.data_ptr(), terms))
+    eng.read_tables(op)
+    assert op.is_real == (not cplx) and op.max_orbital == max(top, 7 if terms > 1 else -1)

@@ -808,8 +808,10 @@ struct Vec16<double> {
 constexpr int kRowsThreads = 128;  // smaller blocks shorten the tail of ragged rows
 
 // RV runs per thread: what 16 bytes hold, or one (8 bytes) for an odd number of complex64 runs.
-// shift != 0: Y = H X + shift X.
-template <typename T, bool VALC, int RV>
+// SHIFT: Y = H X + shift X.  A kernel of its own, its x read as the row is stored: the shift and the x held through
+// the row cost the unshifted FP64 products registers and 10 to 28 % of their time (200 000 rows of 5
+// entries, R = 3: 24.6 -> 29.6 us, R = 16: 94 -> 120).
+template <typename T, bool VALC, int RV, bool SHIFT>
 __global__ void __launch_bounds__(kRowsThreads) spmm_rows_kernel(int64_t n, const int64_t* __restrict__ rp,
                                                                  const int32_t* __restrict__ col,
                                                                  const T* __restrict__ vals, int R, int L, T shift,
@@ -822,8 +824,6 @@ __global__ void __launch_bounds__(kRowsThreads) spmm_rows_kernel(int64_t n, cons
   const int g = (int)(gt - i * L);
   if (i >= n) return;
   const int64_t r0 = (int64_t)g * RV;
-  Q own{};
-  if (shift != T(0)) own = __ldg(reinterpret_cast<const Q*>(X + i * R + r0));
   T ar[RV], ai[RV];
 #pragma unroll
   for (int q = 0; q < RV; ++q) ar[q] = ai[q] = 0;
@@ -867,11 +867,12 @@ __global__ void __launch_bounds__(kRowsThreads) spmm_rows_kernel(int64_t n, cons
   }
   Q out;
   T* os = reinterpret_cast<T*>(&out);
+  const Q own = SHIFT ? __ldg(reinterpret_cast<const Q*>(X + i * R + r0)) : Q{};
   const T* xo = reinterpret_cast<const T*>(&own);
 #pragma unroll
   for (int q = 0; q < RV; ++q) {
-    os[2 * q] = shift != T(0) ? ar[q] + shift * xo[2 * q] : ar[q];
-    os[2 * q + 1] = shift != T(0) ? ai[q] + shift * xo[2 * q + 1] : ai[q];
+    os[2 * q] = SHIFT ? ar[q] + shift * xo[2 * q] : ar[q];
+    os[2 * q + 1] = SHIFT ? ai[q] + shift * xo[2 * q + 1] : ai[q];
   }
   __stcs(reinterpret_cast<Q*>(Y + i * R + r0), out);
 }
@@ -882,12 +883,10 @@ int launch_rows(const edgpu_csr* h, const T* val_c, const T* val_r, T shift, con
   const int L = R / RV;
   const int64_t blocks = (h->n * (int64_t)L + kRowsThreads - 1) / kRowsThreads;
   if (blocks > 0x7fffffffLL) return EDGPU_ERR_ARG;
-  if (val_c)
-    spmm_rows_kernel<T, true, RV><<<(unsigned)blocks, kRowsThreads, 0, s>>>(h->n, h->row_ptr, h->col, val_c, R, L,
-                                                                            shift, x, y);
-  else
-    spmm_rows_kernel<T, false, RV><<<(unsigned)blocks, kRowsThreads, 0, s>>>(h->n, h->row_ptr, h->col, val_r, R, L,
-                                                                             shift, x, y);
+  auto kern = val_c ? spmm_rows_kernel<T, true, RV, false> : spmm_rows_kernel<T, false, RV, false>;
+  if constexpr (sizeof(T) == 4)  // only the float copies are shifted
+    if (shift != T(0)) kern = val_c ? spmm_rows_kernel<T, true, RV, true> : spmm_rows_kernel<T, false, RV, true>;
+  kern<<<(unsigned)blocks, kRowsThreads, 0, s>>>(h->n, h->row_ptr, h->col, val_c ? val_c : val_r, R, L, shift, x, y);
   note_launch();
   return check_launch();
 }

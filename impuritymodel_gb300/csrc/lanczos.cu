@@ -9,6 +9,7 @@
 // row read the row's CSR entries once (broadcast) and gather x[col][0..R) contiguously.
 // All reductions are deterministic: per-block partials in fixed order, summed in fixed order.
 #include <algorithm>
+#include <climits>
 #include <atomic>
 #include <type_traits>
 #include <vector>
@@ -214,9 +215,13 @@ __device__ __forceinline__ typename Cx<T>::V row_products(int64_t e, int64_t e1,
   return y;
 }
 
-// Rows longer than this are split among kStepSplit threads per run.  The sectors' first rows (few
-// bath holes) are the long ones: 3045 of the 47 895 hold 43 % of the entries, about 65 each,
-// against 7 in the others, and one thread's chain of 65 gathers was the launch's length.
+// Rows longer than this are split among kStepSplit threads per run, after the others.  The sectors' first
+// rows (few bath holes) are the long ones: 3045 of the 47 895 hold 43 % of the entries, about 65 each,
+// against 7 in the others, and one thread's chain of 65 gathers was the launch's length.  Not with more
+// than 32 runs: a warp is then one row of 32 runs, and there are warps enough beside the long ones.
+// The block's threads meet only for the long rows: a barrier in every pass of 16 rows cost 200 000 rows and
+// 100 runs 20 % against the row loop without one (6 steps 7.99 -> 6.12 ms; 47 895 rows of the
+// 316-spin-orbital sector 2.83 -> 2.44, split rows given up too).
 constexpr int kStepHeavy = 24;
 constexpr int kStepSplit = 8;
 
@@ -227,7 +232,7 @@ constexpr int kStepSplit = 8;
 template <typename T, bool VALC>
 __global__ void __launch_bounds__(kStepMaxThreads, 2) step_spmm_kernel(int64_t n, const int64_t* __restrict__ rp,
                                                         const int32_t* __restrict__ col, const T* __restrict__ vals,
-                                                        int R, int group, const typename Cx<T>::V* __restrict__ X,
+                                                        int R, int group, int heavy, const typename Cx<T>::V* __restrict__ X,
                                                         typename Cx<T>::V* __restrict__ Y, double* __restrict__ pa,
                                                         const double* __restrict__ pb, double* __restrict__ beta,
                                                         int K, int j, const int32_t* __restrict__ k_max,
@@ -241,24 +246,31 @@ __global__ void __launch_bounds__(kStepMaxThreads, 2) step_spmm_kernel(int64_t n
   const int tid = ti * blockDim.x + tr, lane = tid & 31, warp = tid >> 5;
   const int r = blockIdx.y * blockDim.x + tr;
   double acc = 0.0;
-  for (int64_t base = 0; base / group * group * gridDim.x < n; base += rb) {  // block-uniform; rb may cut a group
+  const auto row_of = [&](int64_t base) {
     const int64_t lin = base + ti;
-    const int64_t i = (lin / group * gridDim.x + blockIdx.x) * group + lin % group;
-    int64_t e0 = 0, e1 = 0;
-    if (i < n) {
-      e0 = __ldg(rp + i);
-      e1 = __ldg(rp + i + 1);
-    }
-    const bool heavy = e1 - e0 > kStepHeavy;
-    if (i < n && !heavy && r < R) {
+    return (lin / group * gridDim.x + blockIdx.x) * group + lin % group;
+  };
+  const auto more = [&](int64_t base) { return base / group * group * gridDim.x < n; };  // block-uniform; rb may cut a group
+  bool any = false;
+  for (int64_t base = 0; more(base); base += rb) {
+    const int64_t i = row_of(base);
+    if (i >= n) continue;
+    const int64_t e0 = __ldg(rp + i), e1 = __ldg(rp + i + 1);
+    if (e1 - e0 > heavy) {
+      any = true;
+    } else if (r < R) {
       const V v = ld(X + i * R + r);
       const V y = row_products<T, VALC>(e0, e1, 1, col, vals, R, r, X);
       Y[i * R + r] = y;
       acc += (double)y.x * (double)v.x + (double)y.y * (double)v.y;
     }
-    // the pass's long rows, listed in thread order: kStepSplit threads per run and row, their
-    // parts added in a fixed order by the first of them
-    const bool mine = heavy && tr == 0;
+  }
+  // the long rows after the others, pass by pass, listed in thread order: kStepSplit threads per run and row,
+  // their parts added in a fixed order by the first of them
+  const bool long_rows = __syncthreads_or(any);
+  for (int64_t base = 0; long_rows && more(base); base += rb) {
+    const int64_t i = row_of(base);
+    const bool mine = tr == 0 && i < n && __ldg(rp + i + 1) - __ldg(rp + i) > heavy;
     const int nh = __syncthreads_count(mine);
     if (nh == 0) continue;
     const int in_warp = (int)(blockDim.x * blockDim.y) - 32 * warp;  // threads of this warp
@@ -1278,14 +1290,15 @@ int lanczos_impl(const edgpu_csr* h, const double* v0, int R, const int32_t* k_m
   // one pass over the rows: single rows dealt to the blocks; several: groups of 8, so that the
   // CSR of neighbouring rows is read by one block
   const int group = (int64_t)t.nrb * t.rb >= n ? 1 : 8;
+  const int heavy = t.nrt > 1 ? INT_MAX : kStepHeavy;
   KernelTimer timer(kernel_ms, K, s);
   for (int j = 0; j < K; ++j) {
     timer.mark(0, j, 0);
     if (valc)
-      step_spmm_kernel<T, true><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, group, Wc, Wb, pa, pb, beta, K, j,
+      step_spmm_kernel<T, true><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, group, heavy, Wc, Wb, pa, pb, beta, K, j,
                                                          k_max, status);
     else
-      step_spmm_kernel<T, false><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, group, Wc, Wb, pa, pb, beta, K, j,
+      step_spmm_kernel<T, false><<<grid, block, red, s>>>(n, h->row_ptr, h->col, vals, R, group, heavy, Wc, Wb, pa, pb, beta, K, j,
                                                           k_max, status);
     note_launch();
     timer.mark(0, j, 1);

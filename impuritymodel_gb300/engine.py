@@ -516,8 +516,7 @@ class Engine:
 
     def _apply_groups(self, states, dop, restr, weight_min, basis, filt, want, conj):
         """H|b> of every state in one pass (edgpu_apply_groups).  ``want``: names of the outputs
-        ("states", "index", "vals", "col", "real"); none: counts only.  Returns (offsets, dict), or None
-        where memory does not hold the outputs twice (32 bytes each in the arena)."""
+        ("states", "index", "vals", "col", "real"); none: counts only.  Returns (offsets, dict)."""
         n, w = states.shape
         dev, lib = self.device, self.lib
         plan = self._plan(dop, w)
@@ -548,10 +547,7 @@ class Engine:
         while True:
             if want and (arena is None or arena.numel() < cap * entry):
                 arena = None
-                try:
-                    arena = torch.empty(cap * entry, dtype=torch.uint8, device=dev)
-                except torch.cuda.OutOfMemoryError:
-                    return None
+                arena = torch.empty(cap * entry, dtype=torch.uint8, device=dev)
             L.check(
                 lib.edgpu_apply_groups(w, _ptr(states), n, _ptr(plan), dop.n_terms, real, rp, weight_min,
                                        _ptr(basis), nb, _ptr(table), 0 if table is None else table.numel(), filt,
@@ -574,16 +570,21 @@ class Engine:
             break
         kinds = {"states": ((total, w), torch.int64), "index": ((total,), torch.int64), "col": ((total,), torch.int32),
                  "vals": ((total, 2), torch.float64), "real": ((total,), torch.float64)}
-        try:
-            out = {k: torch.empty(kinds[k][0], dtype=kinds[k][1], device=dev) for k in want}
-        except torch.cuda.OutOfMemoryError:
-            return None
+        out = {k: torch.empty(kinds[k][0], dtype=kinds[k][1], device=dev) for k in want}
         if total and want:
             L.check(
                 lib.edgpu_apply_groups_gather(w, _ptr(states), n, _ptr(offsets), _ptr(arena),
                                               *(_ptr(out.get(k)) for k in ("states", "index", "col", "vals", "real")),
                                               int(conj), _ptr(ws), wsn, self.stream), "apply_groups_gather")
         return offsets, out
+
+    def _one_pass(self, *args):
+        """:meth:`_apply_groups`, or None where memory does not hold what it adds to the outputs (an arena
+        of 32 bytes each, up to eight bytes of table a basis state, 48 bytes a state)."""
+        try:
+            return self._apply_groups(*args)
+        except torch.cuda.OutOfMemoryError:
+            return None
 
     def _groups_ok(self, dop, w):
         if dop.n_terms and dop.tables_read != _table_versions(dop):
@@ -596,7 +597,7 @@ class Engine:
         n, w = states.shape
         if n and self._groups_ok(dop, w):
             want = [k for k, on in (("states", want_states), ("index", want_index), ("vals", want_vals)) if on]
-            got = self._apply_groups(states, dop, restr, weight_min, basis, filt, want, conj)
+            got = self._one_pass(states, dop, restr, weight_min, basis, filt, want, conj)
             if got is not None:
                 offsets, out = got
                 return offsets, out.get("states"), out.get("index"), out.get("vals")
@@ -799,8 +800,8 @@ class Engine:
         n, w = basis_sorted.shape
         if n and self._groups_ok(dop, w):
             val = "real" if dop.is_real else "vals"
-            got = self._apply_groups(basis_sorted, dop, restr, weight_min, basis_sorted, L.FILTER_IN_BASIS,
-                                     ("col", val), True)
+            got = self._one_pass(basis_sorted, dop, restr, weight_min, basis_sorted, L.FILTER_IN_BASIS,
+                                 ("col", val), True)
             if got is not None:
                 offsets, out = got
                 if dop.is_real:

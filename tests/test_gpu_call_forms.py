@@ -257,14 +257,14 @@ def test_a_read_status_is_spent(eng):
     rank()
 
 
-@pytest.mark.parametrize("grown", [False, True])
-def test_application_without_room_for_its_arena(eng, monkeypatch, grown):
+@pytest.mark.parametrize("what", ["arena", "larger arena", "table"])
+def test_application_without_room_for_its_arena(eng, monkeypatch, what):
     """The two passes, which keep nothing but the outputs, take the call."""
     from impuritymodel_gb300 import _lib as L
     from impuritymodel_gb300.engine import DeviceOp
 
     op = _hopping(26)
-    # without `grown` the first arena is refused, with it the one for 45 outputs a state that follows
+    # refused: the first arena, the one for 45 outputs a state that follows, the hash table of the basis
     op.update({((i, "c"), (j, "a")): 0.01 * (i + 1) * (j + 1) for i in range(26) for j in range(26) if (i - j) % 26 > 1})
     dop = DeviceOp(op, eng.device)
     basis, _ = eng.expand(_start(eng, (0b1011 << 60,)), dop, None)
@@ -276,10 +276,12 @@ def test_application_without_room_for_its_arena(eng, monkeypatch, grown):
     empty = torch.empty
 
     def refuse(*size, **kw):
-        if kw.get("dtype") == torch.uint8 and size[0] >= entry * (first + 1 if grown else first):
+        big = entry * (first + 1 if what == "larger arena" else first)
+        if kw.get("dtype") == torch.uint8 and size[0] >= big if what != "table" else size == (8192,):
             raise torch.cuda.OutOfMemoryError("refused")
         return empty(*size, **kw)
 
+    monkeypatch.setattr(eng, "TABLE_MIN_BASIS", 1)
     monkeypatch.setattr(torch, "empty", refuse)
     got = eng.build_csr(basis, dop, None)
     got_c = eng.apply_columns(basis, dop, None, 0.0, want_states=True, want_vals=True)

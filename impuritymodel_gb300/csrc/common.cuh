@@ -139,6 +139,34 @@ __device__ __forceinline__ int64_t find_state(const uint64_t* basis, int64_t n, 
   return -1;
 }
 
+// Open-addressing hash of product states (edgpu_state_hash_build): slot -> basis index or -1,
+// linear probing in a power-of-two table at most half full, so a lookup is one or two table
+// reads and one basis read instead of ~log2(n) dependent basis reads of a binary search.
+template <int W>
+__device__ __forceinline__ uint64_t state_hash(const uint64_t (&s)[W]) {
+  uint64_t h = 0x243F6A8885A308D3ull;
+#pragma unroll
+  for (int q = 0; q < W; ++q) {
+    h ^= s[q] + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
+    h *= 0xBF58476D1CE4E5B9ull;
+    h ^= h >> 31;
+  }
+  return h;
+}
+
+template <int W>
+__device__ __forceinline__ int64_t hash_find(const uint64_t* __restrict__ basis, const int32_t* __restrict__ table,
+                                             uint64_t mask, const uint64_t (&key)[W]) {
+  uint64_t slot = state_hash<W>(key) & mask;
+  for (uint64_t probe = 0; probe <= mask; ++probe) {
+    const int32_t idx = __ldg(table + slot);
+    if (idx < 0) return -1;
+    if (state_eq<W>(key, basis + (int64_t)idx * W)) return idx;
+    slot = (slot + 1) & mask;
+  }
+  return -1;
+}
+
 // Apply one packed term (up to 4 elementary operators, right to left) to state s.
 // Returns false if Pauli-blocked; otherwise s holds the new state and parity the number
 // of transpositions (sign = (-1)^parity).  Sign rule of upstream create/remove.ubitarray:

@@ -294,44 +294,14 @@ struct GroupParams {
 };
 
 template <int W>
-__device__ __forceinline__ uint64_t group_state_hash(const uint64_t (&s)[W]) {
-  // as edgpu_state_hash_build
-  uint64_t h = 0x243F6A8885A308D3ull;
-#pragma unroll
-  for (int q = 0; q < W; ++q) {
-    h ^= s[q] + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
-    h *= 0xBF58476D1CE4E5B9ull;
-    h ^= h >> 31;
-  }
-  return h;
-}
-
-template <int W>
 __device__ __forceinline__ int64_t group_find(const GroupParams& p, const uint64_t (&s)[W]) {
   if (!p.table) return find_state<W>(p.basis, p.n_basis, s);
-  uint64_t slot = group_state_hash<W>(s) & p.table_mask;
-  for (uint64_t probe = 0; probe <= p.table_mask; ++probe) {
-    const int32_t i = __ldg(p.table + slot);
-    if (i < 0) return -1;
-    if (state_eq<W>(s, p.basis + (int64_t)i * W)) return i;
-    slot = (slot + 1) & p.table_mask;
-  }
-  return -1;
+  return hash_find<W>(p.basis, p.table, p.table_mask, s);
 }
 
 // |v|^2 as CPython computes it; hypot(x, 0) is |x|
 __device__ __forceinline__ double abs2_fast(double re, double im) {
   return im == 0.0 ? __dmul_rn(re, re) : abs2_py(re, im);
-}
-
-template <int W>
-__device__ __forceinline__ bool group_keep(const GroupParams& p, const uint64_t (&s)[W], double re, double im,
-                                           int64_t& idx) {
-  idx = -1;
-  if (!(abs2_fast(re, im) >= p.weight_min) || !restr_ok<W>(p.restr, s)) return false;
-  if (p.filter == EDGPU_FILTER_NONE) return true;
-  idx = group_find<W>(p, s);
-  return p.filter == EDGPU_FILTER_IN_BASIS ? idx >= 0 : idx < 0;
 }
 
 // s with the orbitals of key flipped

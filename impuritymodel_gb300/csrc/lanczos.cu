@@ -60,50 +60,39 @@ inline RunTile make_tile(int64_t n, int R) {
   return t;
 }
 
-// Y = H X and alpha partial Re<Y, X> per run.  T: vector/accumulation scalar, VALC: complex values.
-template <typename T, bool VALC>
-__global__ void spmm_alpha_kernel(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                                  const T* __restrict__ vals, int R, const typename Cx<T>::V* __restrict__ X,
-                                  typename Cx<T>::V* __restrict__ Y, double* __restrict__ partial, int with_alpha) {
-  using V = typename Cx<T>::V;
+// y = H x and the per-block partials of Re<y, x>: one vector, a row per thread (blockDim.y of them).
+template <bool VALC>
+__global__ void spmv_alpha_kernel(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                                  const double* __restrict__ vals, const double2* __restrict__ x,
+                                  double2* __restrict__ y, double* __restrict__ partial) {
   extern __shared__ double red[];
-  const int tr = threadIdx.x, ti = threadIdx.y;
-  const int r = blockIdx.y * blockDim.x + tr;
+  const int ti = threadIdx.y;
   double acc = 0.0;
-  if (r < R) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.y + ti; i < n; i += (int64_t)gridDim.x * blockDim.y) {
-      T yr = 0, yi = 0;
-      const int64_t e1 = rp[i + 1];
-      for (int64_t e = rp[i]; e < e1; ++e) {
-        const int c = col[e];
-        const V x = ld(X + (int64_t)c * R + r);
-        if (VALC) {
-          const T hr = vals[2 * e], hi = vals[2 * e + 1];
-          yr += hr * x.x - hi * x.y;
-          yi += hr * x.y + hi * x.x;
-        } else {
-          const T h = vals[e];
-          yr += h * x.x;
-          yi += h * x.y;
-        }
-      }
-      V y;
-      y.x = yr;
-      y.y = yi;
-      Y[i * R + r] = y;
-      if (with_alpha) {
-        const V v = ld(X + i * R + r);
-        acc += (double)yr * (double)v.x + (double)yi * (double)v.y;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.y + ti; i < n; i += (int64_t)gridDim.x * blockDim.y) {
+    double yr = 0.0, yi = 0.0;
+    const int64_t e1 = rp[i + 1];
+    for (int64_t e = rp[i]; e < e1; ++e) {
+      const double2 xv = x[col[e]];
+      if (VALC) {
+        const double hr = vals[2 * e], hi = vals[2 * e + 1];
+        yr += hr * xv.x - hi * xv.y;
+        yi += hr * xv.y + hi * xv.x;
+      } else {
+        const double h = vals[e];
+        yr += h * xv.x;
+        yi += h * xv.y;
       }
     }
+    y[i] = make_double2(yr, yi);
+    const double2 v = x[i];
+    acc += yr * v.x + yi * v.y;
   }
-  if (!with_alpha) return;
-  red[ti * blockDim.x + tr] = acc;
+  red[ti] = acc;
   __syncthreads();
-  if (ti == 0 && r < R) {
+  if (ti == 0) {
     double s = 0.0;
-    for (int k = 0; k < (int)blockDim.y; ++k) s += red[k * blockDim.x + tr];
-    partial[(int64_t)blockIdx.x * R + r] = s;
+    for (int k = 0; k < (int)blockDim.y; ++k) s += red[k];
+    partial[blockIdx.x] = s;
   }
 }
 
@@ -1486,11 +1475,10 @@ extern "C" int edgpu_lanczos_reorth(const edgpu_csr* h, const double* v0, int j0
     // w = H v_j ; alpha partials
     dim3 grid(nrb, 1), block(1, 256);
     if (h->val_c)
-      spmm_alpha_kernel<double, true><<<grid, block, sizeof(double) * 256, s>>>(n, h->row_ptr, h->col, h->val_c, 1,
-                                                                                vj, w, pa, 1);
+      spmv_alpha_kernel<true><<<grid, block, sizeof(double) * 256, s>>>(n, h->row_ptr, h->col, h->val_c, vj, w, pa);
     else
-      spmm_alpha_kernel<double, false><<<grid, block, sizeof(double) * 256, s>>>(n, h->row_ptr, h->col, h->val_r, 1,
-                                                                                 vj, w, pa, 1); note_launch();
+      spmv_alpha_kernel<false><<<grid, block, sizeof(double) * 256, s>>>(n, h->row_ptr, h->col, h->val_r, vj, w, pa);
+    note_launch();
     reorth_alpha_update_kernel<<<nrb, 256, 0, s>>>(n, w, vj, j > 0 ? V + (int64_t)(j - 1) * n : nullptr, pa, nrb,
                                                    alpha, beta, j, pn); note_launch();
     if ((rc = check_launch())) return rc;

@@ -33,21 +33,6 @@ struct MfPack<double> {
   static constexpr int runs = 1;
 };
 
-// Open-addressing hash of product states (edgpu_state_hash_build): slot -> basis index or -1,
-// linear probing in a power-of-two table at most half full, so a lookup is one or two table
-// reads and one basis read instead of ~log2(n) dependent basis reads of a binary search.
-template <int W>
-__device__ __forceinline__ uint64_t state_hash(const uint64_t (&s)[W]) {
-  uint64_t h = 0x243F6A8885A308D3ull;
-#pragma unroll
-  for (int q = 0; q < W; ++q) {
-    h ^= s[q] + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
-    h *= 0xBF58476D1CE4E5B9ull;
-    h ^= h >> 31;
-  }
-  return h;
-}
-
 template <int W>
 __global__ void state_hash_insert_kernel(const uint64_t* __restrict__ basis, int64_t n, int32_t* table,
                                          uint64_t mask) {
@@ -60,19 +45,6 @@ __global__ void state_hash_insert_kernel(const uint64_t* __restrict__ basis, int
     if (atomicCAS(reinterpret_cast<int*>(table + slot), -1, (int)i) == -1) return;
     slot = (slot + 1) & mask;
   }
-}
-
-template <int W>
-__device__ __forceinline__ int64_t hash_find(const uint64_t* __restrict__ basis, const int32_t* __restrict__ table,
-                                             uint64_t mask, const uint64_t (&key)[W]) {
-  uint64_t slot = state_hash<W>(key) & mask;
-  for (uint64_t probe = 0; probe <= mask; ++probe) {
-    const int32_t idx = __ldg(table + slot);
-    if (idx < 0) return -1;
-    if (state_eq<W>(key, basis + (int64_t)idx * W)) return idx;
-    slot = (slot + 1) & mask;
-  }
-  return -1;
 }
 
 constexpr int kMfWarps = 8;      // warps (rows in flight) per block

@@ -917,14 +917,20 @@ def gemm_timing(eng, peaks, batch=4096, wide=65536, reps=20):
                      "tflops": round(tf, 2), "frac": round(tf / peak, 4) if peak else None}
     target = torch.randn(B, device=dev, generator=g)
 
-    def train_step():
+    def layers():
         net.gradients(X, Xt, target)
         net.adam_step()
 
-    step_us = timed(train_step)
+    layers_us = timed(layers)
+    # what BasisNet.train runs: the same step in one call, occupation words in
+    idx = torch.arange(B, device=dev)
+    states = torch.randint(-(1 << 62), 1 << 62, (B, 5), device=dev, generator=g) * 2
+    ws = torch.empty(eng.lib.edgpu_mlp_step_workspace(B), dtype=torch.uint8, device=dev)
+    loss = torch.empty(1, dtype=torch.float32, device=dev)
+    step_us = timed(lambda: net._train_step(states, target, idx, loss, ws))
     eng.read_status("gemm timing")
     flops = 2.0 * B * (nh * ni + nh * nh) * 3
-    return {"gemms": out, "train_step_us": round(step_us, 1),
+    return {"gemms": out, "train_step_us": round(step_us, 1), "train_step_by_layers_us": round(layers_us, 1),
             "train_tflops": round(flops / step_us / 1e6, 2), "batch": B,
             "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst, of measured)", "inputs": "L2-resident"}
 

@@ -936,10 +936,11 @@ struct KernelTimer {
 // threads per row and run; a warp's rows have nearly equal lengths.  Two grid barriers a step (after the
 // partials of alpha_j and of beta_j^2), the sums of the blocks' partials by a warp per run in one
 // fixed order.
-// Bound by FP64 issue in the products (16 cycles a warp instruction: 9.4 us a step for 3 runs of 47 895
-// rows) and the latency of the barriers and sums.
-// 47 895 rows, 0.93 M entries, 100 steps: 3 runs 4.0 -> 2.56 ms (two launches a step pay their gaps, read
-// H and the vectors again and wait for the long rows); 40 steps of 1 run 1.21 -> 0.81, of 8 2.35 -> 1.82.
+// Bound by latency: of a step's 25 us for 3 runs of 47 895 rows with 458 223 entries the products' FP64
+// issue is 4.4 (16 cycles a warp instruction), their phase 10 to 15 (the long rows, lanes idle beside rows of
+// six entries), the barriers and sums the rest.
+// 100 steps there: 2.54 ms.  40 steps of 1, 3, 8, 16 runs 0.81, 1.12, 1.82, 3.21 ms, in two launches a step 1.12,
+// 1.56, 2.18, 3.21 (their gaps, H and the vectors read again); of 32 runs of 4300 short rows 1.59 and 1.35.
 constexpr int kGridThreads = 1024;
 constexpr int kGridRuns = kGridThreads / 32;
 constexpr int kGridRows = 2048;  // rows of a block at most (their ranks take rows^2 / 1024 steps)
@@ -1214,7 +1215,7 @@ static bool launch_grid(const edgpu_csr* h, const double* v0, int R, const int32
   g.v0 = reinterpret_cast<const double2*>(v0);
   g.R = R;
   g.K = K;
-  // The few long rows of a sector (65 entries of 19 on average) set the products' length: 40 steps of the
+  // The few long rows of a sector (65 entries, 9.6 on average) set the products' length: 40 steps of the
   // 316-spin-orbital sector take 1143, 864, 808 us with 1, 2, 4 threads a row for one run, 1349, 1114,
   // 1286 for 3 runs and 1930, 1822, 2542 for 8.
   g.sub = most * R <= 320 ? 4 : 2;
@@ -3106,7 +3107,9 @@ __global__ void __launch_bounds__(256) shifted_coef_kernel(
 //   s1 += cr (vr + vi), s2 += vi (cr + ci), s3 += vr (ci - cr)
 // the sums are re = s1 - s2, im = s1 + s3; vr + vi is formed once for all shifts, the coefficient
 // sums once per block.  (Written as a sum of products the four compiled to six.)  15 x 50 sums of
-// ~490 vectors of 360 rows: 1.60 -> 0.81 ms.
+// ~490 vectors of 360 rows: 1.60 -> 0.81 ms.  The rounding is bounded by |c| |v| and not by each component, so
+// the smaller of a sum's real and imaginary parts is relatively less accurate than by four products; both errors
+// lie far below the 1e-10 at which the solves stop.
 constexpr int kSumZ = 4, kSumRows = 64, kSumStage = 64;
 __global__ void __launch_bounds__(kSumRows) combine_batched_kernel(const double2* __restrict__ V,
                                                                    const double2* __restrict__ coef,

@@ -12,7 +12,6 @@ judge of the energy error (``pruned_ground_state`` reports both).
 
 from __future__ import annotations
 
-import ctypes as C
 import math
 
 import numpy as np
@@ -149,6 +148,18 @@ class BasisNet:
         self.refresh()
 
     # -- training and inference ----------------------------------------------------------
+    def _train_step(self, states, log_w, idx, loss, ws):
+        """Forward, gradients and Adam of the batch ``states[idx]``, ``log_w[idx]`` in one call
+        (:meth:`inputs`, :meth:`gradients` and :meth:`adam_step`, layer by layer); its loss into
+        ``loss[0]``.  Contiguous device tensors of :meth:`train`; ``ws``: bytes of
+        edgpu_mlp_step_workspace(len(idx))."""
+        e = self.eng
+        L.check(self._lib().edgpu_mlp_train_step(_ptr(states), states.shape[1], _ptr(idx), _ptr(log_w), idx.shape[0],
+                                                 N_IN, N_H, _ptr(self.P), _ptr(self.G), _ptr(self.m), _ptr(self.v),
+                                                 _ptr(self.W1b), _ptr(self.W2b), _ptr(self.W2t),
+                                                 self._next_rate(0.9, 0.999), 0.9, 0.999, 1e-8, _ptr(loss),
+                                                 _ptr(e.status), _ptr(ws), ws.numel(), e.stream), "mlp_train_step")
+
     def train(self, states, log_w, epochs=4, batch=4096, seed=0, log=None):
         """Fit log10 weights ``log_w`` [N] of padded states [N, WORDS] by Adam on shuffled batches."""
         batch = max(ROWS, (batch // ROWS) * ROWS)
@@ -174,14 +185,7 @@ class BasisNet:
         for ep in range(epochs):
             perm = torch.randperm(n, device=dev, generator=gen)
             for s in range(steps):
-                # forward, gradients and Adam of one batch (inputs, gradients and adam_step in one call)
-                lr_t = self._next_rate(0.9, 0.999)
-                L.check(lib.edgpu_mlp_train_step(_ptr(states), states.shape[1], C.c_void_p(perm.data_ptr() + 8 * s * batch),
-                                                 _ptr(log_w), batch, N_IN, N_H, _ptr(self.P), _ptr(self.G),
-                                                 _ptr(self.m), _ptr(self.v), _ptr(self.W1b), _ptr(self.W2b),
-                                                 _ptr(self.W2t), lr_t, 0.9, 0.999, 1e-8,
-                                                 C.c_void_p(loss.data_ptr() + 4 * k), _ptr(e.status), _ptr(ws), wsn,
-                                                 e.stream), "mlp_train_step")
+                self._train_step(states, log_w, perm[s * batch: (s + 1) * batch], loss[k:], ws)
                 k += 1
             if log is not None:
                 log.append(float(torch.stack(list(loss[:k].unbind())[-max(1, steps):]).mean().item()))

@@ -525,7 +525,7 @@ __global__ void mlp_to_bf16_kernel(const float* __restrict__ Wf, int rows, int c
 //     BF16, into the same A buffer as layer two's operand;
 //   * layer two's accumulator is read back, and the head's sum runs in the threads.
 // The BF16 roundings and the order of the K steps are those of the layer-by-layer kernels; the
-// head's FP32 sum runs in another order.  Time for 462 120 states: 0.86 -> 0.145 ms.  Bound: the
+// head's FP32 sum runs in another order.  Time for 462 120 states: 0.86 -> 0.138 ms.  Bound: the
 // phases of a pass follow one another (expansion 1.7k cycles, layer one 6.7k, epilogue, layer two
 // 5.3k, epilogue; the MMAs alone 9.2k).  With 8 epilogue warps and the biases read through L1 the
 // epilogues took 4.7k and 7-9k cycles; 16 warps with the biases in shared memory took 0.03 ms off.

@@ -313,3 +313,33 @@ def test_what_the_host_reads_of_tables(eng, terms, cplx, top):
                          terms=L.Terms(ops.data_ptr(), coeff.data_ptr(), flags.data_ptr(), terms))
     eng.read_tables(op)
     assert op.is_real == (not cplx) and op.max_orbital == max(top, 7 if terms > 1 else -1)
+
+
+@pytest.mark.parametrize("n,R,precision", [
+    (1770, 3, 0), (1770, 160, 0),  # one SM, CSR and sliced rows
+    (5000, 3, 0),                  # one cooperative launch
+    (5000, 40, 0), (5000, 3, 1),   # two launches a step
+])
+def test_a_bad_run_keeps_to_itself(eng, n, R, precision):
+    """A start vector with a NaN or an infinity, or of zeros: its status, and the other runs' bits."""
+    from impuritymodel_gb300 import _lib as L
+
+    K = 9
+    csr, _ = _random_csr(eng, n, n + R, heavy=(0, n // 2))
+    g = torch.Generator(device=eng.device)
+    g.manual_seed(n)
+    v = torch.randn((n, R), dtype=torch.complex128, device=eng.device, generator=g)
+    v /= torch.linalg.vector_norm(v, dim=0)
+    a, b = eng.lanczos(csr, v, [K] * R, precision=precision)
+    others = [r for r in range(R) if r != 1]
+    for value, status in ((float("nan"), L.EDGPU_ERR_NAN), (float("inf"), L.EDGPU_ERR_NAN), (0.0, L.EDGPU_ERR_BREAKDOWN)):
+        w = v.clone()
+        w[slice(None) if value == 0.0 else n // 2, 1] = value
+        with pytest.raises(L.EdgpuError) as err:
+            eng.lanczos(csr, w, [K] * R, precision=precision)
+        assert err.value.status == status
+        a1, b1 = eng.lanczos(csr, w, [K] * R, precision=precision, check=False)
+        assert torch.equal(a[others], a1[others]) and torch.equal(b[others, :K - 1], b1[others, :K - 1])
+        if value != 0.0:
+            assert not bool(torch.isfinite(a1[1]).any())
+    eng.reset_status()

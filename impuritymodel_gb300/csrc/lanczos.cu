@@ -9,8 +9,8 @@
 // row read the row's CSR entries once (broadcast) and gather x[col][0..R) contiguously.
 // All reductions are deterministic: per-block partials in fixed order, summed in fixed order.
 #include <algorithm>
-#include <climits>
 #include <atomic>
+#include <climits>
 #include <type_traits>
 #include <vector>
 
